@@ -61,254 +61,288 @@ __device__ __forceinline__ int ld_relaxed(const int* p) {
   return v;
 }
 
+// ------------------------------------------------------------------------- FP64 tensor-core product
+// mma.sync.m8n8k4.f64 (FP64 has no tcgen05 kind; this is the FP64 tensor path of sm_100a).
+// Fragments: A (8 x 4) lane l holds A[l/4][l%4]; B (4 x 8) holds B[l%4][l/4]; C (8 x 8) holds
+// C[l/4][2(l%4) + {0,1}].  Measured on a B200: 64 fma per clock and SM (57 for the scalar fma),
+// 26 cycles from accumulator to accumulator, and the same bits as the four fma in ascending k
+// (128 000 random outputs of mixed magnitude), so a chain of them keeps the arithmetic contract
+// above; the bitwise tests against the oracle hold that.
+__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+
+// asynchronous copies into shared memory; bytes past `valid` are written as zeros.  The 16-byte
+// form bypasses L1; the 8-byte form (odd strides or offsets) allocates there, which the VM's
+// acquire before each task makes safe: it invalidates this SM's L1.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const double* src, uint32_t valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const double* src, uint32_t valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(valid) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// A thread index the compiler cannot hoist out of the task loop: every routine's thread-dependent
+// values would otherwise be live at once in the one kernel they are inlined into.
+__device__ __forceinline__ int thread_index() {
+  int t;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+  return t;
+}
+
+// Predicated accesses: a branch costs a warp about 30 cycles, and with two warps per scheduler
+// little hides it.
+__device__ __forceinline__ double ldcg_if(const double* p, bool in) {
+  double v;
+  asm volatile("{\n .reg .pred a;\n setp.ne.s32 a, %2, 0;\n mov.f64 %0, 0d0000000000000000;\n @a ld.global.cg.f64 %0, [%1];\n}\n"
+               : "=&d"(v)
+               : "l"(p), "r"((int)in)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_if(double* p, double v, bool in) {
+  asm volatile("{\n .reg .pred a;\n setp.ne.s32 a, %2, 0;\n @a st.global.f64 [%1], %0;\n}\n" ::"d"(v), "l"(p), "r"((int)in)
+               : "memory");
+}
+
+__host__ __device__ constexpr int log2_of(int v) { return v <= 1 ? 0 : 1 + log2_of(v / 2); }
+
+// Four copies of one thread (16 bytes of `valid`, or 8), rows r, r + step, ... below `rows`, the
+// source and the destination advancing by sstep and dstep bytes; predicated, without branches.
+template <bool WIDE>
+__device__ __forceinline__ void copy_rows4(uint32_t& dst, const char*& src, int& r, uint32_t dstep, uint64_t sstep,
+                                           int step, int rows, uint32_t valid) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (WIDE)
+      asm volatile("{\n .reg .pred p;\n setp.lt.s32 p, %2, %3;\n @p cp.async.cg.shared.global [%0], [%1], 16, %4;\n}\n" ::"r"(dst),
+                   "l"(src), "r"(r), "r"(rows), "r"(valid)
+                   : "memory");
+    else
+      asm volatile("{\n .reg .pred p;\n setp.lt.s32 p, %2, %3;\n @p cp.async.ca.shared.global [%0], [%1], 8;\n}\n" ::"r"(dst),
+                   "l"(src), "r"(r), "r"(rows)
+                   : "memory");
+    r += step;
+    src += sstep;
+    dst += dstep;
+  }
+}
+
 // ------------------------------------------------------------------------- GEMM
-// C[m x n] = beta C + alpha op(A) op(B), alpha in {+1, -1}, beta in {0, 1}.
-// CTA tile TM x TN, thread micro-tile RM x RN (rows ty + TY a, columns tx + TX b), k in
-// chunks of KCH staged through shared memory; the next chunk is fetched into registers
-// while the current one is consumed.  Each element's k loop runs in ascending order.
-template <int TM, int TN, int RM, int RN, int KCH>
-__device__ __noinline__ void gemm_cfg(double* __restrict__ C, int ldc, const double* __restrict__ A, int lda,
-                                         bool tA, const double* __restrict__ B, int ldb, bool tB, int m, int n, int k,
-                                         double alpha, double beta, double* smem) {
-  constexpr int TX = TN / RN, TY = TM / RM;
-  static_assert(TX * TY == NT, "thread layout");
-  constexpr int LA = TM + 1, LB = TN + 1;
-  constexpr int AE = TM * KCH, BE = KCH * TN;
-  constexpr int AP = (AE + NT - 1) / NT, BP = (BE + NT - 1) / NT;
-  static_assert((KCH * LA + KCH * LB) * 8 <= VM_SMEM_BYTES, "smem");
-  double* As = smem;             // [KCH][LA]
-  double* Bs = smem + KCH * LA;  // [KCH][LB]
-  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
-  const int nch = (k + KCH - 1) / KCH;
-  for (int i0 = 0; i0 < m; i0 += TM)
-    for (int j0 = 0; j0 < n; j0 += TN) {
-      double acc[RM][RN];
+// C[m x n] = C (or 0, beta = 0) + alpha op(A) op(B); every element's k
+// products in ascending order from beta c_ij (the reference's chain, see above), or with
+// `free_order` a small output's k split over warps.
+//
+// One piece of code for every shape and transposition: a task's instructions have usually been
+// evicted by the tasks before it, so much of what a small product costs is fetching its code
+// (forms specialised by tile shape, ten times the code, ran small shapes at half the speed inside
+// the VM and faster outside of it).  The output is walked in CTA tiles of TM x TN (128 x 16,
+// 64 x 32, 128 x 32, 16 x 64, 64 x 64: the narrowest that covers it) of 16 x 16 warp tiles, one or
+// two side by side per warp, k in chunks of GM_KC through a ring of GM_ST shared-memory stages over
+// (tile, chunk) pairs, so that the loads of the next chunks are in flight during the products.
+// Operands are staged as A[m][k] and B[k][n] whatever their storage, so that a fragment's address
+// is a register and a constant; the strides (4 mod 16 doubles) keep fragment loads free of bank
+// conflicts.
+// What bounds it: the loads' latency and the staging's instructions for small products, the FP64
+// tensor rate (2.1 M cycles for 512^3) and the staging that is not overlapped with it for large ones.
+// Time per instruction on a B200, hop to the next task included (before: SIMT tiles by shape, whose
+// operand loads were waited for before each chunk's products; hop 2.5 us):
+//   64 x 64 x 64     16.5 -> 9.1 us     64 x 16 x 64      15.9 -> 5.5 us
+//   64 x 64 x 256    42   -> 17.6 us    16 x 16 x 512     25   -> 10.8 us (k over 8 warps)
+//   512 x 512 x 512  2630 -> 1655 us    512 x 32 x 512    327  -> 105 us
+//   64 x 8 x 512     43   -> 15.3 us    256 x 1 x 256     48   -> 19 us
+#define GM_KC 64
+#define GM_LD (GM_KC + 4)
+#define GM_ST 2
+#define GM_STAGE (VM_SMEM_BYTES / 8 / GM_ST)  /* doubles: A 128 x 68 and B 64 x 36, or 64 x 68 and 64 x 68 */
+
+// v with its sign bit flipped where `mask` has it set (the factor alpha = -1, exactly: a
+// multiplication would take as long on the FP64 pipe as a product of fragments)
+__device__ __forceinline__ double flip(double v, int mask) {
+  return __hiloint2double(__double2hiint(v) ^ mask, __double2loint(v));
+}
+
+// passes of 8 k each (two steps of 4) on a 16 x (8 NW) warp tile
+template <int NW>
+__device__ __forceinline__ void gemm_passes(double (&acc)[2][4][2], const double* pa, const double* pb, int b_ld,
+                                            int first, int passes, int kw, int sgn) {
+#pragma unroll 1
+  for (int s = first; s < passes; s += kw) {
+    double av[2][2], bv[2][NW];
 #pragma unroll
-      for (int a = 0; a < RM; ++a)
+    for (int h = 0; h < 2; ++h) {
 #pragma unroll
-        for (int b = 0; b < RN; ++b) {
-          const int r = i0 + ty + TY * a, c = j0 + tx + TX * b;
-          acc[a][b] = (beta != 0.0 && r < m && c < n) ? ldcg(&C[(size_t)r * ldc + c]) : 0.0;
-        }
-      double ra[AP], rb[BP];
-#define PP_GEMM_FETCH(K0)                                                                                     \
-  do {                                                                                                        \
-    const int k0_ = (K0);                                                                                     \
-    _Pragma("unroll") for (int p = 0; p < AP; ++p) {                                                          \
-      const int e = tid + p * NT;                                                                             \
-      int r, kk;                                                                                              \
-      if (!tA) { r = e / KCH; kk = e % KCH; }                                                                 \
-      else { kk = e / TM; r = e % TM; }                                                                       \
-      double v = 0.0;                                                                                         \
-      if (e < AE && k0_ + kk < k && i0 + r < m)                                                               \
-        v = tA ? ldcg(&A[(size_t)(k0_ + kk) * lda + i0 + r]) : ldcg(&A[(size_t)(i0 + r) * lda + k0_ + kk]);   \
-      ra[p] = v * alpha; /* exact: alpha is +-1 */                                                            \
-    }                                                                                                         \
-    _Pragma("unroll") for (int p = 0; p < BP; ++p) {                                                          \
-      const int e = tid + p * NT;                                                                             \
-      int c, kk;                                                                                              \
-      if (!tB) { kk = e / TN; c = e % TN; }                                                                   \
-      else { c = e / KCH; kk = e % KCH; }                                                                     \
-      double v = 0.0;                                                                                         \
-      if (e < BE && k0_ + kk < k && j0 + c < n)                                                               \
-        v = tB ? ldcg(&B[(size_t)(j0 + c) * ldb + k0_ + kk]) : ldcg(&B[(size_t)(k0_ + kk) * ldb + j0 + c]);   \
-      rb[p] = v;                                                                                              \
-    }                                                                                                         \
-  } while (0)
-      if (nch > 0) PP_GEMM_FETCH(0);
-      for (int ch = 0; ch < nch; ++ch) {
-        __syncthreads();
+      for (int i = 0; i < 2; ++i) av[h][i] = pa[8 * i * GM_LD + 4 * h];
 #pragma unroll
-        for (int p = 0; p < AP; ++p) {
-          const int e = tid + p * NT;
-          if (e < AE) {
-            int r, kk;
-            if (!tA) { r = e / KCH; kk = e % KCH; }
-            else { kk = e / TM; r = e % TM; }
-            As[kk * LA + r] = ra[p];
+      for (int j = 0; j < NW; ++j) bv[h][j] = pb[4 * h * b_ld + 8 * j];
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const double a = flip(av[h][i], sgn);
+#pragma unroll
+        for (int j = 0; j < NW; ++j) dmma(acc[i][j][0], acc[i][j][1], a, bv[h][j]);
+      }
+    pa += 8 * kw;
+    pb += 8 * kw * b_ld;
+  }
+}
+
+__device__ __forceinline__ void dev_gemm(double* __restrict__ C, int ldc, const double* __restrict__ A, int lda, bool tA,
+                                         const double* __restrict__ B, int ldb, bool tB, int m, int n, int k,
+                                         double alpha, double beta, bool free_order) {
+  extern __shared__ __align__(16) double vm_smem[];
+  const int tid = thread_index(), warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3;
+  // tile shape (log2 of TM and TN), this warp's 16 x 16 tile and whether it has the next one too,
+  // and the warps that share a tile's k (free order, outputs of at most four warp tiles)
+  int lm, ln, r1, c1, wide_n = 0, kw = 1, kp = 0;
+  if (n <= 16) { lm = 7; ln = 4; r1 = 16 * warp; c1 = 0; }
+  else if (n <= 32 && m <= 64) { lm = 6; ln = 5; r1 = 16 * (warp & 3); c1 = 16 * (warp >> 2); }
+  else if (n <= 32) { lm = 7; ln = 5; r1 = 16 * warp; c1 = 0; wide_n = 1; }
+  else if (m <= 16) { lm = 4; ln = 6; r1 = 0; c1 = 16 * warp; }
+  else { lm = 6; ln = 6; r1 = 16 * (warp & 3); c1 = 32 * (warp >> 2); wide_n = 1; }
+  if (free_order && m <= 32 && n <= 32 && k >= 64) {
+    const int wt = (m > 16 ? 1 : 0) + (n > 16 ? 1 : 0);  // 2^wt warp tiles
+    lm = 5; ln = 5; wide_n = 0;
+    kw = 8 >> wt;
+    kp = warp >> wt;
+    const int t = warp & ((1 << wt) - 1);
+    r1 = m > 16 ? 16 * (t & 1) : 0;
+    c1 = n > 16 ? 16 * (t >> (wt - 1)) : 0;
+  }
+  const int TM = 1 << lm, TN = 1 << ln, b_ld = TN + 4, AE = TM * GM_LD, sgn = alpha == -1.0 ? (int)0x80000000 : 0;
+  const bool scaled = alpha != 1.0 && alpha != -1.0;  // no generated program; A is scaled in its stage
+  const int nch = (k + GM_KC - 1) / GM_KC, total = ((m + TM - 1) >> lm) * ((n + TN - 1) >> ln) * max(nch, 1);
+  // Staging: warps 0-3 copy A, warps 4-7 copy B.  A thread keeps a column (or an aligned pair) of
+  // its operand as stored and walks down the rows; `krows`: the stored rows run along k.
+  const bool opB = warp >= 4, krows = opB ? !tB : tA;
+  const double* src = opB ? B : A;
+  const int sld = opB ? ldb : lda, osize = opB ? n : m, lo = opB ? ln : lm, lk = log2_of(GM_KC);
+  const bool trans = opB ? tB : tA, wide = !trans && !((sld | (int)(reinterpret_cast<uintptr_t>(src) >> 3)) & 1);
+  const int lp = (krows ? lo : lk) - (wide ? 1 : 0), sc = ((tid & 127) & ((1 << lp) - 1)) << (wide ? 1 : 0);
+  const int sr = (tid & 127) >> lp, sstep = 128 >> lp, dld = opB ? b_ld : GM_LD;
+  const uint32_t sdst = smem_u32(vm_smem) + 8u * (uint32_t)((opB ? AE : 0) + (trans ? sc * dld + sr : sr * dld + sc));
+  const uint32_t ddst = 8u * (uint32_t)(trans ? sstep : sstep * dld);
+  const uint64_t dsrc = 8ull * (uint64_t)((uint32_t)sstep * (uint32_t)sld);
+  const double* sthr = src + (size_t)sr * sld + sc;
+  int pi = 0, pj = 0, pc = 0, ps = 0;  // (tile, chunk) of the next stage to fill, and its slot
+  int i0 = 0, j0 = 0, ch = 0, cs = 0;
+  double acc[2][4][2];
+#pragma unroll 1
+  for (int q = 1 - GM_ST; q < total; ++q) {
+    if (q >= 0) {
+      if (ch == 0) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int r = i0 + r1 + 8 * i + fa, c = j0 + c1 + 2 * fb;
+          const double* p = C + (size_t)r * ldc + c;
+          const bool in = beta != 0.0 && r < m && kp == 0;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            acc[i][j][0] = ldcg_if(p + 8 * j, in && (j < 2 || wide_n) && c + 8 * j < n);
+            acc[i][j][1] = ldcg_if(p + 8 * j + 1, in && (j < 2 || wide_n) && c + 8 * j + 1 < n);
           }
         }
+      }
+      cp_async_wait<GM_ST - 2>();
+      __syncthreads();  // stage q has landed for every thread, and stage q - 1 is free
+    }
+    if (q + GM_ST - 1 < total && nch > 0) {
+      const int o0 = opB ? pj : pi, osz = min(1 << lo, osize - o0), kc = min(GM_KC, k - pc);
+      const int rows = krows ? kc : osz, cols = krows ? osz : kc;
+      const char* sp = reinterpret_cast<const char*>(sthr + (krows ? (size_t)pc * sld + o0 : (size_t)o0 * sld + pc));
+      uint32_t dp = sdst + (uint32_t)ps * (8u * GM_STAGE);
+      if (sc < cols) {
+        int r = sr;
+        if (wide) {
+          const uint32_t v = cols - sc > 1 ? 16u : 8u;
+#pragma unroll 1
+          while (r < rows) copy_rows4<true>(dp, sp, r, ddst, dsrc, sstep, rows, v);
+        } else {
+#pragma unroll 1
+          while (r < rows) copy_rows4<false>(dp, sp, r, ddst, dsrc, sstep, rows, 8u);
+        }
+      }
+      if (kc & 7) {  // k past the end, up to the next multiple of 8, is zero
+        double* st = vm_smem + ps * GM_STAGE;
+        for (int e = tid; e < TM * 8; e += NT)
+          if ((e & 7) >= (kc & 7)) st[(e >> 3) * GM_LD + (kc & ~7) + (e & 7)] = 0.0;
+        for (int e = tid; e < TN * 8; e += NT)
+          if ((e >> ln) >= (kc & 7)) st[AE + ((kc & ~7) + (e >> ln)) * b_ld + (e & (TN - 1))] = 0.0;
+      }
+      ps = ps + 1 == GM_ST ? 0 : ps + 1;
+      pc += GM_KC;
+      if (pc >= k) {
+        pc = 0;
+        pj += TN;
+        if (pj >= n) { pj = 0; pi += TM; }
+      }
+    }
+    cp_async_commit();
+    if (q < 0) continue;
+    if (scaled) {
+      for (int e = tid; e < TM * GM_LD; e += NT) vm_smem[cs * GM_STAGE + e] *= alpha;
+      __syncthreads();
+    }
+    if (nch > 0 && i0 + r1 < m && j0 + c1 < n) {
+      const int passes = (min(GM_KC, k - ch * GM_KC) + 7) >> 3, first = (kp - ch * (GM_KC / 8)) & (kw - 1);
+      const double* st = vm_smem + cs * GM_STAGE;
+      const double *pa = st + (r1 + fa) * GM_LD + fb + 8 * first, *pb = st + AE + (fb + 8 * first) * b_ld + c1 + fa;
+      if (wide_n && j0 + c1 + 16 < n) gemm_passes<4>(acc, pa, pb, b_ld, first, passes, kw, sgn);
+      else gemm_passes<2>(acc, pa, pb, b_ld, first, passes, kw, sgn);
+    }
+    cs = cs + 1 == GM_ST ? 0 : cs + 1;
+    if (++ch >= nch) {
+      if (kw > 1) {  // the k parts of a tile, added in order (one CTA tile only)
+        const int wt = kw == 8 ? 0 : kw == 4 ? 1 : 2;
+        cp_async_wait<0>();
+        __syncthreads();
+        if (kp > 0) {
 #pragma unroll
-        for (int p = 0; p < BP; ++p) {
-          const int e = tid + p * NT;
-          if (e < BE) {
-            int c, kk;
-            if (!tB) { kk = e / TN; c = e % TN; }
-            else { c = e / KCH; kk = e % KCH; }
-            Bs[kk * LB + c] = rb[p];
-          }
+          for (int e = 0; e < 8; ++e) vm_smem[warp * 256 + e * 32 + lane] = acc[e >> 2][(e >> 1) & 1][e & 1];
         }
         __syncthreads();
-        if (ch + 1 < nch) PP_GEMM_FETCH((ch + 1) * KCH);
-        const int kc = min(KCH, k - ch * KCH);
-        for (int kk = 0; kk < kc; ++kk) {
-          double av[RM], bv[RN];
+        if (kp == 0) {
+#pragma unroll 1
+          for (int p = 1; p < kw; ++p)
 #pragma unroll
-          for (int a = 0; a < RM; ++a) av[a] = As[kk * LA + ty + TY * a];
-#pragma unroll
-          for (int b = 0; b < RN; ++b) bv[b] = Bs[kk * LB + tx + TX * b];
-#pragma unroll
-          for (int a = 0; a < RM; ++a)
-#pragma unroll
-            for (int b = 0; b < RN; ++b) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
+            for (int e = 0; e < 8; ++e)
+              acc[e >> 2][(e >> 1) & 1][e & 1] += vm_smem[(warp + (p << wt)) * 256 + e * 32 + lane];
         }
       }
 #pragma unroll
-      for (int a = 0; a < RM; ++a)
+      for (int i = 0; i < 2; ++i) {
+        const int r = i0 + r1 + 8 * i + fa, c = j0 + c1 + 2 * fb;
+        double* p = C + (size_t)r * ldc + c;
+        const bool in = r < m && kp == 0;
 #pragma unroll
-        for (int b = 0; b < RN; ++b) {
-          const int r = i0 + ty + TY * a, c = j0 + tx + TX * b;
-          if (r < m && c < n) C[(size_t)r * ldc + c] = acc[a][b];
+        for (int j = 0; j < 4; ++j) {
+          st_if(p + 8 * j, acc[i][j][0], in && (j < 2 || wide_n) && c + 8 * j < n);
+          st_if(p + 8 * j + 1, acc[i][j][1], in && (j < 2 || wide_n) && c + 8 * j + 1 < n);
         }
-    }
-  __syncthreads();
-}
-
-// C[m x n] (m, n <= 16) = beta C + alpha op(A) op(B) for a long k, in free order: each warp
-// sums a contiguous k slice (ascending, 8 outputs per lane), the slices are then added in
-// warp order.  Deterministic, but not the reference's single ascending chain per element.
-__device__ __noinline__ void gemm_splitk(double* __restrict__ C, int ldc, const double* __restrict__ A, int lda,
-                                         bool tA, const double* __restrict__ B, int ldb, bool tB, int m, int n, int k,
-                                         double alpha, double beta, double* smem) {
-  constexpr int KW = 16, NW = NT / 32, LW = 17;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* As = smem + w * (2 * KW * LW);  // [KW][LW] (kk, r), this warp's
-  double* Bs = As + KW * LW;              // [KW][LW] (kk, c)
-  const int kseg = (k + NW - 1) / NW;
-  const int kb = min(k, w * kseg), ke = min(k, kb + kseg);
-  const int c_out = lane & 15;
-  double acc[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) acc[q] = 0.0;
-  double ra[8], rb[8];
-#define PP_SPLITK_FETCH(K0)                                                                                   \
-  do {                                                                                                        \
-    const int k0_ = (K0);                                                                                     \
-    _Pragma("unroll") for (int p = 0; p < 8; ++p) {                                                           \
-      const int e = lane + 32 * p;                                                                            \
-      const int kk = tA ? (e >> 4) : (e & 15), r = tA ? (e & 15) : (e >> 4);                                  \
-      double v = 0.0;                                                                                         \
-      if (r < m && k0_ + kk < ke)                                                                             \
-        v = tA ? ldcg(&A[(size_t)(k0_ + kk) * lda + r]) : ldcg(&A[(size_t)r * lda + k0_ + kk]);               \
-      ra[p] = v * alpha;                                                                                      \
-      const int kb_ = tB ? (e & 15) : (e >> 4), c = tB ? (e >> 4) : (e & 15);                                 \
-      double u = 0.0;                                                                                         \
-      if (c < n && k0_ + kb_ < ke)                                                                            \
-        u = tB ? ldcg(&B[(size_t)c * ldb + k0_ + kb_]) : ldcg(&B[(size_t)(k0_ + kb_) * ldb + c]);            \
-      rb[p] = u;                                                                                              \
-    }                                                                                                         \
-  } while (0)
-  if (kb < ke) PP_SPLITK_FETCH(kb);
-  for (int k0 = kb; k0 < ke; k0 += KW) {
-#pragma unroll
-    for (int p = 0; p < 8; ++p) {
-      const int e = lane + 32 * p;
-      As[(tA ? (e >> 4) : (e & 15)) * LW + (tA ? (e & 15) : (e >> 4))] = ra[p];
-      Bs[(tB ? (e & 15) : (e >> 4)) * LW + (tB ? (e >> 4) : (e & 15))] = rb[p];
-    }
-    __syncwarp();
-    if (k0 + KW < ke) PP_SPLITK_FETCH(k0 + KW);
-    const int kc = min(KW, ke - k0);
-    for (int kk = 0; kk < kc; ++kk) {
-      const double b = Bs[kk * LW + c_out];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) acc[q] = fma(As[kk * LW + ((lane + 32 * q) >> 4)], b, acc[q]);
-    }
-    __syncwarp();
-  }
-#undef PP_SPLITK_FETCH
-  __syncthreads();
-  double* red = smem;  // [NW][256] partial sums, output o = r * 16 + c
-#pragma unroll
-  for (int q = 0; q < 8; ++q) red[w * 256 + lane + 32 * q] = acc[q];
-  __syncthreads();
-  {
-    const int o = threadIdx.x, r = o >> 4, c = o & 15;
-    if (r < m && c < n) {
-      double s = red[o];
-      for (int ww = 1; ww < NW; ++ww) s += red[ww * 256 + o];
-      double* p = &C[(size_t)r * ldc + c];
-      *p = beta != 0.0 ? ldcg(p) + s : s;
+      }
+      ch = 0;
+      j0 += TN;
+      if (j0 >= n) { j0 = 0; i0 += TM; }
     }
   }
-  __syncthreads();
-}
-
-// C[1 x n] (n <= 32) = beta C + alpha op(A)[1 x k] op(B)[k x n] in free order (a row vector
-// times a tall skinny matrix, e.g. x^T V in a solve): thread t sums k = t, t + NT, ... into
-// n partial sums, then warps and the CTA reduce them.
-__device__ __noinline__ void gemv_row(double* __restrict__ C, const double* __restrict__ A, int lda, bool tA,
-                                      const double* __restrict__ B, int ldb, bool tB, int n, int k, double alpha,
-                                      double beta, double* smem) {
-  constexpr int NC = 32;
-  double acc[NC];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) acc[c] = 0.0;
-#pragma unroll 2
-  for (int kk = threadIdx.x; kk < k; kk += NT) {
-    const double a = tA ? ldcg(&A[(size_t)kk * lda]) : ldcg(&A[kk]);
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-      if (c < n) acc[c] = fma(a, tB ? ldcg(&B[(size_t)c * ldb + kk]) : ldcg(&B[(size_t)kk * ldb + c]), acc[c]);
-  }
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    if (c < n) {
-      double v = acc[c];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) smem[w * NC + c] = v;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < n) {
-    double v = 0.0;
-    for (int q = 0; q < NT / 32; ++q) v += smem[q * NC + threadIdx.x];
-    v *= alpha;
-    C[threadIdx.x] = beta != 0.0 ? ldcg(&C[threadIdx.x]) + v : v;
-  }
+  cp_async_wait<0>();
   __syncthreads();
 }
 
 template <int NB, int RU, int TC>
 __device__ __noinline__ void trmv_impl(double* O, int ldo, const double* S, int lds, const double* M, int ldm, int m,
-                                       int n, int mode, int rbeg, int rows, double* smem, double alpha = 1.0,
-                                       double beta = 0.0);
-
-__device__ __forceinline__ void dev_gemm(double* __restrict__ C, int ldc, const double* __restrict__ A, int lda, bool tA,
-                         const double* __restrict__ B, int ldb, bool tB, int m, int n, int k, double alpha,
-                         double beta, double* smem, bool free_order = false) {
-  if (free_order && m == 1 && n <= 32 && k >= 64)
-    gemv_row(C, A, lda, tA, B, ldb, tB, n, k, alpha, beta, smem);
-  else if (free_order && !tA && !tB && m > 16 && n <= 16 && k >= 64 && k <= 512) {
-    // rows of A times a skinny B (the solves' products): B staged in shared memory, warps take
-    // rows of A with lanes along k and every load of a row batch issued first, a warp reduction
-    // per row and column; no per-element ascending-k order (work and right-hand-side targets)
-    if (k <= 256) {
-      if (n <= 4) trmv_impl<4, 4, 8>(C, ldc, B, ldb, A, lda, k, n, 2, 0, m, smem, alpha, beta);
-      else if (n <= 8) trmv_impl<8, 2, 8>(C, ldc, B, ldb, A, lda, k, n, 2, 0, m, smem, alpha, beta);
-      else trmv_impl<16, 2, 8>(C, ldc, B, ldb, A, lda, k, n, 2, 0, m, smem, alpha, beta);
-    } else {
-      if (n <= 4) trmv_impl<4, 2, 16>(C, ldc, B, ldb, A, lda, k, n, 2, 0, m, smem, alpha, beta);
-      else if (n <= 8) trmv_impl<8, 2, 16>(C, ldc, B, ldb, A, lda, k, n, 2, 0, m, smem, alpha, beta);
-      else trmv_impl<16, 1, 16>(C, ldc, B, ldb, A, lda, k, n, 2, 0, m, smem, alpha, beta);
-    }
-  }
-  else if (free_order && m <= 16 && n <= 16 && k >= 256)
-    gemm_splitk(C, ldc, A, lda, tA, B, ldb, tB, m, n, k, alpha, beta, smem);
-  else if (m <= 16 && n <= 16) gemm_cfg<16, 16, 1, 1, 128>(C, ldc, A, lda, tA, B, ldb, tB, m, n, k, alpha, beta, smem);
-  else if (m <= 32 && n <= 32) gemm_cfg<32, 32, 2, 2, 64>(C, ldc, A, lda, tA, B, ldb, tB, m, n, k, alpha, beta, smem);
-  else if (n == 1) gemm_cfg<256, 1, 1, 1, 16>(C, ldc, A, lda, tA, B, ldb, tB, m, n, k, alpha, beta, smem);
-  else if (n <= 16) gemm_cfg<128, 16, 8, 1, 32>(C, ldc, A, lda, tA, B, ldb, tB, m, n, k, alpha, beta, smem);
-  else if (m <= 16) gemm_cfg<16, 128, 1, 8, 32>(C, ldc, A, lda, tA, B, ldb, tB, m, n, k, alpha, beta, smem);
-  // tall or wide skinny products over a long k (a dense block times a low-rank factor): 10 loads
-  // in flight per thread, 16 FMAs per thread and k step
-  else if (n <= 32 && m >= 128) gemm_cfg<128, 32, 4, 4, 16>(C, ldc, A, lda, tA, B, ldb, tB, m, n, k, alpha, beta, smem);
-  else if (m <= 32 && n >= 128) gemm_cfg<32, 128, 4, 4, 16>(C, ldc, A, lda, tA, B, ldb, tB, m, n, k, alpha, beta, smem);
-  else if (m > 64 && n > 64) gemm_cfg<128, 128, 8, 8, 16>(C, ldc, A, lda, tA, B, ldb, tB, m, n, k, alpha, beta, smem);
-  else gemm_cfg<64, 64, 4, 4, 32>(C, ldc, A, lda, tA, B, ldb, tB, m, n, k, alpha, beta, smem);
-}
+                                       int n, int mode, int rbeg, int rows, double* smem);
 
 // ------------------------------------------------------------------------- tensor-core GEMM
 // Mixed-precision contraction on the 5th-generation tensor cores:
@@ -344,8 +378,6 @@ struct TcCtx {
   uint32_t u;
   int* abort;
 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
@@ -1208,67 +1240,10 @@ __device__ __noinline__ void dev_trsmr(double* B, int ldb, const double* U, int 
   __syncthreads();
 }
 
-// Triangular solves on blocks up to 4 x TL rows, inside one CTA: diagonal TL-blocks by the
-// routines above, the coupling between blocks by ordered GEMMs.  Every element gets the same
-// update sequence as the tiled DAG would apply (i ascending), so results are identical.
-__device__ __noinline__ void dev_trsml_big(double* B, int ldb, const double* L, int ldl, int m, int n, double* smem) {
-  for (int d = 0; d < m; d += TL) {
-    const int md = min(TL, m - d);
-    dev_trsml(B + (size_t)d * ldb, ldb, L + (size_t)d * ldl + d, ldl, md, n, smem);
-    if (d + md < m)  // B_below -= L(below, d) B_d
-      dev_gemm(B + (size_t)(d + md) * ldb, ldb, L + (size_t)(d + md) * ldl + d, ldl, false, B + (size_t)d * ldb, ldb,
-               false, m - d - md, n, md, -1.0, 1.0, smem);
-  }
-}
-
-__device__ __noinline__ void dev_trsmu_big(double* B, int ldb, const double* U, int ldu, int m, int n, double* smem) {
-  const int nb = (m + TL - 1) / TL;
-  for (int bi = nb - 1; bi >= 0; --bi) {
-    const int d = bi * TL, md = min(TL, m - d);
-    dev_trsmu(B + (size_t)d * ldb, ldb, U + (size_t)d * ldu + d, ldu, md, n, smem);
-    if (d > 0)  // B_above -= U(above, d) B_d
-      dev_gemm(B, ldb, U + d, ldu, false, B + (size_t)d * ldb, ldb, false, d, n, md, -1.0, 1.0, smem);
-  }
-}
-
-__device__ __noinline__ void dev_trsmr_big(double* B, int ldb, const double* U, int ldu, int m, int n, double* smem) {
-  for (int d = 0; d < n; d += TL) {
-    const int nd = min(TL, n - d);
-    dev_trsmr(B + d, ldb, U + (size_t)d * ldu + d, ldu, m, nd, smem);
-    if (d + nd < n)  // B(:, right) -= B_d U(d, right)
-      dev_gemm(B + d + nd, ldb, B + d, ldb, false, U + (size_t)d * ldu + d + nd, ldu, false, m, n - d - nd, nd, -1.0,
-               1.0, smem);
-  }
-}
-
-__device__ __noinline__ void dev_trsmrt_big(double* V, int ldv, const double* U, int ldu, int m, int n, double* smem) {
-  for (int d = 0; d < m; d += TL) {
-    const int md = min(TL, m - d);
-    dev_trsmrt(V + (size_t)d * ldv, ldv, U + (size_t)d * ldu + d, ldu, md, n, smem);
-    if (d + md < m)  // V_below -= U(d, below)^T V_d
-      dev_gemm(V + (size_t)(d + md) * ldv, ldv, U + (size_t)d * ldu + d + md, ldu, true, V + (size_t)d * ldv, ldv,
-               false, m - d - md, n, md, -1.0, 1.0, smem);
-  }
-}
-
 // ------------------------------------------------------------------------- TRINV / TRMV
 // Explicit inverses of a factored diagonal leaf (factor phase) and their application (solve
 // phase).  A solve then costs one triangular matrix-vector product per leaf, whose loads are
 // all independent, instead of a substitution whose steps form a chain.
-
-// Columns [c0, c0 + w) of L^-1 (upper = 0) or U^-1 (upper = 1), A = L\U (m x m, ld lda),
-// into I (the column block, m x w, ld ldi): identity columns, then the blocked sweep on the
-// sub-triangle the block needs (rows c0.. of L^-1 are the only nonzeros; rows ..c0+w of U^-1).
-__device__ __noinline__ void dev_trinv(double* I, int ldi, const double* A, int lda, int m, int w, int c0, int upper,
-                                       double* smem) {
-  for (int e = threadIdx.x; e < m * w; e += NT) {
-    const int r = e / w, j = e % w;
-    I[(size_t)r * ldi + j] = r == c0 + j ? 1.0 : 0.0;
-  }
-  __syncthreads();
-  if (!upper) dev_trsml_big(I + (size_t)c0 * ldi, ldi, A + (size_t)c0 * lda + c0, lda, m - c0, w, smem);
-  else dev_trsmu_big(I, ldi, A, lda, c0 + w, w, smem);
-}
 
 // Rows [r0, r0 + rows) of M S into O (row r at O row r - r0), M (m x m, m <= 32 TC) lower
 // (mode 0) or upper (mode 1) triangular or full (mode 2, then any number of rows), S (m x n);
@@ -1278,8 +1253,7 @@ __device__ __noinline__ void dev_trinv(double* I, int ldi, const double* A, int 
 // dot products, so a row's result does not depend on which rows the call covers.
 template <int NB, int RU, int TC>
 __device__ __noinline__ void trmv_impl(double* O, int ldo, const double* S, int lds, const double* M, int ldm, int m,
-                                       int n, int mode, int rbeg, int rows, double* smem, double alpha,
-                                       double beta) {
+                                       int n, int mode, int rbeg, int rows, double* smem) {
   // S staged as m rows of NB values, row stride NB + 1 for NB > 1: the lanes of a warp read
   // consecutive rows, which then fall in distinct shared-memory banks
   constexpr int SB = NB > 1 ? NB + 1 : 1;
@@ -1324,8 +1298,7 @@ __device__ __noinline__ void trmv_impl(double* O, int ldo, const double* S, int 
 #pragma unroll
         for (int q = 0; q < NB; ++q)
           if (q < n) {
-            double* o = &O[(size_t)(r - rbeg) * ldo + q];
-            *o = beta != 0.0 ? fma(alpha, acc[q], ldcg(o)) : alpha * acc[q];
+            O[(size_t)(r - rbeg) * ldo + q] = acc[q];
           }
       }
     }
@@ -1355,56 +1328,184 @@ __device__ __forceinline__ bool dev_trmv(const pp_task& T, double* smem) {
   return true;
 }
 
-// ------------------------------------------------------------------------- GEMM3 / GEMM4
-// Reference association orders (kernel.cu:886-955), intermediates in task scratch.
-__device__ __noinline__ void dev_gemm3(const pp_task& T, double* smem) {
-  const bool tA = T.flags & PP_T(1), tB = T.flags & PP_T(2), tC = T.flags & PP_T(3);
-  double* t1 = T.tmp;
-  const int m = T.m, n = T.n, k = T.k, l = T.l;
-  if (T.ctrl) {  // (A B) C, t1: m x l
-    dev_gemm(t1, l, T.p[1], T.ld[1], tA, T.p[2], T.ld[2], tB, m, l, k, 1.0, 0.0, smem);
-    dev_gemm(T.p[0], T.ld[0], t1, l, false, T.p[3], T.ld[3], tC, m, n, l, T.alpha, 1.0, smem);
-  } else {       // A (B C), t1: k x n
-    dev_gemm(t1, n, T.p[2], T.ld[2], tB, T.p[3], T.ld[3], tC, k, n, l, 1.0, 0.0, smem);
-    dev_gemm(T.p[0], T.ld[0], T.p[1], T.ld[1], tA, t1, n, false, m, n, k, T.alpha, 1.0, smem);
-  }
-}
+// ------------------------------------------------------------------------- composite instructions
+// Instructions made of triangular solves on TL-blocks and of products: the VM has one copy of the
+// product's code, so each of them is walked as a sequence of such steps.
 
-__device__ __noinline__ void dev_gemm4(const pp_task& T, double* smem) {
-  const bool tA = T.flags & PP_T(1), tB = T.flags & PP_T(2), tC = T.flags & PP_T(3), tD = T.flags & PP_T(4);
-  const double *A = T.p[1], *B = T.p[2], *Cm = T.p[3], *D = T.p[4];
-  const int la = T.ld[1], lb = T.ld[2], lc = T.ld[3], ld = T.ld[4];
+// One product of the reference's association orders of GEMM3 / GEMM4 (kernel.cu:886-955): step 0,
+// 1 (, 2) of the instruction, intermediates t1 (and t2) in task scratch.
+struct Product {
+  double* C;
+  const double *A, *B;
+  int ldc, lda, ldb, m, n, k;
+  bool tA, tB;
+  double alpha, beta;
+};
+
+__device__ __forceinline__ bool chain_step(const pp_task& T, int step, Product& P) {
   const int m = T.m, n = T.n, k = T.k, l = T.l, o = T.o;
-  double* t1 = T.tmp;
-  double* t2 = T.tmp + T.aux;  // second intermediate (reference gemm_4x `offset`)
-  double* M = T.p[0];
-  const int lm = T.ld[0];
+  double *t1 = T.tmp, *t2 = T.tmp + T.aux;  // second intermediate (reference gemm_4x `offset`)
+  auto operand = [&](int i, const double*& p, int& ld, bool& t) {
+    p = T.p[i];
+    ld = T.ld[i];
+    t = (T.flags & PP_T(i)) != 0;
+  };
+  auto work = [&](const double* w, int wld, const double*& p, int& ld, bool& t) {
+    p = w;
+    ld = wld;
+    t = false;
+  };
+  auto target = [&](double* c, int ldc, int mm, int nn, int kk, bool last) {
+    P.C = c;
+    P.ldc = ldc;
+    P.m = mm;
+    P.n = nn;
+    P.k = kk;
+    P.alpha = last ? T.alpha : 1.0;
+    P.beta = last ? 1.0 : 0.0;
+  };
+  if (T.op == PP_OP_GEMM) {
+    if (step > 0) return false;
+    operand(1, P.A, P.lda, P.tA);
+    operand(2, P.B, P.ldb, P.tB);
+    target(T.p[0], T.ld[0], m, n, k, true);
+    P.beta = T.beta;
+    return true;
+  }
+  if (T.op == PP_OP_GEMM3) {
+    if (step > 1) return false;
+    if (T.ctrl) {  // (A B) C, t1: m x l
+      if (step == 0) { operand(1, P.A, P.lda, P.tA); operand(2, P.B, P.ldb, P.tB); target(t1, l, m, l, k, false); }
+      else { work(t1, l, P.A, P.lda, P.tA); operand(3, P.B, P.ldb, P.tB); target(T.p[0], T.ld[0], m, n, l, true); }
+    } else {       // A (B C), t1: k x n
+      if (step == 0) { operand(2, P.A, P.lda, P.tA); operand(3, P.B, P.ldb, P.tB); target(t1, n, k, n, l, false); }
+      else { operand(1, P.A, P.lda, P.tA); work(t1, n, P.B, P.ldb, P.tB); target(T.p[0], T.ld[0], m, n, k, true); }
+    }
+    return true;
+  }
+  if (step > 2) return false;
   switch (T.ctrl) {
     case 0:  // ((A B) C) D; t1 m x l, t2 m x o
-      dev_gemm(t1, l, A, la, tA, B, lb, tB, m, l, k, 1.0, 0.0, smem);
-      dev_gemm(t2, o, t1, l, false, Cm, lc, tC, m, o, l, 1.0, 0.0, smem);
-      dev_gemm(M, lm, t2, o, false, D, ld, tD, m, n, o, T.alpha, 1.0, smem);
+      if (step == 0) { operand(1, P.A, P.lda, P.tA); operand(2, P.B, P.ldb, P.tB); target(t1, l, m, l, k, false); }
+      else if (step == 1) { work(t1, l, P.A, P.lda, P.tA); operand(3, P.B, P.ldb, P.tB); target(t2, o, m, o, l, false); }
+      else { work(t2, o, P.A, P.lda, P.tA); operand(4, P.B, P.ldb, P.tB); target(T.p[0], T.ld[0], m, n, o, true); }
       break;
     case 1:  // (A (B C)) D; t1 k x o, t2 m x o
-      dev_gemm(t1, o, B, lb, tB, Cm, lc, tC, k, o, l, 1.0, 0.0, smem);
-      dev_gemm(t2, o, A, la, tA, t1, o, false, m, o, k, 1.0, 0.0, smem);
-      dev_gemm(M, lm, t2, o, false, D, ld, tD, m, n, o, T.alpha, 1.0, smem);
+      if (step == 0) { operand(2, P.A, P.lda, P.tA); operand(3, P.B, P.ldb, P.tB); target(t1, o, k, o, l, false); }
+      else if (step == 1) { operand(1, P.A, P.lda, P.tA); work(t1, o, P.B, P.ldb, P.tB); target(t2, o, m, o, k, false); }
+      else { work(t2, o, P.A, P.lda, P.tA); operand(4, P.B, P.ldb, P.tB); target(T.p[0], T.ld[0], m, n, o, true); }
       break;
     case 2:  // A ((B C) D); t1 k x o, t2 k x n
-      dev_gemm(t1, o, B, lb, tB, Cm, lc, tC, k, o, l, 1.0, 0.0, smem);
-      dev_gemm(t2, n, t1, o, false, D, ld, tD, k, n, o, 1.0, 0.0, smem);
-      dev_gemm(M, lm, A, la, tA, t2, n, false, m, n, k, T.alpha, 1.0, smem);
+      if (step == 0) { operand(2, P.A, P.lda, P.tA); operand(3, P.B, P.ldb, P.tB); target(t1, o, k, o, l, false); }
+      else if (step == 1) { work(t1, o, P.A, P.lda, P.tA); operand(4, P.B, P.ldb, P.tB); target(t2, n, k, n, o, false); }
+      else { operand(1, P.A, P.lda, P.tA); work(t2, n, P.B, P.ldb, P.tB); target(T.p[0], T.ld[0], m, n, k, true); }
       break;
     case 3:  // A (B (C D)); t1 l x n, t2 k x n
-      dev_gemm(t1, n, Cm, lc, tC, D, ld, tD, l, n, o, 1.0, 0.0, smem);
-      dev_gemm(t2, n, B, lb, tB, t1, n, false, k, n, l, 1.0, 0.0, smem);
-      dev_gemm(M, lm, A, la, tA, t2, n, false, m, n, k, T.alpha, 1.0, smem);
+      if (step == 0) { operand(3, P.A, P.lda, P.tA); operand(4, P.B, P.ldb, P.tB); target(t1, n, l, n, o, false); }
+      else if (step == 1) { operand(2, P.A, P.lda, P.tA); work(t1, n, P.B, P.ldb, P.tB); target(t2, n, k, n, l, false); }
+      else { operand(1, P.A, P.lda, P.tA); work(t2, n, P.B, P.ldb, P.tB); target(T.p[0], T.ld[0], m, n, k, true); }
       break;
     default:  // 4: (A B) (C D); t1 m x l, t2 l x n
-      dev_gemm(t1, l, A, la, tA, B, lb, tB, m, l, k, 1.0, 0.0, smem);
-      dev_gemm(t2, n, Cm, lc, tC, D, ld, tD, l, n, o, 1.0, 0.0, smem);
-      dev_gemm(M, lm, t1, l, false, t2, n, false, m, n, l, T.alpha, 1.0, smem);
+      if (step == 0) { operand(1, P.A, P.lda, P.tA); operand(2, P.B, P.ldb, P.tB); target(t1, l, m, l, k, false); }
+      else if (step == 1) { operand(3, P.A, P.lda, P.tA); operand(4, P.B, P.ldb, P.tB); target(t2, n, l, n, o, false); }
+      else { work(t1, l, P.A, P.lda, P.tA); work(t2, n, P.B, P.ldb, P.tB); target(T.p[0], T.ld[0], m, n, l, true); }
       break;
+  }
+  return true;
+}
+
+// One step of a triangular solve with a triangle of `size` rows, op one of the TRSM* kinds: even
+// steps solve a diagonal TL-block (triangle *t at offset d in both), odd ones couple it to the rest.
+// Every element gets the update sequence the tiled DAG would apply (i ascending), so results are
+// identical.
+__device__ __forceinline__ bool tri_step(int op, double* B, int ldb, const double* T, int ldt, int size, int lines,
+                                         int step, int& d, int& len, Product& P) {
+  const int nb = (size + TL - 1) / TL, at = step >> 1;
+  if (at >= nb) return false;
+  const int b = op == PP_OP_TRSMU ? nb - 1 - at : at;
+  d = b * TL;
+  len = min(TL, size - d);
+  if (!(step & 1)) return true;
+  const int e = d + len, rest = op == PP_OP_TRSMU ? d : size - e;
+  if (rest <= 0) return false;
+  P.alpha = -1.0;
+  P.beta = 1.0;
+  P.ldc = ldb;
+  P.k = len;
+  P.tA = P.tB = false;
+  if (op == PP_OP_TRSMR) {  // B(:, right) -= B_d U(d, right)
+    P.C = B + e;
+    P.A = B + d;
+    P.lda = ldb;
+    P.B = T + (size_t)d * ldt + e;
+    P.ldb = ldt;
+    P.m = lines;
+    P.n = rest;
+    return true;
+  }
+  P.B = B + (size_t)d * ldb;
+  P.ldb = ldb;
+  P.lda = ldt;
+  P.m = rest;
+  P.n = lines;
+  if (op == PP_OP_TRSML) {  // B_below -= L(below, d) B_d
+    P.C = B + (size_t)e * ldb;
+    P.A = T + (size_t)e * ldt + d;
+  } else if (op == PP_OP_TRSMRT) {  // V_below -= U(d, below)^T V_d
+    P.C = B + (size_t)e * ldb;
+    P.A = T + (size_t)d * ldt + e;
+    P.tA = true;
+  } else {  // B_above -= U(above, d) B_d
+    P.C = B;
+    P.A = T + d;
+  }
+  return true;
+}
+
+__device__ __forceinline__ void run_composite(const pp_task& T, double* smem) {
+  const bool product = T.op == PP_OP_GEMM || T.op == PP_OP_GEMM3 || T.op == PP_OP_GEMM4;
+  const bool free_order = T.op == PP_OP_GEMM && (T.flags & PP_FREE_ORDER);
+  int op = T.op, size = T.op == PP_OP_TRSMR ? T.n : T.m, lines = T.op == PP_OP_TRSMR ? T.m : T.n;
+  double* B = T.p[0];
+  const double* A = T.p[1];
+  const int ldb = T.ld[0], lda = T.ld[1];
+  if (T.op == PP_OP_TRINV) {
+    // columns [o, o + n) of L^-1 (ctrl 0) or U^-1 (1): identity columns, then the solve on the
+    // sub-triangle they need (rows o.. of L^-1 are the only nonzeros; rows ..o + n of U^-1)
+    const int w = T.n, c0 = T.o;
+    for (int e = threadIdx.x; e < T.m * w; e += NT) {
+      const int r = e / w, j = e % w;
+      B[(size_t)r * ldb + j] = r == c0 + j ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    op = T.ctrl ? PP_OP_TRSMU : PP_OP_TRSML;
+    size = T.ctrl ? c0 + w : T.m - c0;
+    lines = w;
+    if (!T.ctrl) {
+      B += (size_t)c0 * ldb;
+      A += (size_t)c0 * lda + c0;
+    }
+  }
+#pragma unroll 1
+  for (int step = 0;; ++step) {
+    Product P;
+    if (product) {
+      if (!chain_step(T, step, P)) break;
+    } else {
+      int d = 0, len = 0;
+      if (!tri_step(op, B, ldb, A, lda, size, lines, step, d, len, P)) break;
+      if (!(step & 1)) {
+        const double* D = A + (size_t)d * lda + d;
+        switch (op) {
+          case PP_OP_TRSML: dev_trsml(B + (size_t)d * ldb, ldb, D, lda, len, lines, smem); break;
+          case PP_OP_TRSMRT: dev_trsmrt(B + (size_t)d * ldb, ldb, D, lda, len, lines, smem); break;
+          case PP_OP_TRSMR: dev_trsmr(B + d, ldb, D, lda, lines, len, smem); break;
+          default: dev_trsmu(B + (size_t)d * ldb, ldb, D, lda, len, lines, smem); break;
+        }
+        continue;
+      }
+    }
+    dev_gemm(P.C, P.ldc, P.A, P.lda, P.tA, P.B, P.ldb, P.tB, P.m, P.n, P.k, P.alpha, P.beta, free_order);
   }
 }
 
@@ -1546,12 +1647,6 @@ __device__ __noinline__ void accum_tn(const double* X, int lx, int a, const doub
 // A (8 x 4) lane l holds A[l/4][l%4]; B (4 x 8) holds B[l%4][l/4]; C (8 x 8) holds
 // C[l/4][2(l%4) + {0,1}].  Rows are taken four at a time (one k step), several k steps of
 // loads issued before their products.  Warp partials are combined as in accum_tn (fixed order).
-__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
-}
-
 template <int KB, bool XG, bool WG>
 __device__ __noinline__ void accum_tn_mma(const double* X, int lx, int a, const double* W1, int lw1, int b1,
                                           const double* W2, int lw2, int b2, int L, double* out1, double* out2,
@@ -2109,24 +2204,14 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
         return true;
       }
       if (T.m > PP_VM_TRI) return false;
-      if (T.m > TL) dev_trsml_big(T.p[0], T.ld[0], T.p[1], T.ld[1], T.m, T.n, smem);
-      else dev_trsml(T.p[0], T.ld[0], T.p[1], T.ld[1], T.m, T.n, smem);
-      return true;
+      break;
     case PP_OP_TRSMR:
       if (T.n > PP_VM_TRI) return false;
-      if (T.n > TL) dev_trsmr_big(T.p[0], T.ld[0], T.p[1], T.ld[1], T.m, T.n, smem);
-      else dev_trsmr(T.p[0], T.ld[0], T.p[1], T.ld[1], T.m, T.n, smem);
-      return true;
+      break;
     case PP_OP_TRSMRT:
-      if (T.m > PP_VM_TRI) return false;
-      if (T.m > TL) dev_trsmrt_big(T.p[0], T.ld[0], T.p[1], T.ld[1], T.m, T.n, smem);
-      else dev_trsmrt(T.p[0], T.ld[0], T.p[1], T.ld[1], T.m, T.n, smem);
-      return true;
     case PP_OP_TRSMU:
       if (T.m > PP_VM_TRI) return false;
-      if (T.m > TL) dev_trsmu_big(T.p[0], T.ld[0], T.p[1], T.ld[1], T.m, T.n, smem);
-      else dev_trsmu(T.p[0], T.ld[0], T.p[1], T.ld[1], T.m, T.n, smem);
-      return true;
+      break;
     case PP_OP_GEMM:
       if (T.prec == PP_PREC_BF16) {
         if (!tc.active || T.m < 128 || T.m % 128 || T.k < 64 || T.k % 64 || T.l < 0 || T.l % 64 ||
@@ -2146,11 +2231,9 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
           err = PP_VM_MMA_TIMEOUT;
         return true;
       }
-      dev_gemm(T.p[0], T.ld[0], T.p[1], T.ld[1], T.flags & PP_T(1), T.p[2], T.ld[2], T.flags & PP_T(2), T.m, T.n,
-               T.k, T.alpha, T.beta, smem, (T.flags & PP_FREE_ORDER) != 0);
-      return true;
-    case PP_OP_GEMM3: dev_gemm3(T, smem); return true;
-    case PP_OP_GEMM4: dev_gemm4(T, smem); return true;
+      break;
+    case PP_OP_GEMM3:
+    case PP_OP_GEMM4: break;
     case PP_OP_ACCUM:
       if (T.k > PP_VM_MAX_RANK || T.k < 1 || T.l > PP_VM_MAX_RANK || T.l < 0) return false;
       dev_accum(T, smem);
@@ -2160,8 +2243,7 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
       return true;
     case PP_OP_TRINV:
       if (T.m > PP_VM_INV || T.n < 1 || T.o < 0 || T.o + T.n > T.m) return false;
-      dev_trinv(T.p[0], T.ld[0], T.p[1], T.ld[1], T.m, T.n, T.o, T.ctrl, smem);
-      return true;
+      break;
     case PP_OP_TRMV: return dev_trmv(T, smem);
     case PP_OP_ORTH:
       if (T.n < 1 || T.n > PP_VM_MAX_RANK || T.ld[0] != T.n) return false;
@@ -2189,6 +2271,8 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
       return true;
     default: return false;
   }
+  run_composite(T, smem);
+  return true;
 }
 
 __global__ void vm_init(const int32_t* __restrict__ indeg, const int32_t* __restrict__ ready, int n_ready, int n,
@@ -2217,7 +2301,7 @@ __device__ __forceinline__ unsigned smid() {
 __global__ void __launch_bounds__(NT, 1)
     vm_kernel(const pp_task* __restrict__ tasks, int n_tasks, const int32_t* __restrict__ succ, int32_t* counters,
               int32_t* slots, pp_vm_state* st, long long wait_ns, unsigned long long* trace, int use_tc) {
-  extern __shared__ double smem[];
+  extern __shared__ __align__(16) double smem[];
   __shared__ __align__(16) pp_task s_task;
   __shared__ int s_id;
   __shared__ int s_keep;  // position (in the successor list) of the successor run next
@@ -2916,7 +3000,7 @@ __global__ void absmax2_kernel(const double* __restrict__ x, const double* __res
 
 // One ACCUM on caller buffers; its scratch (T.tmp) is the static array below.
 __global__ void __launch_bounds__(NT) accum_noalloc_kernel(pp_task T) {
-  extern __shared__ double smem[];
+  extern __shared__ __align__(16) double smem[];
   dev_accum(T, smem);
 }
 
