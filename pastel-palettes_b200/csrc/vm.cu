@@ -889,24 +889,37 @@ __device__ __noinline__ bool dev_gemm_bf16(double* __restrict__ C, int ldc, cons
   return ok;
 }
 
-// ------------------------------------------------------------------------- tiles in smem
-// rows x cols (<= TL x TL) from global (L2) into S (ld LDS); every thread issues its up to
-// sixteen loads before it stores any, so a tile costs one memory latency, not sixteen
-__device__ void load_tile(double* S, const double* __restrict__ G, int ld, int rows, int cols) {
-  const int total = rows * cols;
-  for (int e0 = 0; e0 < total; e0 += 16 * NT) {
-    double v[16];
-#pragma unroll
-    for (int p = 0; p < 16; ++p) {
-      const int e = e0 + threadIdx.x + p * NT;
-      v[p] = e < total ? ldcg(&G[(size_t)(e / cols) * ld + e % cols]) : 0.0;
-    }
-#pragma unroll
-    for (int p = 0; p < 16; ++p) {
-      const int e = e0 + threadIdx.x + p * NT;
-      if (e < total) S[(e / cols) * LDS + e % cols] = v[p];
-    }
-  }
+// ------------------------------------------------------------------------- quotients
+// A division takes 128 cycles of dependent work on this chip, and the triangular routines have one
+// per row on their critical path.  These are the same correctly rounded quotients from published
+// iterations (P. Markstein, Computation of elementary functions on the IBM RISC System/6000, 1990):
+// a reciprocal estimate (special-function unit, about 20 bits) is brought to RN(1 / t) by a
+// third-order and a second-order step, and with y = RN(1 / t) two corrections q += (x - t q) y of
+// q = RN(x y), the residual exact in an fma, leave RN(x / t), as long as nothing over- or underflows.
+// quotient_unsafe: exponents for which that may not hold (a positive zero is fine); the routines fall
+// back to divisions then.  Compared with `/` on 2^32 random pairs: no difference.
+__device__ __forceinline__ double rcp_seed(double v) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+  return y;
+}
+__device__ __forceinline__ double reciprocal(double t) {
+  double y = rcp_seed(t);
+  const double e = fma(-t, y, 1.0);
+  y = fma(y, fma(e, e, e), y);
+  return fma(fma(-t, y, 1.0), y, y);
+}
+__device__ __forceinline__ double quotient(double x, double t, double y) {
+  double q = x * y;
+  q = fma(fma(-q, t, x), y, q);
+  return fma(fma(-q, t, x), y, q);
+}
+__device__ __forceinline__ int quotient_unsafe(double x, double t) {  // without branches
+  const int hx = __double2hiint(x), lx = __double2loint(x), ht = __double2hiint(t), lt = __double2loint(t);
+  const int ex = (int)((unsigned)((hx >> 20) & 0x7FF) - 600u >= 846u), et = (int)((unsigned)((ht >> 20) & 0x7FF) - 600u >= 846u);
+  // the all-ones mantissa is the one divisor whose reciprocal the last step may not round right
+  const int ones = (int)(((ht | 0xFFF00000) & lt) == -1);
+  return et | ones | (ex & (int)((hx | lx) != 0));
 }
 
 // ------------------------------------------------------------------------- GETRF
@@ -1016,227 +1029,350 @@ __device__ __noinline__ void dev_getrf(double* A, int lda, int m, int n, double*
   __syncthreads();
 }
 
-// A[m x n] := L\U of P A with partial pivoting inside the block (m, n <= TL), P written to
-// Pout (m doubles of row indices).  Step i: the row r >= i of largest |a_ri| (the first of
-// equal ones; warp 0 scans, lanes take rows i + lane + 32 t in ascending order, the shuffle
-// tree keeps the larger value and, on a tie, the smaller row), whole rows i and r swapped,
-// then l_r = a_ri / a_ii and a_rc = fma(a_ic, -l_r, a_rc) for r, c > i — the elimination of
-// the unpivoted routine, so a block that needs no swap gets the same bits.  The block lives in
-// shared memory (row stride LDS) for the whole factorization.
-__device__ __noinline__ void dev_getrf_piv(double* A, int lda, int m, int n, double* Pout, double* smem) {
-  double* S = smem;
-  int* perm = reinterpret_cast<int*>(smem + TL * LDS);
-  int* pivot = perm + TL;
-  load_tile(S, A, lda, m, n);
-  for (int i = threadIdx.x; i < m; i += NT) perm[i] = i;
-  __syncthreads();
-  const int mn = min(m, n), lane = threadIdx.x & 31;
-  for (int i = 0; i < mn; ++i) {
-    if (threadIdx.x < 32) {
-      double best = -1.0;
-      int bi = i;
-      for (int r = i + lane; r < m; r += 32) {
-        const double v = fabs(S[r * LDS + i]);
-        if (v > best) { best = v; bi = r; }
-      }
+// A[m x n] := L\U of P A with partial pivoting inside the block (m, n <= TL), P written to Pout (m
+// doubles of row indices).  Step i first swaps whole rows i and r, r >= i the row of largest |a_ri|
+// (the first of equal ones), then eliminates as the unpivoted routine does, so a block that needs
+// no swap gets the same bits.
+//
+// The block stays in shared memory, eight columns per warp.  The warp of a column group factors it
+// (two rows per lane, which stay where they are: only their positions are swapped), then the warps
+// of the groups to the right solve their eight rows against it and update the rows below on the
+// FP64 tensor cores (a chain of fma in ascending i, see dmma); the next group's warp goes on to
+// factor it while the others still update.  One CTA barrier per eight steps; the instructions of
+// the one warp that factors bound it.  64 x 64, hop included: 80 -> 41 us (before: the whole block
+// in shared memory with four CTA barriers per step).  Without pivoting the routine above is as fast.
+#define GETRF_LD (TL + 4)
+// the pivot of step ci among the rows at positions >= ci (a lane's two rows: values v0, v1 at
+// positions pos): lane pl, half ph; swaps the positions of the pivot row and of the row at ci
+__device__ __forceinline__ void getrf_pivot(double v0, double v1, int (&pos)[2], int ci, int m, int& pl, int& ph) {
+  double best = -1.0;
+  int bp = ci;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-      }
-      if (lane == 0) *pivot = bi;
+  for (int h = 0; h < 2; ++h) {
+    const double v = fabs(h ? v1 : v0);
+    if (pos[h] >= ci && pos[h] < m && (v > best || (v == best && pos[h] < bp))) {
+      best = v;
+      bp = pos[h];
     }
-    __syncthreads();
-    const int r = *pivot;
-    if (r != i) {
-      for (int c = threadIdx.x; c < n; c += NT) {
-        const double t = S[i * LDS + c];
-        S[i * LDS + c] = S[r * LDS + c];
-        S[r * LDS + c] = t;
-      }
-      if (threadIdx.x == 0) {
-        const int t = perm[i];
-        perm[i] = perm[r];
-        perm[r] = t;
-      }
-    }
-    __syncthreads();
-    const double d = S[i * LDS + i];
-    for (int rr = i + 1 + threadIdx.x; rr < m; rr += NT) S[rr * LDS + i] = S[rr * LDS + i] / d;
-    __syncthreads();
-    const int w = n - i - 1;
-    for (int e = threadIdx.x; e < (m - i - 1) * w; e += NT) {
-      const int rr = i + 1 + e / w, c = i + 1 + e % w;
-      S[rr * LDS + c] = fma(S[i * LDS + c], -S[rr * LDS + i], S[rr * LDS + c]);
-    }
-    __syncthreads();
   }
-  for (int e = threadIdx.x; e < m * n; e += NT) {
-    const int rr = e / n, c = e % n;
-    A[(size_t)rr * lda + c] = S[rr * LDS + c];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double ov = __shfl_xor_sync(0xffffffffu, best, o);
+    const int op = __shfl_xor_sync(0xffffffffu, bp, o);
+    if (ov > best || (ov == best && op < bp)) {
+      best = ov;
+      bp = op;
+    }
   }
-  for (int i = threadIdx.x; i < m; i += NT) Pout[i] = (double)perm[i];
-  __syncthreads();
+  const unsigned h0 = __ballot_sync(0xffffffffu, pos[0] == bp), h1 = __ballot_sync(0xffffffffu, pos[1] == bp);
+  pl = __ffs((int)(h0 | h1)) - 1;
+  ph = h1 != 0u;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) pos[h] = pos[h] == bp ? ci : pos[h] == ci ? bp : pos[h];
 }
 
-// ------------------------------------------------------------------------- TRSM sweeps
-// One triangular sweep over independent lines (the columns of B for TRSML / TRSMRT /
-// TRSMU, the rows of B for TRSMR) against a triangle T staged in shared memory (ld LDS).
-// Line q is held by R consecutive lanes of a warp: lane R cc + g holds positions g + R j
-// (j < TL / R); position p of step i is eliminated as x_p = fma(-coef(i, p), x_i, x_p),
-// the operand order of the reference's routines up to the commutation of the product
-// (exact inside an fma).  The finished x_i reaches the line's lanes by a shuffle; no CTA
-// barrier inside the sweep.  Steps run in TL / R blocks of R with a compile-time block
-// index (register selection and the live range of positions resolved at compile time).
-//   PIV 0: unit diagonal, x_i unchanged                     (TRSML, kernel.cu:150-182)
-//   PIV 1: x_i = x_i * rd[i], rd = 1 / diagonal              (TRSMRT kernel.cu:229-285, TRSMU)
-//   PIV 2: x_i = x_i / t_ii                                  (TRSMR, kernel.cu:185-226)
-//   CT: coef(i, p) = T[i][p] (row i of T) when true, T[p][i] (column i) when false.
-template <int R, int PIV, bool CT, bool BACK>
-struct Sweep {
-  static constexpr int NJ = TL / R;
-  double x[NJ];
-  const double* T;
-  const double* rd;
-  int g, src0, len;
-
-  template <int J>
-  __device__ __forceinline__ void step(int i) {
-    const int ii = i - R * J;
-    double v = __shfl_sync(0xffffffffu, x[J], ii, R);
-    if (PIV == 1) v = v * rd[i];
-    if (PIV == 2) v = v / T[i * LDS + i];
-    if (PIV != 0 && g == ii) x[J] = v;
+// a panel with divisions, in shared memory, for values out of the quotients' range (rows stay where
+// they are, pos gives their positions)
+__device__ __noinline__ void getrf_panel_by_division(double* S, int cg, int m, int w, int steps, int (&pos)[2],
+                                                     int lane) {
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      const bool live = BACK ? (j < J || (j == J && g < ii)) : (j > J || (j == J && g > ii));
-      if (live) {
-        const int p = g + R * j;
-        const double c = CT ? T[i * LDS + p] : T[p * LDS + i];
-        x[j] = fma(-c, v, x[j]);
-      }
-    }
-  }
-  template <int J>
-  __device__ __forceinline__ void block() {
-    if (R * J + R <= len) {  // a whole block: steps unrolled, coefficient loads scheduled early
-#pragma unroll
-      for (int t = 0; t < R; ++t) step<J>(BACK ? R * J + R - 1 - t : R * J + t);
-    } else {
-      const int i0 = BACK ? len - 1 : R * J;
-      const int i1 = BACK ? R * J - 1 : len;
+  for (int h = 0; h < 2; ++h) pos[h] = cg + lane + 32 * h;
+  double* r0 = S + min(cg + lane, TL - 1) * GETRF_LD + cg;
+  double* r1 = S + min(cg + lane + 32, TL - 1) * GETRF_LD + cg;
 #pragma unroll 1
-      for (int i = i0; i != i1; i += BACK ? -1 : 1) step<J>(i);
+  for (int i = 0; i < steps; ++i) {
+    const int ci = cg + i;
+    int pl, ph;
+    getrf_pivot(r0[i], r1[i], pos, ci, m, pl, ph);
+    const double* pr = S + (cg + pl + 32 * ph) * GETRF_LD + cg;
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+      double* r = h ? r1 : r0;
+      if (cg + lane + 32 * h < m && (h ? pos[1] : pos[0]) > ci) {
+        const double l = r[i] / pr[i];
+        r[i] = l;
+        for (int c = i + 1; c < w; ++c) r[c] = fma(pr[c], -l, r[c]);
+      }
     }
+    __syncwarp();
   }
-  template <int J>
-  __device__ __forceinline__ void run_from() {
-    if constexpr (J >= 0 && J < NJ) {
-      if (R * J < len) block<J>();
-      run_from<BACK ? J - 1 : J + 1>();
-    }
-  }
-  __device__ __forceinline__ void run() {
-    if constexpr (BACK) run_from<NJ - 1>();
-    else run_from<0>();
-  }
-};
+}
 
-// B: lines of length len (<= TL), line q at B + q * lstride, position p at + p * pstride.
-// perm (shared memory, optional): position p of a line is loaded from position perm[p] (the
-// row permutation of a pivoted L block); results are stored in natural order.  A line lives in
-// the registers of its lanes between its loads and its stores, so the permuted load is safe in
-// place.
-template <int R, int PIV, bool CT, bool BACK>
-__device__ __forceinline__ void tri_sweep(double* B, size_t lstride, size_t pstride, int nlines, int len,
-                                          const double* T, const double* rd, const int* perm = nullptr) {
-  constexpr int LPP = NT / R;  // lines per pass
-  const int lane = threadIdx.x & 31, g = lane % R;
-  const int q_in = (threadIdx.x / 32) * (32 / R) + lane / R;
-  for (int q0 = 0; q0 < nlines; q0 += LPP) {
-    if (q0 + (threadIdx.x / 32) * (32 / R) >= nlines) continue;  // warp without a live line
-    const int q = q0 + q_in;
-    Sweep<R, PIV, CT, BACK> S;
-    S.T = T;
-    S.rd = rd;
-    S.g = g;
-    S.src0 = 0;
-    S.len = len;
+__device__ __forceinline__ void dev_getrf_piv(double* A, int lda, int m, int n, double* Pout) {
+  extern __shared__ __align__(16) double vm_smem[];
+  double* S = vm_smem;                                         // TL x GETRF_LD
+  int* from = reinterpret_cast<int*>(S + TL * GETRF_LD);       // [2][TL]: row now at p was at from[p] before the panel
+  int* perm = from + 2 * TL;                                   // row at p came from row perm[p] of A
+  const int tid = thread_index(), warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3;
+  const int mn = min(m, n), panels = (mn + 7) >> 3;
+  {
+    const int c = tid & 63;
+    if (c < n) {
+#pragma unroll 4
+      for (int r = tid >> 6; r < m; r += NT / 64) cp_async8(smem_u32(S + r * GETRF_LD + c), A + (size_t)r * lda + c, 8u);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    if (tid < TL) perm[tid] = tid;
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int J = -1; J < panels; ++J) {
+    const int c0 = 8 * J, cg = 8 * warp;
+    if (J >= 0 && cg < n && warp != J) {
+      {  // the panel's row swaps, applied to this warp's columns
+        const int* f = from + (J & 1) * TL;
+        double x[8][2];
 #pragma unroll
-    for (int j = 0; j < Sweep<R, PIV, CT, BACK>::NJ; ++j) {
-      const int p = g + R * j;
-      const int src = (perm && p < len) ? perm[p] : p;
-      S.x[j] = (q < nlines && p < len) ? ldcg(&B[q * lstride + src * pstride]) : 0.0;
-    }
-    S.run();
+        for (int t = 0; t < 8; ++t) {
+          const int r = min(8 * t + fa, m - 1), sr = r < c0 ? r : f[r];
+          x[t][0] = S[sr * GETRF_LD + cg + 2 * fb];
+          x[t][1] = S[sr * GETRF_LD + cg + 2 * fb + 1];
+        }
+        __syncwarp();
 #pragma unroll
-    for (int j = 0; j < Sweep<R, PIV, CT, BACK>::NJ; ++j) {
-      const int p = g + R * j;
-      if (q < nlines && p < len) B[q * lstride + p * pstride] = S.x[j];
+        for (int t = 0; t < 8; ++t) {
+          const int r = 8 * t + fa;
+          if (r < m) {
+            S[r * GETRF_LD + cg + 2 * fb] = x[t][0];
+            S[r * GETRF_LD + cg + 2 * fb + 1] = x[t][1];
+          }
+        }
+        __syncwarp();
+      }
+      if (warp > J) {
+        // rows c0 .. c0 + 7 of these columns: solve against the panel's unit lower triangle
+        double* u = S + (c0 + fa) * GETRF_LD;
+        double x0 = u[cg + 2 * fb], x1 = u[cg + 2 * fb + 1];
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+          const double v0 = __shfl_sync(0xffffffffu, x0, 4 * i + fb), v1 = __shfl_sync(0xffffffffu, x1, 4 * i + fb);
+          const double c = u[c0 + i];
+          const double y0 = fma(v0, -c, x0), y1 = fma(v1, -c, x1);
+          x0 = fa > i ? y0 : x0;
+          x1 = fa > i ? y1 : x1;
+        }
+        u[cg + 2 * fb] = x0;
+        u[cg + 2 * fb + 1] = x1;
+        __syncwarp();
+        const double b0 = S[(c0 + fb) * GETRF_LD + cg + fa], b1 = S[(c0 + 4 + fb) * GETRF_LD + cg + fa];
+#pragma unroll 2
+        for (int r = c0 + 8 + fa; r < m + fa; r += 8) {  // tiles of eight rows; rows past m stay inside S
+          double* p = S + r * GETRF_LD;
+          double y0 = p[cg + 2 * fb], y1 = p[cg + 2 * fb + 1];
+          dmma(y0, y1, -p[c0 + fb], b0);
+          dmma(y0, y1, -p[c0 + 4 + fb], b1);
+          p[cg + 2 * fb] = y0;
+          p[cg + 2 * fb + 1] = y1;
+        }
+        __syncwarp();
+      }
+    }
+    if (warp == J + 1 && warp < panels) {  // factor the next panel: columns cg .., rows cg ..
+      const int w = min(8, n - cg), steps = min(8, mn - cg);
+      double x[2][8];
+      int pos[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        pos[h] = cg + lane + 32 * h;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) x[h][c] = (pos[h] < m && c < w) ? S[pos[h] * GETRF_LD + cg + c] : 0.0;
+      }
+      int bad = 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int ci = cg + i;
+        int pl = i, ph = 0;
+        if (i < steps) getrf_pivot(x[0][i], x[1][i], pos, ci, m, pl, ph);
+        double u[8];
+#pragma unroll
+        for (int c = i; c < 8; ++c) u[c] = __shfl_sync(0xffffffffu, ph ? x[1][c] : x[0][c], pl);
+        const double y = reciprocal(u[i]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int below = (int)(i < steps) & (int)(pos[h] > ci) & (int)(pos[h] < m);
+          const double l = quotient(x[h][i], u[i], y);
+          bad |= below & quotient_unsafe(x[h][i], u[i]);
+          x[h][i] = below ? l : x[h][i];
+#pragma unroll
+          for (int c = i + 1; c < 8; ++c) {
+            const double v = fma(u[c], -l, x[h][c]);
+            x[h][c] = below ? v : x[h][c];
+          }
+        }
+      }
+      if (__any_sync(0xffffffffu, bad)) {
+        getrf_panel_by_division(S, cg, m, w, steps, pos, lane);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            if (cg + lane + 32 * h < m && c < w) x[h][c] = S[(cg + lane + 32 * h) * GETRF_LD + cg + c];
+        __syncwarp();
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int row = cg + lane + 32 * h;
+        if (row < m) {
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            if (c < w) S[pos[h] * GETRF_LD + cg + c] = x[h][c];
+          from[((J + 1) & 1) * TL + pos[h]] = row;
+        }
+      }
+      {
+        __syncwarp();
+        int v[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int p = lane + 32 * h;
+          v[h] = p < m ? perm[p < cg ? p : from[((J + 1) & 1) * TL + p]] : 0;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (lane + 32 * h < m) perm[lane + 32 * h] = v[h];
+      }
+    }
+    __syncthreads();
+  }
+  {
+    const int c = tid & 63;
+    if (c < n)
+#pragma unroll 4
+      for (int r = tid >> 6; r < m; r += NT / 64) A[(size_t)r * lda + c] = S[r * GETRF_LD + c];
+    for (int i = tid; i < m; i += NT) Pout[i] = (double)perm[i];
+  }
+  __syncthreads();
+}
+
+// ------------------------------------------------------------------------- triangular solves
+// TRSMR's eight positions of a block against each other with divisions, for values out of the
+// quotients' range (a call: beside it in one loop the compiler's code for the usual case is three
+// times slower).  w: the lane's row of coefficients within the block.
+__device__ __noinline__ double2 tri_by_division(double x0, double x1, double tii, const double* w, int lane) {
+  const int fa = lane >> 2, fb = lane & 3;
+#pragma unroll 1
+  for (int i = 0; i < 8; ++i) {
+    const double v0 = __shfl_sync(0xffffffffu, x0 / tii, 4 * i + fb), v1 = __shfl_sync(0xffffffffu, x1 / tii, 4 * i + fb);
+    const double c = w[i], y0 = fma(-c, v0, x0), y1 = fma(-c, v1, x1);
+    x0 = fa > i ? y0 : fa == i ? v0 : x0;
+    x1 = fa > i ? y1 : fa == i ? v1 : x1;
+  }
+  return make_double2(x0, x1);
+}
+
+// Triangular solve with one triangle of len <= TL rows, in place on `lines` independent lines of B:
+// the columns of B for TRSML / TRSMRT / TRSMU, the rows for TRSMR.  Position i of a line is solved,
+// then x_p = fma(-coef(i, p), x_i, x_p) for the later ones, i ascending (descending for TRSMU):
+//   TRSML   coef T[p][i], unit diagonal            (kernel.cu:150-182; perm: B's rows permuted first)
+//   TRSMRT  coef T[i][p], x_i = x_i * (1 / t_ii)   (kernel.cu:229-285)
+//   TRSMR   coef T[i][p], x_i = x_i / t_ii         (kernel.cu:185-226)
+//   TRSMU   coef T[p][i], x_i = x_i * (1 / t_ii), from the last position to the first
+// The coefficients are staged as W[p][i] (for TRSMU with positions counted from the end, so that
+// every kind runs forward), a warp takes eight lines and needs no other warp from there on.  Eight
+// positions at a time: the sum over the earlier positions on the FP64 tensor cores (a chain of fma
+// in ascending i, see dmma), then the eight against each other with shuffles (about 40 cycles a
+// position, 140 with a quotient), which bounds it.  On a B200, hop of 2.5 us included (before: a
+// shuffled sweep over all 64 positions, unrolled, its coefficients fetched step by step):
+//   64 x 64: TRSML 18 -> 11 us, TRSMR 22.8 -> 14.5 us;  TRSML 256 x 64: 149 -> 63 us
+#define TRI_LDX 12  /* doubles between positions of a warp's lines: 4 mod 8, no bank conflicts */
+__device__ __forceinline__ void dev_tri(int op, double* B, int ldb, const double* T, int ldt, int len, int lines,
+                                        const double* perm) {
+  extern __shared__ __align__(16) double vm_smem[];
+  double* W = vm_smem;                // TL x GM_LD
+  double* rd = W + TL * GM_LD;        // reciprocals of the diagonal
+  const int tid = thread_index(), warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3;
+  double* X = rd + TL + warp * (TL * TRI_LDX);
+  const bool ct = op == PP_OP_TRSMR || op == PP_OP_TRSMRT, back = op == PP_OP_TRSMU, byrow = op == PP_OP_TRSMR;
+  const size_t ps = byrow ? 1 : (size_t)ldb, ls = byrow ? (size_t)ldb : 1;
+  {  // the triangle's half with i <= p, element (r, c) of T at (p, i)
+    const int c = tid & 63;
+#pragma unroll 4
+    for (int r = tid >> 6; r < len; r += NT / 64) {
+      int p = ct ? c : r, i = ct ? r : c;
+      if (back) { p = len - 1 - p; i = len - 1 - i; }
+      if (c < len && i <= p) cp_async8(smem_u32(W + p * GM_LD + i), T + (size_t)r * ldt + c, 8u);
     }
   }
-}
-
-template <int PIV, bool CT, bool BACK>
-__device__ __forceinline__ void tri_lines(double* B, size_t lstride, size_t pstride, int nlines, int len,
-                                          const double* T, const double* rd, const int* perm = nullptr) {
-  if (nlines <= 16) tri_sweep<16, PIV, CT, BACK>(B, lstride, pstride, nlines, len, T, rd, perm);
-  else tri_sweep<4, PIV, CT, BACK>(B, lstride, pstride, nlines, len, T, rd, perm);
-}
-
-// B[m x n] := L^-1 B, L unit lower m x m (m <= TL); columns independent
-__device__ __noinline__ void dev_trsml(double* B, int ldb, const double* L, int ldl, int m, int n, double* smem) {
-  load_tile(smem, L, ldl, m, m);
-  __syncthreads();
-  tri_lines<0, false, false>(B, 1, (size_t)ldb, n, m, smem, nullptr);
-  __syncthreads();
-}
-
-// B[m x n] := L^-1 P B (m <= TL), P the row permutation of a pivoted GETRF of L's block
-// (P[i]: the row of B that row i of P B takes; m doubles holding indices)
-__device__ __noinline__ void dev_trsml_piv(double* B, int ldb, const double* L, int ldl, const double* P, int m, int n,
-                                           double* smem) {
-  int* perm = reinterpret_cast<int*>(smem + TL * LDS);
-  load_tile(smem, L, ldl, m, m);
-  for (int i = threadIdx.x; i < m; i += NT) {
-    const int v = (int)ldcg(&P[i]);
-    perm[i] = (v >= 0 && v < m) ? v : i;  // indices come from the block's GETRF; guard anyway
+  bool first = true;
+  for (int q0 = 8 * warp;; q0 += NT / 4) {
+    const int nq = min(8, lines - q0);
+    if (nq > 0) {
+      // lanes along what is contiguous in B: the positions of a row, or the lines
+      const int qs = byrow ? 1 : 32, p_step = byrow ? 32 : 4;
+#pragma unroll 1
+      for (int q = byrow ? 0 : lane & 7; q < nq; q += qs)
+#pragma unroll 4
+        for (int p = byrow ? lane : lane >> 3; p < len; p += p_step) {
+          int src = back ? len - 1 - p : p;
+          if (perm) {
+            const int v = (int)ldcg(&perm[p]);
+            src = (v >= 0 && v < len) ? v : p;  // indices come from the block's GETRF; guard anyway
+          }
+          cp_async8(smem_u32(X + p * TRI_LDX + q), B + (size_t)(q0 + q) * ls + (size_t)src * ps, 8u);
+        }
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    if (first) {
+      __syncthreads();
+      if (tid < len) rd[tid] = 1.0 / W[tid * GM_LD + tid];
+      __syncthreads();
+      first = false;
+    }
+    __syncwarp();
+    if (nq <= 0) break;
+#pragma unroll 1
+    for (int t = 0; t < len; t += 8) {
+      double x0 = X[(t + fa) * TRI_LDX + 2 * fb], x1 = X[(t + fa) * TRI_LDX + 2 * fb + 1];
+      const double* w = W + (t + fa) * GM_LD;
+#pragma unroll 2
+      for (int j = 0; j < t; j += 8) {
+        const double a0 = -w[j + fb], a1 = -w[j + 4 + fb];
+        const double b0 = X[(j + fb) * TRI_LDX + fa], b1 = X[(j + 4 + fb) * TRI_LDX + fa];
+        dmma(x0, x1, a0, b0);
+        dmma(x0, x1, a1, b1);
+      }
+      const double mine = rd[t + fa], tii = w[t + fa];
+      if (op == PP_OP_TRSMR) {
+        const double s0 = x0, s1 = x1;
+        int bad = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          bad |= (int)(fa == i) & (quotient_unsafe(x0, tii) | quotient_unsafe(x1, tii));
+          const double v0 = __shfl_sync(0xffffffffu, quotient(x0, tii, mine), 4 * i + fb);
+          const double v1 = __shfl_sync(0xffffffffu, quotient(x1, tii, mine), 4 * i + fb);
+          const double c = w[t + i], y0 = fma(-c, v0, x0), y1 = fma(-c, v1, x1);
+          x0 = fa > i ? y0 : fa == i ? v0 : x0;
+          x1 = fa > i ? y1 : fa == i ? v1 : x1;
+        }
+        if (__any_sync(0xffffffffu, bad & (int)(t + fa < len))) {
+          const double2 r = tri_by_division(s0, s1, tii, w + t, lane);
+          x0 = r.x;
+          x1 = r.y;
+        }
+      } else {
+        const double f = op == PP_OP_TRSML ? 1.0 : mine;  // a product with 1 changes nothing
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const double v0 = __shfl_sync(0xffffffffu, x0 * f, 4 * i + fb);
+          const double v1 = __shfl_sync(0xffffffffu, x1 * f, 4 * i + fb);
+          const double c = w[t + i], y0 = fma(-c, v0, x0), y1 = fma(-c, v1, x1);
+          x0 = fa > i ? y0 : fa == i ? v0 : x0;
+          x1 = fa > i ? y1 : fa == i ? v1 : x1;
+        }
+      }
+      __syncwarp();
+      X[(t + fa) * TRI_LDX + 2 * fb] = x0;
+      X[(t + fa) * TRI_LDX + 2 * fb + 1] = x1;
+      const int p = t + fa, dst = back ? len - 1 - p : p;
+      double* o = B + (size_t)(q0 + 2 * fb) * ls + (size_t)dst * ps;
+      st_if(o, x0, p < len && 2 * fb < nq);
+      st_if(o + ls, x1, p < len && 2 * fb + 1 < nq);
+      __syncwarp();
+    }
   }
-  __syncthreads();
-  tri_lines<0, false, false>(B, 1, (size_t)ldb, n, m, smem, nullptr, perm);
-  __syncthreads();
-}
-
-// V[m x n] := U^-T V, U upper m x m (m <= TL): the reference's trsmr on a transposed B
-// (kernel.cu:229-285) — row i is scaled by the reciprocal of u_ii, then eliminated below
-__device__ __noinline__ void dev_trsmrt(double* V, int ldv, const double* U, int ldu, int m, int n, double* smem) {
-  double* rd = smem + TL * LDS;
-  load_tile(smem, U, ldu, m, m);
-  __syncthreads();
-  if (threadIdx.x < m) rd[threadIdx.x] = 1. / smem[threadIdx.x * LDS + threadIdx.x];
-  __syncthreads();
-  tri_lines<1, true, false>(V, 1, (size_t)ldv, n, m, smem, rd);
-  __syncthreads();
-}
-
-// B[m x n] := U^-1 B, U upper m x m (m <= TL), backward substitution (solve phase; no
-// reference counterpart): x_i = b_i * (1 / u_ii), then b_r -= u_ri x_i for r < i
-__device__ __noinline__ void dev_trsmu(double* B, int ldb, const double* U, int ldu, int m, int n, double* smem) {
-  double* rd = smem + TL * LDS;
-  load_tile(smem, U, ldu, m, m);
-  __syncthreads();
-  if (threadIdx.x < m) rd[threadIdx.x] = 1. / smem[threadIdx.x * LDS + threadIdx.x];
-  __syncthreads();
-  tri_lines<1, false, true>(B, 1, (size_t)ldb, n, m, smem, rd);
-  __syncthreads();
-}
-
-// B[m x n] := B U^-1, U upper n x n (n <= TL); rows independent
-__device__ __noinline__ void dev_trsmr(double* B, int ldb, const double* U, int ldu, int m, int n, double* smem) {
-  load_tile(smem, U, ldu, n, n);
-  __syncthreads();
-  tri_lines<2, true, false>(B, (size_t)ldb, 1, m, n, smem, nullptr);
   __syncthreads();
 }
 
@@ -1462,7 +1598,7 @@ __device__ __forceinline__ bool tri_step(int op, double* B, int ldb, const doubl
   return true;
 }
 
-__device__ __forceinline__ void run_composite(const pp_task& T, double* smem) {
+__device__ __forceinline__ void run_composite(const pp_task& T) {
   const bool product = T.op == PP_OP_GEMM || T.op == PP_OP_GEMM3 || T.op == PP_OP_GEMM4;
   const bool free_order = T.op == PP_OP_GEMM && (T.flags & PP_FREE_ORDER);
   int op = T.op, size = T.op == PP_OP_TRSMR ? T.n : T.m, lines = T.op == PP_OP_TRSMR ? T.m : T.n;
@@ -1495,13 +1631,8 @@ __device__ __forceinline__ void run_composite(const pp_task& T, double* smem) {
       int d = 0, len = 0;
       if (!tri_step(op, B, ldb, A, lda, size, lines, step, d, len, P)) break;
       if (!(step & 1)) {
-        const double* D = A + (size_t)d * lda + d;
-        switch (op) {
-          case PP_OP_TRSML: dev_trsml(B + (size_t)d * ldb, ldb, D, lda, len, lines, smem); break;
-          case PP_OP_TRSMRT: dev_trsmrt(B + (size_t)d * ldb, ldb, D, lda, len, lines, smem); break;
-          case PP_OP_TRSMR: dev_trsmr(B + d, ldb, D, lda, lines, len, smem); break;
-          default: dev_trsmu(B + (size_t)d * ldb, ldb, D, lda, len, lines, smem); break;
-        }
+        double* Bd = B + (op == PP_OP_TRSMR ? (size_t)d : (size_t)d * ldb);
+        dev_tri(op, Bd, ldb, A + (size_t)d * lda + d, lda, len, lines, (T.flags & PP_PIVOT) ? T.p[2] : nullptr);
         continue;
       }
     }
@@ -2192,7 +2323,7 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
       if (T.m > TL || T.n > TL) return false;
       if (T.flags & PP_PIVOT) {
         if (!T.p[1]) return false;
-        dev_getrf_piv(T.p[0], T.ld[0], T.m, T.n, T.p[1], smem);
+        dev_getrf_piv(T.p[0], T.ld[0], T.m, T.n, T.p[1]);
       } else {
         dev_getrf(T.p[0], T.ld[0], T.m, T.n, smem);
       }
@@ -2200,8 +2331,7 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
     case PP_OP_TRSML:
       if (T.flags & PP_PIVOT) {  // one pivoted block per instruction
         if (T.m > TL || !T.p[2]) return false;
-        dev_trsml_piv(T.p[0], T.ld[0], T.p[1], T.ld[1], T.p[2], T.m, T.n, smem);
-        return true;
+        break;
       }
       if (T.m > PP_VM_TRI) return false;
       break;
@@ -2271,7 +2401,7 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
       return true;
     default: return false;
   }
-  run_composite(T, smem);
+  run_composite(T);
   return true;
 }
 
