@@ -1640,647 +1640,475 @@ __device__ __forceinline__ void run_composite(const pp_task& T) {
   }
 }
 
-// ------------------------------------------------------------------------- ACCUM
-// U1 V1^T := Q Q^T (U1 V1^T + alpha U2 V2^T), Q spanning (U1 V1^T + alpha U2 V2^T) R:
-// the reference's randomized accumulation (kernel.cu:1255-1280) with Q from shifted
-// CholeskyQR3 (three Gram passes) in place of the reference's Givens sweeps.
-// m = ny, n = nx, k = k1 (target rank), l = k2; k1, k2 <= PP_VM_MAX_RANK.
-//   S  = R^T [V1 V2]                      (k1 x (k1 + k2), one pass over the nx rows)
-//   Y  = U1 S1^T + alpha U2 S2^T          (ny x k1, a thread per row)
+// ------------------------------------------------------------------------- low-rank instructions
+// ACCUM, ORTH and LRTRUNC, made of four pieces with one copy of code each (see dev_gemm for why):
+//   tn    S = X^T [W1 W2], small outputs over many rows, on the FP64 tensor cores
+//   rows  Y = A1 S1^T + alpha A2 S2^T row by row, on the FP64 tensor cores
+//   chol  Cholesky G = C^T C of a Gram matrix: C itself, or S1 = C^-T with Y C^-1 = Y S1^T
+//   svd   one-sided Jacobi on C and the rank decision: the matrix S2 of kept singular directions
+// ACCUM: U1 V1^T := Q Q^T (U1 V1^T + alpha U2 V2^T), Q spanning (U1 V1^T + alpha U2 V2^T) R, the
+// reference's randomized accumulation (kernel.cu:1255-1280) with Q from shifted CholeskyQR3 (three
+// Gram passes) in place of the reference's Givens sweeps; m = ny, n = nx, k = k1 (target rank),
+// l = k2; k1, k2 <= PP_VM_MAX_RANK:
+//   [S1 S2] = R^T [V1 V2],  Y = U1 S1^T + alpha U2 S2^T            (the sketch, ny x k1)
 //   3x: G = Y^T Y (+ shift), G = C^T C, Y := Y C^-1
-//   P  = Y^T [U1 U2]                      (one pass over the ny rows)
-//   V1 := V1 P1^T + alpha V2 P2^T,  U1 := Y
-// Y stays in shared memory when it fits (ny k1 <= the Y capacity: a 512 x 32 sketch does),
-// else in the task's global scratch.  The long reductions are warp-sliced (lanes own output
-// columns, warps own row slices) and the warp partials are summed in a fixed order through
-// two slots, so results are deterministic.
-#define ACC_LG (PP_VM_MAX_RANK + 1)
-
+//   [S1 S2] = Y^T [U1 U2],  V1 := V1 S1^T + alpha V2 S2^T,  U1 := Y
+//   adaptive (PP_ADAPT_RANK): U1 V1^T = Y V1^T with Y orthonormal, so the singular values are those
+//   of V1; both factors are turned into the eigenbasis of V1^T V1 and the directions whose singular
+//   value exceeds beta times the largest are kept (zero columns beyond the new rank)
+// ORTH: the three passes on Y = p[0] alone.  LRTRUNC: the adaptive part on U = p[0] (orthonormal
+// columns) and V = p[1].  The sketch stays in shared memory when it fits, else in the task's scratch.
+//
+// Measured on a B200, hop included (before: reductions with one k step of loads in flight, a
+// one-warp Cholesky, substitutions, a two-sided Jacobi on the Gram matrix):
+//   ACCUM 128 x 128, k 32, adaptive   430 -> 134 us      ACCUM 94 x 94, k 16   54 -> 24 us
+//   ORTH  512 x 32                    144 ->  78 us      LRTRUNC 512 x 512, k 32   420 -> 130 us
+// 17 us of the first are products at the FP64 tensor rate, 79 the chain of Jacobi steps.
 template <int KB>
-struct AccumSmem {
-  // a partial slot holds a KB x 2KB output (ld 2KB); the first one also holds the Jacobi
-  // workspace (Z, rotations, pairs) of the adaptive truncation
-  static constexpr int SLOT0 = KB * 2 * KB, JAC = KB * ACC_LG + 3 * KB + 4;
-  static constexpr int SLOT = SLOT0 > JAC ? SLOT0 : (JAC + 7) & ~7;
-  static constexpr int RED = 2 * SLOT;
-  static constexpr int SOFF = SLOT;            // S (then P): k1 x (k1 + k2), ld 2 KB, in the second
-                                               // slot (written only after the slots are summed)
-  static constexpr int G = KB * ACC_LG + KB;   // Gram / Cholesky factor + reciprocals
-  static constexpr int YCAP = VM_SMEM_BYTES / 8 - RED - G;
+struct LrSmem {  // doubles; KB: largest rank, 16 or 32
+  static constexpr int LD = KB + 4;                       // row stride: 4 mod 16, no bank conflicts
+  static constexpr int S1 = 0, S2 = KB * LD, G = 2 * KB * LD, MISC = 3 * KB * LD, Y = MISC + 288;
+  static constexpr int YCAP = VM_SMEM_BYTES / 8 - Y;
 };
 
-// whether ACCUM keeps its ny x k1 sketch in shared memory (rows padded to k1 + 1 doubles, so
-// that a thread per row reads distinct banks); otherwise it lives in the task's scratch (ld k1)
+// whether ACCUM keeps its ny x k1 sketch in shared memory; otherwise it lives in the task's scratch
 __host__ __device__ constexpr bool accum_y_on_chip(long long ny, int k1, int k2) {
-  return ny * (k1 + 1) <= ((k1 <= 16 && k2 <= 16) ? AccumSmem<16>::YCAP : AccumSmem<32>::YCAP);
+  return ny * (k1 + 1) <= ((k1 <= 16 && k2 <= 16) ? LrSmem<16>::YCAP : LrSmem<32>::YCAP);
 }
 
-// out1 = the first b1, out2 = the next b2 columns of the a x (b1 + b2) sum of the two slots
-// (each read before any is written, so out may alias the slots)
+// a double anywhere (shared or global) under a predicate, else zero
+__device__ __forceinline__ double ld_if(const double* p, bool in) {
+  double v;
+  asm volatile("{\n .reg .pred a;\n setp.ne.s32 a, %2, 0;\n mov.f64 %0, 0d0000000000000000;\n @a ld.f64 %0, [%1];\n}\n"
+               : "=&d"(v)
+               : "l"(p), "r"((int)in)
+               : "memory");
+  return v;
+}
+
+// a matrix of rows with strides (row, column); null: absent (zero)
+struct LrMat {
+  const double* p;
+  int sr, sc, cols;
+};
+
+// NJ 8 x 8 tiles of X^T W over L rows: tile row mi of X's columns, tile columns j0 .. of W's
+template <int NJ>
+__device__ __forceinline__ void lr_tn_tiles(double (&acc)[4][2], const LrMat& X, const LrMat& W, int mi, int j0, int L,
+                                            int fa, int fb) {
+  constexpr int U = 4;  // k steps (of 4 rows) whose loads go out together
+  const bool xin = 8 * mi + fa < X.cols;
+  const double* xp = X.p + (size_t)fb * X.sr + (size_t)(8 * mi + fa) * X.sc;
+  const double* wp = W.p + (size_t)fb * W.sr + (size_t)(8 * j0 + fa) * W.sc;
+#pragma unroll 1
+  for (int l = fb; l < L + fb; l += 4 * U) {
+    double x[U], w[U][NJ];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = l + 4 * u < L;
+      x[u] = ld_if(xp + (size_t)(4 * u) * X.sr, in && xin);
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) w[u][j] = ld_if(wp + (size_t)(4 * u) * W.sr + (size_t)(8 * j) * W.sc, in && 8 * (j0 + j) + fa < W.cols);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) dmma(acc[j][0], acc[j][1], x[u], w[u][j]);
+    xp += (size_t)(4 * U) * X.sr;
+    wp += (size_t)(4 * U) * W.sr;
+  }
+}
+
+// out1 = X^T W1 and out2 = X^T W2 (when W2.p is set), zero-padded KB x KB blocks of stride KB + 4.
+// Every warp owns output tiles and walks all rows: no partial sums to combine, ascending row order.
 template <int KB>
-__device__ __forceinline__ void accum_combine(const double* red, int a, int b1, int b2, double* out1, double* out2,
-                                              int ldo) {
-  constexpr int SW = 2 * KB, SL = AccumSmem<KB>::SLOT, PER = (KB * 2 * KB + NT - 1) / NT;
-  const int bt = b1 + b2;
-  double v[PER];
+__device__ __forceinline__ void lr_tn(const LrMat& X, const LrMat& W1, const LrMat& W2, int L, double* out1, double* out2) {
+  constexpr int MT = KB / 8, LD = LrSmem<KB>::LD;
+  const int tid = thread_index(), warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3;
+  const int mi = warp % MT, part = warp / MT;  // 8 / MT warps share a tile row
+  const bool both = W2.p != nullptr;
+  double acc[4][2];
 #pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int e = threadIdx.x + q * NT;
-    v[q] = 0.0;
-    if (e < a * bt) {
-      const int i = e / bt, j = e % bt, col = j < b1 ? j : KB + (j - b1);
-      v[q] = red[i * SW + col] + red[SL + i * SW + col];
-    }
+  for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = 0.0;
+  int nj, j0;
+  const bool second = both && part >= 4 / MT;
+  if (KB == 32) {  // both: two warps of four tiles each; one: two of two
+    nj = both ? 4 : 2;
+    j0 = both ? 0 : 2 * part;
+  } else {         // both: four warps of one tile each; one: the first two
+    nj = both || part < 2 ? 1 : 0;
+    j0 = part & 1;
   }
-  __syncthreads();
+  const LrMat W = second ? W2 : W1;
+  if (KB == 32 && both) lr_tn_tiles<4>(acc, X, W, mi, j0, L, fa, fb);
+  else if (KB == 32) lr_tn_tiles<2>(acc, X, W, mi, j0, L, fa, fb);
+  else if (nj) lr_tn_tiles<1>(acc, X, W, mi, j0, L, fa, fb);
+  __syncthreads();  // the operands may lie where the results go
+  double* o = (second ? out2 : out1) + (8 * mi + fa) * LD + 8 * j0 + 2 * fb;
 #pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int e = threadIdx.x + q * NT;
-    if (e < a * bt) {
-      const int i = e / bt, j = e % bt;
-      if (j < b1) out1[i * ldo + j] = v[q];
-      else out2[i * ldo + (j - b1)] = v[q];
+  for (int j = 0; j < 4; ++j)
+    if (j < nj) {
+      o[8 * j] = acc[j][0];
+      o[8 * j + 1] = acc[j][1];
     }
-  }
-  __syncthreads();
-}
-
-template <bool GLOBAL>
-__device__ __forceinline__ double ld_any(const double* p) {
-  if constexpr (GLOBAL) return ldcg(p);
-  else return *p;
-}
-
-// out1[a x b1] = X^T W1 and out2[a x b2] = X^T W2 (shared memory, ld ldo), X: L x a,
-// W*: L x b* (or stored transposed when tW*).  Warp w sums rows [w L/8, (w+1) L/8); lane j
-// owns column j of W1 and of W2; row l of X reaches the lanes by shuffles (XG: X in global
-// memory, read once per row by lanes i < a) or as shared-memory broadcasts.
-template <int KB, bool XG, bool WG>
-__device__ __noinline__ void accum_tn(const double* X, int lx, int a, const double* W1, int lw1, bool tW1, int b1,
-                                      const double* W2, int lw2, bool tW2, int b2, int L, double* out1,
-                                      double* out2, int ldo, double* red) {
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double acc1[KB], acc2[KB];
-#pragma unroll
-  for (int i = 0; i < KB; ++i) acc1[i] = acc2[i] = 0.0;
-  const int per = (L + 7) / 8, l0 = min(L, w * per), l1 = min(L, l0 + per);
-  // rows in groups of RG: every load of a group is issued before the first product, so a
-  // warp waits for one memory latency per group, not per row
-  constexpr int RG = 8;
-  for (int lb = l0; lb < l1; lb += RG) {
-    double w1[RG], w2[RG], xr[RG];
-#pragma unroll
-    for (int t = 0; t < RG; ++t) {
-      const int l = lb + t;
-      const bool in = l < l1;
-      w1[t] = in && lane < b1 ? ld_any<WG>(tW1 ? &W1[(size_t)lane * lw1 + l] : &W1[(size_t)l * lw1 + lane]) : 0.0;
-      w2[t] = in && lane < b2 ? ld_any<WG>(tW2 ? &W2[(size_t)lane * lw2 + l] : &W2[(size_t)l * lw2 + lane]) : 0.0;
-      xr[t] = 0.0;
-      if constexpr (XG) xr[t] = in && lane < a ? ldcg(&X[(size_t)l * lx + lane]) : 0.0;
-    }
-#pragma unroll
-    for (int t = 0; t < RG; ++t) {
-      const int l = lb + t;
-      if (l >= l1) break;
-#pragma unroll
-      for (int i = 0; i < KB; ++i) {
-        if (i < a) {
-          double xi;
-          if constexpr (XG) xi = __shfl_sync(0xffffffffu, xr[t], i);
-          else xi = X[(size_t)l * lx + i];
-          acc1[i] = fma(xi, w1[t], acc1[i]);
-          acc2[i] = fma(xi, w2[t], acc2[i]);
-        }
-      }
-    }
-  }
-  // warp partials through two slots: warps 6, 7 store theirs, then 4, 5, then 2, 3, then 0, 1
-  // add theirs; the two slots are summed last
-  constexpr int SW = 2 * KB, SL = AccumSmem<KB>::SLOT;
-  for (int rd = 3; rd >= 0; --rd) {
-    if ((w >> 1) == rd) {
-      double* slot = red + (w & 1) * SL;
-#pragma unroll
-      for (int i = 0; i < KB; ++i)
-        if (i < a) {
-          if (lane < b1) slot[i * SW + lane] = rd == 3 ? acc1[i] : acc1[i] + slot[i * SW + lane];
-          if (lane < b2) slot[i * SW + KB + lane] = rd == 3 ? acc2[i] : acc2[i] + slot[i * SW + KB + lane];
-        }
-    }
-    __syncthreads();
-  }
-  accum_combine<KB>(red, a, b1, b2, out1, out2, ldo);
-}
-
-// FP64 tensor-core form of accum_tn for untransposed W (the usual case): per warp, its row
-// slice is the k dimension of out = X^T [W1 W2] computed with mma.sync.m8n8k4.f64 (FP64 has
-// no tcgen05 kind; this is the FP64 tensor path of sm_100a).  Fragment layouts of m8n8k4.f64:
-// A (8 x 4) lane l holds A[l/4][l%4]; B (4 x 8) holds B[l%4][l/4]; C (8 x 8) holds
-// C[l/4][2(l%4) + {0,1}].  Rows are taken four at a time (one k step), several k steps of
-// loads issued before their products.  Warp partials are combined as in accum_tn (fixed order).
-template <int KB, bool XG, bool WG>
-__device__ __noinline__ void accum_tn_mma(const double* X, int lx, int a, const double* W1, int lw1, int b1,
-                                          const double* W2, int lw2, int b2, int L, double* out1, double* out2,
-                                          int ldo, double* red) {
-  constexpr int MT = KB / 8, NTL = KB / 8;  // m tiles of X^T; n tiles per W
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qr = lane >> 2, qc = lane & 3;
-  double c1[MT][NTL][2], c2[MT][NTL][2];
-#pragma unroll
-  for (int i = 0; i < MT; ++i)
-#pragma unroll
-    for (int j = 0; j < NTL; ++j) c1[i][j][0] = c1[i][j][1] = c2[i][j][0] = c2[i][j][1] = 0.0;
-  const int per = (((L + 7) / 8) + 3) & ~3, l0 = min(L, w * per), l1 = min(L, l0 + per);
-  constexpr int KS = KB >= 32 ? 1 : 4;  // k steps (of 4 rows) whose loads go out together
-  for (int lb = l0; lb < l1; lb += 4 * KS) {
-    double fa[KS][MT], f1[KS][NTL], f2[KS][NTL];
-#pragma unroll
-    for (int s = 0; s < KS; ++s) {
-      const int l = lb + 4 * s + qc;  // the row this lane feeds (A col / B row = lane % 4)
-      const bool in = l < l1;
-#pragma unroll
-      for (int i = 0; i < MT; ++i) {
-        const int col = 8 * i + qr;
-        fa[s][i] = (in && col < a) ? ld_any<XG>(&X[(size_t)l * lx + col]) : 0.0;
-      }
-#pragma unroll
-      for (int j = 0; j < NTL; ++j) {
-        const int col = 8 * j + qr;
-        f1[s][j] = (in && col < b1) ? ld_any<WG>(&W1[(size_t)l * lw1 + col]) : 0.0;
-        f2[s][j] = (in && col < b2) ? ld_any<WG>(&W2[(size_t)l * lw2 + col]) : 0.0;
-      }
-    }
-#pragma unroll
-    for (int s = 0; s < KS; ++s)
-#pragma unroll
-      for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int j = 0; j < NTL; ++j) {
-          if (8 * j < b1) dmma(c1[i][j][0], c1[i][j][1], fa[s][i], f1[s][j]);
-          if (8 * j < b2) dmma(c2[i][j][0], c2[i][j][1], fa[s][i], f2[s][j]);
-        }
-  }
-  constexpr int SW = 2 * KB, SL = AccumSmem<KB>::SLOT;
-  auto deposit = [&](int slot, bool add) {
-#pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-      for (int j = 0; j < NTL; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int r = 8 * i + qr, c = 8 * j + 2 * qc + e;
-          if (r < a && c < b1) {
-            double* p = &red[slot * SL + r * SW + c];
-            *p = add ? c1[i][j][e] + *p : c1[i][j][e];
-          }
-          if (r < a && c < b2) {
-            double* p = &red[slot * SL + r * SW + KB + c];
-            *p = add ? c2[i][j][e] + *p : c2[i][j][e];
-          }
-        }
-  };
-  // warps 6, 7 store, then 4, 5, then 2, 3, then 0, 1 add (two slots), then the slots are summed
-  for (int rd = 3; rd >= 0; --rd) {
-    if ((w >> 1) == rd) deposit(w & 1, rd != 3);
-    __syncthreads();
-  }
-  accum_combine<KB>(red, a, b1, b2, out1, out2, ldo);
-}
-
-// out = X^T [W1 W2]: the tensor-core form when both W are untransposed, else the SIMT form
-template <int KB, bool XG, bool WG>
-__device__ __forceinline__ void accum_tn_any(const double* X, int lx, int a, const double* W1, int lw1, bool tW1,
-                                             int b1, const double* W2, int lw2, bool tW2, int b2, int L,
-                                             double* out1, double* out2, int ldo, double* red) {
-  if (!tW1 && !tW2) accum_tn_mma<KB, XG, WG>(X, lx, a, W1, lw1, b1, W2, lw2, b2, L, out1, out2, ldo, red);
-  else accum_tn<KB, XG, WG>(X, lx, a, W1, lw1, tW1, b1, W2, lw2, tW2, b2, L, out1, out2, ldo, red);
-}
-
-// Y[l][0..k) = A1[l] S1^T + alpha A2[l] S2^T for every row l (a thread per row), S1: k x c1,
-// S2: k x c2 in shared memory (ld lds).  Y may alias A1 (each row is read before written).
-template <int KB, bool A1G>
-__device__ __noinline__ void accum_rows(double* Y, int ly, const double* A1, int la1, int c1, const double* A2,
-                                       int la2, bool tA2, int c2, double alpha, const double* S1,
-                                       const double* S2, int lds, int k, int L) {
-  for (int l = threadIdx.x; l < L; l += NT) {
-    double y[KB], u[KB];
-#pragma unroll
-    for (int j = 0; j < KB; ++j) u[j] = j < c1 ? ld_any<A1G>(&A1[(size_t)l * la1 + j]) : 0.0;
-#pragma unroll
-    for (int i = 0; i < KB; ++i) {
-      double t = 0.0;
-      if (i < k) {
-#pragma unroll
-        for (int j = 0; j < KB; ++j)
-          if (j < c1) t = fma(u[j], S1[i * lds + j], t);
-      }
-      y[i] = t;
-    }
-#pragma unroll
-    for (int j = 0; j < KB; ++j)
-      u[j] = j < c2 ? ldcg(tA2 ? &A2[(size_t)j * la2 + l] : &A2[(size_t)l * la2 + j]) : 0.0;
-#pragma unroll
-    for (int i = 0; i < KB; ++i) {
-      if (i < k) {
-        double t = 0.0;
-#pragma unroll
-        for (int j = 0; j < KB; ++j)
-          if (j < c2) t = fma(u[j], S2[i * lds + j], t);
-        y[i] = fma(alpha, t, y[i]);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < KB; ++i)
-      if (i < k) Y[(size_t)l * ly + i] = y[i];
-  }
-}
-
-// FP64 tensor-core form of accum_rows for an untransposed A2: warp w takes 8-row tiles
-// r0 = 8 (w + 8 t); Y tile (8 x k) = A1 tile S1^T + alpha A2 tile S2^T with mma.m8n8k4.f64
-// (A fragments from the rows, B fragments from S in shared memory).  A warp reads all of its
-// tile's rows before it stores any, so Y may alias A1.
-template <int KB, bool A1G>
-__device__ __noinline__ void accum_rows_mma(double* Y, int ly, const double* A1, int la1, int c1, const double* A2,
-                                           int la2, int c2, double alpha, const double* S1, const double* S2,
-                                           int lds, int k, int L) {
-  constexpr int NTL = KB / 8, KST = KB / 4;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qr = lane >> 2, qc = lane & 3;
-  for (int r0 = 8 * w; r0 < L; r0 += 8 * (NT / 32)) {
-    const int row = r0 + qr;
-    const bool rin = row < L;
-    double fa1[KST], fa2[KST];
-#pragma unroll
-    for (int s = 0; s < KST; ++s) {
-      const int col = 4 * s + qc;
-      fa1[s] = (rin && col < c1) ? ld_any<A1G>(&A1[(size_t)row * la1 + col]) : 0.0;
-      fa2[s] = (rin && col < c2) ? ldcg(&A2[(size_t)row * la2 + col]) : 0.0;
-    }
-    double y1[NTL][2], y2[NTL][2];
-#pragma unroll
-    for (int j = 0; j < NTL; ++j) y1[j][0] = y1[j][1] = y2[j][0] = y2[j][1] = 0.0;
-#pragma unroll
-    for (int s = 0; s < KST; ++s) {
-      const int kk = 4 * s + qc;
-#pragma unroll
-      for (int j = 0; j < NTL; ++j) {
-        const int n = 8 * j + qr;
-        if (4 * s < c1) dmma(y1[j][0], y1[j][1], fa1[s], (n < k && kk < c1) ? S1[n * lds + kk] : 0.0);
-        if (4 * s < c2) dmma(y2[j][0], y2[j][1], fa2[s], (n < k && kk < c2) ? S2[n * lds + kk] : 0.0);
-      }
-    }
-    if (rin) {
-#pragma unroll
-      for (int j = 0; j < NTL; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int col = 8 * j + 2 * qc + e;
-          if (col < k) Y[(size_t)row * ly + col] = fma(alpha, y2[j][e], y1[j][e]);
-        }
-    }
-  }
-}
-
-// Y = A1 S1^T + alpha A2 S2^T: the tensor-core form unless A2 is stored transposed
-template <int KB, bool A1G>
-__device__ __forceinline__ void accum_rows_any(double* Y, int ly, const double* A1, int la1, int c1, const double* A2,
-                                              int la2, bool tA2, int c2, double alpha, const double* S1,
-                                              const double* S2, int lds, int k, int L) {
-  if (!tA2) accum_rows_mma<KB, A1G>(Y, ly, A1, la1, c1, A2, la2, c2, alpha, S1, S2, lds, k, L);
-  else accum_rows<KB, A1G>(Y, ly, A1, la1, c1, A2, la2, tA2, c2, alpha, S1, S2, lds, k, L);
-}
-
-// One CholeskyQR pass on Y (m x k, ld ly): G = Y^T Y (+ shift I), G = C^T C, Y := Y C^-1.
-// A non-positive pivot marks a rank-deficient column, which is zeroed.  The Cholesky and the
-// substitution are rolled loops (a few hundred instructions): this code runs once per task in
-// a kernel whose other instructions evict it from the instruction cache, and fully unrolled
-// forms of it (thousands of instructions, each line fetched once) ran ten times longer.
-template <int KB, bool YG>
-__device__ __noinline__ void accum_cholqr(double* Y, int ly, int m, int k, bool shifted, double* G, double* red) {
-  double* rinv = G + KB * ACC_LG;
-  accum_tn_any<KB, YG, YG>(Y, ly, k, Y, ly, false, k, nullptr, 0, false, 0, m, G, nullptr, ACC_LG, red);
-  if (threadIdx.x < 32) {  // right-looking Cholesky in shared memory: row j of C over row j of G
-    const int lane = threadIdx.x;
-    double tr = 0.0;
-    for (int j = 0; j < k; ++j) tr += G[j * ACC_LG + j];
-    const double tiny = 1e-28 * tr;
-    if (shifted && lane < k) {
-      // shift of shifted CholeskyQR3: 11 (m k + k (k + 1)) u ||Y||_F^2, u = 2^-53
-      G[lane * ACC_LG + lane] += 11.0 * ((double)m * k + (double)k * (k + 1)) * 1.1102230246251565e-16 * tr;
-    }
-    __syncwarp();
-    for (int j = 0; j < k; ++j) {
-      const double d = G[j * ACC_LG + j];
-      const bool live = d > tiny;
-      const double ri = live ? rsqrt(d) : 0.0;  // 1 / c_jj
-      __syncwarp();
-      if (lane >= j && lane < k) G[j * ACC_LG + lane] = lane == j ? d * ri : G[j * ACC_LG + lane] * ri;  // C[j][lane]
-      if (lane == j) rinv[j] = ri;
-      __syncwarp();
-      // G[c1][lane] -= C[j][c1] C[j][lane] for j < c1 <= lane
-      if (lane > j && lane < k) {
-        const double cjl = G[j * ACC_LG + lane];
-        for (int c1 = j + 1; c1 <= lane; ++c1)
-          G[c1 * ACC_LG + lane] = fma(-G[j * ACC_LG + c1], cjl, G[c1 * ACC_LG + lane]);
-      }
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-  // Y := Y C^-1, a thread per row (two rows at a time, two independent chains), right-looking:
-  // x_j = s_j / c_jj, then s_c -= x_j c_jc for c > j (each s_c receives its updates in
-  // ascending j, the order of the substitution x_j = (y_j - sum_{p<j} x_p c_pj) / c_jj); x[0]
-  // is always the current column.  Positions past column k - 1 take updates from entries
-  // beyond C's rows (in bounds of G and its reciprocals) but are never stored and never feed
-  // a column below k.
-  for (int r = threadIdx.x; r < m; r += 2 * NT) {
-    const int r2 = r + NT;
-    const bool two = r2 < m;
-    double x[KB], z[KB];
-#pragma unroll
-    for (int j = 0; j < KB; ++j) {
-      x[j] = j < k ? ld_any<YG>(&Y[(size_t)r * ly + j]) : 0.0;
-      z[j] = (two && j < k) ? ld_any<YG>(&Y[(size_t)r2 * ly + j]) : 0.0;
-    }
-    for (int j = 0; j < k; ++j) {
-      const double rj = rinv[j];
-      const double xj = x[0] * rj, zj = z[0] * rj;
-      Y[(size_t)r * ly + j] = xj;
-      if (two) Y[(size_t)r2 * ly + j] = zj;
-      const double* crow = G + j * ACC_LG + j;
-#pragma unroll
-      for (int c = 1; c < KB; ++c) {
-        const double g = crow[c];
-        x[c - 1] = fma(-xj, g, x[c]);
-        z[c - 1] = fma(-zj, g, z[c]);
-      }
-      x[KB - 1] = 0.0;
-      z[KB - 1] = 0.0;
-    }
-  }
   __syncthreads();
 }
 
-// Symmetric eigen-decomposition G = Z diag(lambda) Z^T of a k x k matrix (k <= 32, shared
-// memory, ld ACC_LG) by cyclic Jacobi in round-robin order: every step rotates k/2 disjoint
-// index pairs at once (every pair once per sweep).  A step is one pass of independent 2 x 2
-// block updates: the thread of block (pair a, pair b) reads G's entries at rows {p_a, q_a} and
-// columns {p_b, q_b}, derives both pairs' rotations itself from the diagonal blocks (read before
-// any entry changes), and writes J_a^T G_ab J_b; Z's columns of pair b turn with J_b in the same
-// pass.  A pair is rotated only while |g_pq| > 1e-15 max_i g_ii: above the rounding noise a
-// rotation of the largest entries leaves behind (a few units in the last place of max g_ii, so
-// the sweeps end), and about the precision the Gram matrix has in the first place (its entries
-// are rounded to about 1e-16 of the largest); sweeps stop after one without a rotation, or after
-// 12.  The rotation of a pair is the symmetric Schur decomposition of its 2 x 2 block (Golub &
-// Van Loan, sym.schur2), t = tan(theta) written as 2 g_pq sgn(d) / (|d| + h), d = g_qq - g_pp,
-// h = sqrt(d^2 + 4 g_pq^2): cos = r / s, sin = 2 g_pq sgn(d) / s with r = |d| + h,
-// s = sqrt(r^2 + 4 g_pq^2) (one square root and one reciprocal square root).
-__device__ __forceinline__ void jacobi_pair(const double* G, int k, int kk, int r, int jp, double thr, int& p, int& q,
-                                            double& c, double& sn) {
-  // round-robin positions of pair jp in step r: 1 + (pos - 1 + r) mod (kk - 1), the sum below
-  // 2 (kk - 1); position 0 stays
-  const int pos_b = kk - 1 - jp;
-  int ua = jp - 1 + r, ub = pos_b - 1 + r;
-  if (ua >= kk - 1) ua -= kk - 1;
-  if (ub >= kk - 1) ub -= kk - 1;
-  p = jp == 0 ? 0 : 1 + ua;
-  q = pos_b == 0 ? 0 : 1 + ub;
-  if (p > q) {
-    const int t = p;
-    p = q;
-    q = t;
-  }
-  c = 1.0;
-  sn = 0.0;
-  if (q < k) {
-    const double app = G[p * ACC_LG + p], aqq = G[q * ACC_LG + q], apq = G[p * ACC_LG + q];
-    if (fabs(apq) > thr) {
-      const double d = aqq - app, g2 = 2.0 * apq * (d >= 0.0 ? 1.0 : -1.0);
-      const double h = sqrt(fma(d, d, g2 * g2)), rr = fabs(d) + h;
-      const double w = rsqrt(fma(rr, rr, g2 * g2));
-      c = rr * w;
-      sn = g2 * w;
-    }
-  }
-}
-
-__device__ __noinline__ void jacobi_eig(double* G, double* Z, int k, double* flag) {
-  const int kk = (k + 1) & ~1, np = kk / 2;  // an odd k gets a dummy index k that never rotates
-  for (int e = threadIdx.x; e < k * k; e += NT) Z[(e / k) * ACC_LG + e % k] = (e / k == e % k) ? 1.0 : 0.0;
-  // this thread's block (pair a, pair b) and, for Z, rows zi and zi + 16 of pair b
-  const int ta = threadIdx.x / 16, tb = threadIdx.x % 16;
-  const bool blk = ta < np && tb < np;
-  for (int sweep = 0; sweep < 12; ++sweep) {
-    if (threadIdx.x < 32) {
-      double dm = 0.0;
-      for (int i = threadIdx.x; i < k; i += 32) dm = fmax(dm, fabs(G[i * ACC_LG + i]));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) dm = fmax(dm, __shfl_xor_sync(0xffffffffu, dm, o));
-      if (threadIdx.x == 0) {
-        flag[0] = 0.0;  // rotations in this sweep
-        flag[1] = 1e-15 * dm;
-      }
-    }
-    __syncthreads();
-    const double thr = flag[1];
-    for (int r = 0; r < kk - 1; ++r) {
-      int pa = 0, qa = 0, pb = 0, qb = 0;
-      double ca = 1.0, sa = 0.0, cb = 1.0, sb = 0.0;
-      // pair b's rotation also turns Z's rows ta, ta + 16 (every ta, also beyond np)
-      if (tb < np) jacobi_pair(G, k, kk, r, tb, thr, pb, qb, cb, sb);
-      if (blk) jacobi_pair(G, k, kk, r, ta, thr, pa, qa, ca, sa);
-      const bool ra = sa != 0.0, rb = sb != 0.0;
-      double g11 = 0.0, g12 = 0.0, g21 = 0.0, g22 = 0.0;
-      const bool qa_in = qa < k, qb_in = qb < k;
-      if (blk && (ra || rb)) {
-        g11 = G[pa * ACC_LG + pb];
-        if (qb_in) g12 = G[pa * ACC_LG + qb];
-        if (qa_in) g21 = G[qa * ACC_LG + pb];
-        if (qa_in && qb_in) g22 = G[qa * ACC_LG + qb];
-      }
-      if (ta == tb && ra) flag[0] = 1.0;
-      __syncthreads();  // every entry is read before any changes
-      if (blk && (ra || rb)) {
-        // columns: [g11 g12; g21 g22] J_b
-        const double h11 = cb * g11 - sb * g12, h12 = sb * g11 + cb * g12;
-        const double h21 = cb * g21 - sb * g22, h22 = sb * g21 + cb * g22;
-        // rows: J_a^T [h]
-        G[pa * ACC_LG + pb] = ca * h11 - sa * h21;
-        if (qb_in) G[pa * ACC_LG + qb] = ca * h12 - sa * h22;
-        if (qa_in) G[qa * ACC_LG + pb] = sa * h11 + ca * h21;
-        if (qa_in && qb_in) G[qa * ACC_LG + qb] = sa * h12 + ca * h22;
-      }
-      if (tb < np && rb && qb_in) {  // Z J_b: rows ta and ta + 16 of pair b's columns
-        for (int i = ta; i < k; i += 16) {
-          const double zp = Z[i * ACC_LG + pb], zq = Z[i * ACC_LG + qb];
-          Z[i * ACC_LG + pb] = cb * zp - sb * zq;
-          Z[i * ACC_LG + qb] = sb * zp + cb * zq;
-        }
-      }
-      __syncthreads();
-    }
-    const bool done = flag[0] == 0.0;
-    __syncthreads();
-    if (done) break;
-  }
-}
-
-// Rank decision of the adaptive accumulation: eigenvalues (the diagonal of G) sorted in
-// decreasing order, rank r = #{ lambda_i > tol^2 lambda_0 } (singular values above tol times
-// the largest), and S[i][j] = Z[j][perm[i]] for i < r (zero rows beyond), so that a row
-// times S^T is its coordinates in the kept singular directions.  Returns r.
+// Y[l][0 .. k) = A1[l] S1^T + alpha A2[l] S2^T (A2 absent when null) for every row l, S1 and S2
+// zero-padded KB x KB blocks of stride KB + 4.  A warp takes 16 rows and reads them before it
+// writes, so Y may be A1.
 template <int KB>
-__device__ __noinline__ int accum_truncate(const double* G, const double* Z, int k, double tol, double* S, int lds,
-                                           int* perm, int rmax = PP_VM_MAX_RANK) {
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < k; ++i) perm[i] = i;
-    for (int i = 0; i < k; ++i) {
-      int best = i;
-      for (int j = i + 1; j < k; ++j)
-        if (G[perm[j] * ACC_LG + perm[j]] > G[perm[best] * ACC_LG + perm[best]]) best = j;
-      const int t = perm[i];
-      perm[i] = perm[best];
-      perm[best] = t;
+__device__ __forceinline__ void lr_rows(double* Y, int ly, const LrMat& A1, const LrMat& A2, double alpha,
+                                        const double* S1, const double* S2, int k, int L) {
+  constexpr int LD = LrSmem<KB>::LD, NJ = KB / 8, KS = KB / 4;
+  const int tid = thread_index(), warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3;
+#pragma unroll 1
+  for (int r0 = 16 * warp; r0 < L; r0 += 128) {
+    double acc[2][NJ][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) acc[h][j][0] = acc[h][j][1] = 0.0;
+#pragma unroll 1
+    for (int o = 0; o < 2; ++o) {
+      const LrMat A = o ? A2 : A1;
+      if (!A.p) continue;
+      const double* S = (o ? S2 : S1) + fa * LD + fb;
+      const double f = o ? alpha : 1.0;
+      const double* ap = A.p + (size_t)(r0 + fa) * A.sr + (size_t)fb * A.sc;
+      double a[2][KS];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int t = 0; t < KS; ++t)
+          a[h][t] = ld_if(ap + (size_t)(8 * h) * A.sr + (size_t)(4 * t) * A.sc, r0 + 8 * h + fa < L && 4 * t + fb < A.cols);
+      if (f != 1.0) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int t = 0; t < KS; ++t) a[h][t] *= f;
+      }
+#pragma unroll
+      for (int t = 0; t < KS; ++t)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          const double b = S[8 * j * LD + 4 * t];
+          dmma(acc[0][j][0], acc[0][j][1], a[0][t], b);
+          dmma(acc[1][j][0], acc[1][j][1], a[1][t], b);
+        }
     }
-    const double l0 = G[perm[0] * ACC_LG + perm[0]];
-    int r = 0;
-    if (l0 > 0.0)
-      while (r < k && r < rmax && G[perm[r] * ACC_LG + perm[r]] > tol * tol * l0) ++r;
-    perm[KB] = r;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      double* y = Y + (size_t)(r0 + 8 * h + fa) * ly + 2 * fb;
+      const bool in = r0 + 8 * h + fa < L;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        if (in && 8 * j + 2 * fb < k) y[8 * j] = acc[h][j][0];
+        if (in && 8 * j + 2 * fb + 1 < k) y[8 * j + 1] = acc[h][j][1];
+      }
+    }
   }
   __syncthreads();
-  const int r = perm[KB];
-  for (int e = threadIdx.x; e < KB * KB; e += NT) {
-    const int i = e / KB, j = e % KB;
-    S[i * lds + j] = (i < r && j < k) ? Z[j * ACC_LG + perm[i]] : 0.0;
+}
+
+// Cholesky of a Gram matrix G = Y^T Y (k x k, zero-padded) of a Y of m rows, G (+ shift) = C^T C:
+// S1 := C^-T, so that Y C^-1 = Y S1^T (one Cholesky-QR pass), or S1 := C itself (factor); G is
+// overwritten.  Elimination of [G | I] without pivoting, eight rows at a time: one warp eliminates
+// them against each other (a column of G and one of the right half per lane, the eight rows in
+// registers, multipliers by shuffles), then all warps update the rows below on the FP64 tensor cores.
+// A non-positive pivot marks a rank-deficient column, which becomes zero.  The chain of one pivot's
+// reciprocal after the other bounds it (a form with every thread on its own entries and a barrier
+// per row took three times as long).
+template <int KB>
+__device__ __forceinline__ void lr_chol(double* G, double* S1, double* misc, int k, int m, bool shifted, bool factor) {
+  constexpr int LD = LrSmem<KB>::LD;
+  const int tid = thread_index(), warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3, col = lane & (KB - 1);
+  double tr = lane < k ? G[lane * LD + lane] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
+  // an even power of two brings the trace near 1: every live pivot is then within the range of
+  // `reciprocal`
+  const int ex = (__double2hiint(tr) >> 20) & 0x7FF;
+  const int half = ex > 0 && ex < 0x7FF ? (ex - 1023) >> 1 : 0;
+  const double down = __hiloint2double((1023 - half) << 20, 0), up = __hiloint2double((1023 + half) << 20, 0);
+  const double down2 = down * down;
+  // shift of shifted CholeskyQR3: 11 (m k + k (k + 1)) u ||Y||_F^2, u = 2^-53
+  const double sh = shifted ? 11.0 * ((double)m * k + (double)k * (k + 1)) * 1.1102230246251565e-16 * (tr * down2) : 0.0;
+  const double tiny = 1e-28 * (tr * down2);
+  __syncthreads();
+  for (int e = tid; e < KB * LD; e += NT) {
+    const int r = e / LD, c = e % LD;
+    G[e] = fma(G[e], down2, (r == c && r < k) ? sh : 0.0);
+    S1[e] = r == c ? 1.0 : 0.0;
   }
   __syncthreads();
+  const int nb = (k + 7) >> 3;
+#pragma unroll 1
+  for (int J = 0; J < nb; ++J) {
+    if (warp == 0) {
+      double *g = G + 8 * J * LD + col, *s = S1 + 8 * J * LD + col;
+      double x[8], z[8], d[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        x[i] = g[i * LD];
+        z[i] = s[i * LD];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        d[i] = __shfl_sync(0xffffffffu, x[i], 8 * J + i);
+        const double ri = d[i] > tiny ? reciprocal(d[i]) : 0.0;
+#pragma unroll
+        for (int a = i + 1; a < 8; ++a) {
+          const double f = __shfl_sync(0xffffffffu, x[i], 8 * J + a) * ri;
+          x[a] = fma(-f, x[i], x[a]);
+          z[a] = fma(-f, z[i], z[a]);
+        }
+      }
+      double mine = d[0];
+#pragma unroll
+      for (int i = 1; i < 8; ++i) mine = (lane & 7) == i ? d[i] : mine;
+      const double rs = mine > tiny ? rsqrt(mine) : 0.0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const double f = __shfl_sync(0xffffffffu, rs, i);
+        if (lane < KB) {
+          g[i * LD] = x[i] * f;
+          s[i * LD] = z[i] * f;
+        }
+      }
+    }
+    __syncthreads();
+    // rows of block t below: tiles u >= t of G, tiles u <= J of the right half
+    const int items = (nb - 1 - J) * nb;
+#pragma unroll 1
+    for (int it = warp; it < items; it += NT / 32) {
+      const int t = J + 1 + it / nb, u = it % nb;
+      if (u > J && u < t) continue;
+      double* M = u <= J ? S1 : G;
+      const double *a = G + (8 * J + fb) * LD + 8 * t + fa, *b = M + (8 * J + fb) * LD + 8 * u + fa;
+      double* c = M + (8 * t + fa) * LD + 8 * u + 2 * fb;
+      double y0 = c[0], y1 = c[1];
+      dmma(y0, y1, -a[0], b[0]);
+      dmma(y0, y1, -a[4 * LD], b[4 * LD]);
+      c[0] = y0;
+      c[1] = y1;
+    }
+    __syncthreads();
+  }
+  for (int e = tid; e < KB * LD; e += NT) S1[e] = factor ? (e % LD >= e / LD ? G[e] * up : 0.0) : S1[e] * down;
+  __syncthreads();
+}
+
+// Singular directions of a matrix V from the Cholesky factor C (k x k, k rows of B, stride LD,
+// zero-padded) of its Gram matrix, V^T V = C^T C: one-sided Jacobi makes the rows of C orthogonal,
+// their norms are then V's singular values and the rows themselves, normalized, its right singular
+// vectors.  Then the rank decision: rows in decreasing order of norm, r = #{ norm_i > tol norm_0 }, at
+// most rmax, and S[i] = the i-th direction for i < r (zero rows beyond), so that a row of V times S^T
+// is its coordinates in the kept directions.  Returns r.
+//
+// The factor of a graded Gram matrix is close to row-orthogonal already: 7 or 8 sweeps where the
+// two-sided Jacobi on the Gram matrix took 12 (its limit), a third of the shared-memory traffic, and
+// the directions are orthogonal to rounding however small their singular value.  Round-robin order,
+// k/2 disjoint pairs at once, eight lanes of the first four warps per pair, which all compute its
+// rotation; one barrier of those warps per step.  A pair is rotated while |b_p . b_q| > 1e-13 |b_p| |b_q| and the smaller norm counts for the
+// rank (> 1e-2 tol of the largest); a sweep whose rotations were all below 1e-8 is the last (the next
+// would find products of such angles), and at most 14 are made.  The rotation is the symmetric
+// Schur decomposition of the pair's 2 x 2 Gram matrix (Golub & Van Loan, sym.schur2), t = tan(theta)
+// written as 2 a sgn(d) / (|d| + h), d = |b_q|^2 - |b_p|^2, h = sqrt(d^2 + 4 a^2): cos = r / s,
+// sin = 2 a sgn(d) / s with r = |d| + h, s = sqrt(r^2 + 4 a^2).  h only steers the angle and comes
+// from an estimate of the reciprocal root; 1 / s, which makes the rotation orthogonal, is corrected
+// to full precision (y (1 + e/2 + 3 e^2/8), e = 1 - s^2 y^2, binomial series).
+__device__ __forceinline__ double rsqrt_seed(double v) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+  return y;
+}
+__device__ __forceinline__ void round_robin(int kk, int r, int jp, int& p, int& q) {
+  // positions of pair jp in step r: 1 + (pos - 1 + r) mod (kk - 1); position 0 stays
+  int ua = jp - 1 + r, ub = kk - 2 - jp + r;
+  ua -= ua >= kk - 1 ? kk - 1 : 0;
+  ub -= ub >= kk - 1 ? kk - 1 : 0;
+  const int a = jp == 0 ? 0 : 1 + ua, b = kk - 1 - jp == 0 ? 0 : 1 + ub;
+  p = min(a, b);
+  q = max(a, b);
+}
+__device__ __forceinline__ double sum8(double v) {
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// barrier of the CTA's first 128 threads; whether any of them has `flag` set
+__device__ __forceinline__ int bar128_or(int flag) {
+  int r;
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.s32 q, %1, 0;\n barrier.cta.red.or.pred p, 1, 128, q;\n selp.b32 %0, 1, 0, p;\n}\n"
+      : "=r"(r)
+      : "r"(flag)
+      : "memory");
   return r;
 }
-
-template <int KB, bool YG>
-__device__ __forceinline__ void accum_impl(const pp_task& T, double* smem) {
-  using SM = AccumSmem<KB>;
-  const int ny = T.m, nx = T.n, k1 = T.k, k2 = T.l;
-  const bool tU2 = T.flags & PP_T(2), tV2 = T.flags & PP_T(3);
-  double *U1 = T.p[0], *V1 = T.p[1];
-  const double *U2 = T.p[2], *V2 = T.p[3], *R = T.p[4];
-  const int lu1 = T.ld[0], lv1 = T.ld[1], lu2 = T.ld[2], lv2 = T.ld[3], lr = T.ld[4];
-  double* red = smem;
-  double* S = red + SM::SOFF;  // k1 x 2KB: S1 | S2, later P1 | P2
-  double* G = red + SM::RED;
-  double* Y = YG ? T.tmp : G + SM::G;
-  const int ly = YG ? k1 : k1 + 1;  // on chip: rows padded (a thread per row reads distinct banks)
-  const double al = T.alpha;
-  constexpr int LS = 2 * KB;
-  // S1 = R^T V1, S2 = R^T V2
-  accum_tn_any<KB, true, true>(R, lr, k1, V1, lv1, false, k1, V2, lv2, tV2, k2, nx, S, S + KB, LS, red);
-  // Y = U1 S1^T + alpha U2 S2^T
-  accum_rows_any<KB, true>(Y, ly, U1, lu1, k1, U2, lu2, tU2, k2, al, S, S + KB, LS, k1, ny);
-  __syncthreads();
-  accum_cholqr<KB, YG>(Y, ly, ny, k1, true, G, red);
-  accum_cholqr<KB, YG>(Y, ly, ny, k1, false, G, red);
-  accum_cholqr<KB, YG>(Y, ly, ny, k1, false, G, red);
-  // P1 = Y^T U1, P2 = Y^T U2
-  accum_tn_any<KB, YG, true>(Y, ly, k1, U1, lu1, false, k1, U2, lu2, tU2, k2, ny, S, S + KB, LS, red);
-  // V1 := V1 P1^T + alpha V2 P2^T (rows read before written)
-  accum_rows_any<KB, true>(V1, lv1, V1, lv1, k1, V2, lv2, tV2, k2, al, S, S + KB, LS, k1, nx);
-  __syncthreads();
-  if ((T.flags & PP_ADAPT_RANK) && T.beta > 0.0) {
-    // adaptive rank: U1 V1^T = Y V1^T with Y orthonormal, so the singular values are those of
-    // V1; rotate both factors into the eigenbasis of V1^T V1 and keep the directions whose
-    // singular value exceeds beta times the largest (zero columns beyond the new rank)
-    accum_tn_any<KB, true, true>(V1, lv1, k1, V1, lv1, false, k1, nullptr, 0, false, 0, nx, G, nullptr, ACC_LG, red);
-    double* Z = red;
-    double* cs = red + KB * ACC_LG;
-    double* flag = cs + 2 * KB;
-    int* pq = reinterpret_cast<int*>(flag + 2);
-    jacobi_eig(G, Z, k1, flag);
-    const int r = accum_truncate<KB>(G, Z, k1, T.beta, S, LS, pq);
-    accum_rows_any<KB, true>(V1, lv1, V1, lv1, k1, nullptr, 0, false, 0, 1.0, S, S, LS, k1, nx);
-    accum_rows_any<KB, YG>(Y, ly, Y, ly, k1, nullptr, 0, false, 0, 1.0, S, S, LS, k1, ny);
-    __syncthreads();
-    if (threadIdx.x == 0 && T.p[5]) T.p[5][0] = (double)r;
+template <int KB>
+__device__ __forceinline__ void lr_norms(const double* B, double* n2, int tid) {
+  constexpr int LD = LrSmem<KB>::LD;
+#pragma unroll
+  for (int h = 0; h < KB; h += 16) {
+    const double* b = B + ((tid >> 3) + h) * LD + (tid & 7);
+    double s = 0.0;
+#pragma unroll
+    for (int i = 0; i < KB; i += 8) s = fma(b[i], b[i], s);
+    s = sum8(s);
+    if ((tid & 7) == 0) n2[(tid >> 3) + h] = s;
   }
-  // U1 := Y
-  for (int e = threadIdx.x; e < ny * k1; e += NT) {
-    const int r = e / k1, c = e % k1;
-    U1[(size_t)r * lu1 + c] = ld_any<YG>(&Y[(size_t)r * ly + c]);
+}
+template <int KB>
+__device__ __forceinline__ int lr_svd(double* B, double* S, double* misc, int k, double tol, int rmax) {
+  constexpr int LD = LrSmem<KB>::LD, NE = KB / 8;
+  // an odd k gets a row k of zeros (B is zero-padded), which never rotates
+  const int tid = thread_index(), lane = tid & 31, kk = (k + 1) & ~1, np = kk / 2, pair = tid >> 3, l = tid & 7;
+  double* n2 = misc;  // squared norms
+  int* perm = reinterpret_cast<int*>(misc + 32);
+  if (tid < 128) {
+#pragma unroll 1
+    for (int sweep = 0; sweep < 14; ++sweep) {
+      lr_norms<KB>(B, n2, tid);
+      bar128_or(0);
+      double top = n2[lane & (KB - 1)];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+      const double floor2 = 1e-4 * tol * tol * top;
+      int seen = 0;
+#pragma unroll 1
+      for (int r = 0; r < kk - 1; ++r) {
+        int p, q;
+        round_robin(kk, r, min(pair, np - 1), p, q);
+        double *bp = B + p * LD + l, *bq = B + q * LD + l;
+        double x[NE], y[NE], dot = 0.0;
+#pragma unroll
+        for (int i = 0; i < NE; ++i) {
+          x[i] = bp[8 * i];
+          y[i] = bq[8 * i];
+        }
+#pragma unroll
+        for (int i = 0; i < NE; ++i) dot = fma(x[i], y[i], dot);
+        const double app = n2[p], aqq = n2[q], a = sum8(dot);
+        const double d = aqq - app, g2 = d >= 0.0 ? 2.0 * a : -2.0 * a, gg = g2 * g2, v = fma(d, d, gg);
+        const double rr = fma(v, rsqrt_seed(v), fabs(d)), s2 = fma(rr, rr, gg), y0 = rsqrt_seed(s2);
+        const double e = fma(-s2 * y0, y0, 1.0), w = fma(y0 * e, fma(0.375, e, 0.5), y0);
+        const double a2 = a * a, both = app * aqq;
+        const int rot = (int)(a2 > 1e-26 * both) & (int)(fmin(app, aqq) > floor2) & (int)(v > 1e-280) &
+                        (int)(s2 < 1e280) & (int)(pair < np);
+        if (rot) {
+          const double c = rr * w, sn = g2 * w;
+#pragma unroll
+          for (int i = 0; i < NE; ++i) {
+            bp[8 * i] = fma(c, x[i], -sn * y[i]);
+            bq[8 * i] = fma(sn, x[i], c * y[i]);
+          }
+          if (l == 0) {
+            n2[p] = fma(c * c, app, fma(sn * sn, aqq, -2.0 * c * sn * a));
+            n2[q] = fma(sn * sn, app, fma(c * c, aqq, 2.0 * c * sn * a));
+          }
+        }
+        seen |= rot & (int)(a2 > 1e-16 * both);
+        asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
+      }
+      if (!bar128_or(seen)) break;
+    }
+    lr_norms<KB>(B, n2, tid);
   }
   __syncthreads();
+  // the place of norm_i among the others (equal ones in index order)
+  const double mine = lane < k ? n2[lane & (KB - 1)] : -1.0;
+  double top = mine;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+  int place = 0;
+  for (int j = 0; j < k; ++j) {
+    const double v = n2[j];
+    place += (v > mine || (v == mine && j < lane)) ? 1 : 0;
+  }
+  const unsigned kept = __ballot_sync(0xffffffffu, lane < k && top > 0.0 && mine > tol * tol * top);
+  if (tid < k) {
+    perm[place] = tid;
+    misc[64 + place] = mine > 0.0 ? rsqrt(mine) : 0.0;
+  }
+  __syncthreads();
+  const int rank = min(__popc(kept), rmax);
+  for (int e = tid; e < KB * KB; e += NT) {
+    const int i = e / KB, j = e % KB;
+    S[i * LD + j] = (i < rank && j < k) ? B[perm[i] * LD + j] * misc[64 + i] : 0.0;
+  }
+  __syncthreads();
+  return rank;
 }
 
-// Y (m x k, ld k, global) := an orthonormal basis of its range by shifted CholeskyQR3, the
-// range finder of the sketched low-rank update (same passes as inside ACCUM); a Y of up to the
-// sketch capacity is copied to shared memory for the three passes and back
 template <int KB>
-__device__ __forceinline__ void orth_impl(double* Y, int m, int k, double* smem) {
-  using SM = AccumSmem<KB>;
-  double* red = smem;
-  double* G = red + SM::RED;
-  const int total = m * k, ls = k + 1;
-  if ((long long)m * ls <= SM::YCAP) {
-    double* Ys = G + SM::G;  // rows padded to k + 1
-    for (int e0 = threadIdx.x; e0 < total; e0 += 8 * NT) {
-      double v[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) v[q] = e0 + q * NT < total ? ldcg(&Y[e0 + q * NT]) : 0.0;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int e = e0 + q * NT;
-        if (e < total) Ys[(e / k) * ls + e % k] = v[q];
-      }
-    }
+__device__ __forceinline__ void lowrank_impl(const pp_task& T) {
+  extern __shared__ __align__(16) double vm_smem[];
+  using SM = LrSmem<KB>;
+  double *S1 = vm_smem + SM::S1, *S2 = vm_smem + SM::S2, *G = vm_smem + SM::G, *misc = vm_smem + SM::MISC;
+  const bool accum = T.op == PP_OP_ACCUM, orth = T.op == PP_OP_ORTH;
+  const int m = T.m, n = T.n, k = orth ? T.n : T.k, k2 = accum ? T.l : 0;
+  const bool on_chip = (accum || orth) && accum_y_on_chip(m, k, k2);
+  const int pad = (long long)m * (k + 4) <= SM::YCAP ? 4 : (long long)m * (k + 2) <= SM::YCAP ? 2 : 1;
+  double* U = T.p[0];
+  double* Y = on_chip ? vm_smem + SM::Y : accum ? T.tmp : U;
+  const int ly = on_chip ? k + pad : accum ? k : T.ld[0];
+  const bool adapt = !orth && (!accum || ((T.flags & PP_ADAPT_RANK) && T.beta > 0.0));
+  const LrMat none{nullptr, 0, 0, 0};
+  const LrMat My{Y, ly, 1, k}, Mu{U, T.ld[0], 1, k}, Mv{T.p[1], T.ld[1], 1, k};
+  LrMat Mu2 = none, Mv2 = none;
+  if (accum && k2 > 0) {
+    Mu2 = (T.flags & PP_T(2)) ? LrMat{T.p[2], 1, T.ld[2], k2} : LrMat{T.p[2], T.ld[2], 1, k2};
+    Mv2 = (T.flags & PP_T(3)) ? LrMat{T.p[3], 1, T.ld[3], k2} : LrMat{T.p[3], T.ld[3], 1, k2};
+  }
+  if (orth && on_chip) {
+    for (int e = threadIdx.x; e < m * k; e += NT) Y[(e / k) * ly + e % k] = ldcg(&U[e]);
     __syncthreads();
-    accum_cholqr<KB, false>(Ys, ls, m, k, true, G, red);
-    accum_cholqr<KB, false>(Ys, ls, m, k, false, G, red);
-    accum_cholqr<KB, false>(Ys, ls, m, k, false, G, red);
-    for (int e = threadIdx.x; e < total; e += NT) Y[e] = Ys[(e / k) * ls + e % k];
+  }
+  // without a tolerance or a smaller limit there is nothing to truncate
+  const int rmax = (!accum && T.o > 0) ? min(T.o, k) : k;
+  int rank = k;
+  if (!accum && !orth && T.beta <= 0.0 && rmax == k) {
+    if (threadIdx.x == 0 && T.p[5]) T.p[5][0] = (double)rank;
     __syncthreads();
     return;
   }
-  accum_cholqr<KB, true>(Y, k, m, k, true, G, red);
-  accum_cholqr<KB, true>(Y, k, m, k, false, G, red);
-  accum_cholqr<KB, true>(Y, k, m, k, false, G, red);
-}
-
-// U V^T (U: m x k orthonormal columns, V: n x k, both global) := its best rank-r form: the
-// singular values are those of V; rotate both factors into the eigenbasis of V^T V (Jacobi)
-// and keep the directions above tol times the largest (at most rmax), as ACCUM's adaptive form
-template <int KB>
-__device__ __forceinline__ void lrtrunc_impl(const pp_task& T, double* smem) {
-  using SM = AccumSmem<KB>;
-  constexpr int LS = 2 * KB;
-  double *U = T.p[0], *V = T.p[1];
-  const int lu = T.ld[0], lv = T.ld[1], m = T.m, n = T.n, k = T.k;
-  double* red = smem;
-  double* S = red + SM::SOFF;
-  double* G = red + SM::RED;
-  accum_tn_any<KB, true, true>(V, lv, k, V, lv, false, k, nullptr, 0, false, 0, n, G, nullptr, ACC_LG, red);
-  double* Z = red;
-  double* cs = red + KB * ACC_LG;
-  double* flag = cs + 2 * KB;
-  int* pq = reinterpret_cast<int*>(flag + 2);
-  jacobi_eig(G, Z, k, flag);
-  const int r = accum_truncate<KB>(G, Z, k, T.beta, S, LS, pq, T.o > 0 ? T.o : k);
-  accum_rows_any<KB, true>(V, lv, V, lv, k, nullptr, 0, false, 0, 1.0, S, S, LS, k, n);
-  accum_rows_any<KB, true>(U, lu, U, lu, k, nullptr, 0, false, 0, 1.0, S, S, LS, k, m);
-  __syncthreads();
-  if (threadIdx.x == 0 && T.p[5]) T.p[5][0] = (double)r;
+  // phases: 0 the sketch, 1-3 the Cholesky-QR passes, 4 the projection, 5 the truncation of V and
+  // 6 of the orthonormal factor
+#pragma unroll 1
+  for (int ph = accum ? 0 : orth ? 1 : 5; ph <= (orth ? 3 : adapt ? 6 : 4); ++ph) {
+    if (ph < 6) {
+      const LrMat X = ph == 0 ? LrMat{T.p[4], T.ld[4], 1, k} : ph == 5 ? Mv : My;
+      const LrMat W1 = ph == 0 || ph == 5 ? Mv : ph == 4 ? Mu : My;
+      const LrMat W2 = ph == 0 ? Mv2 : ph == 4 ? Mu2 : none;
+      const bool gram = ph != 0 && ph != 4;
+      lr_tn<KB>(X, W1, W2, ph == 0 || ph == 5 ? n : m, gram ? G : S1, S2);
+      if (ph >= 1 && ph != 4) lr_chol<KB>(G, S1, misc, k, m, ph == 1, ph == 5);
+      if (ph == 5) rank = lr_svd<KB>(S1, S2, misc, k, T.beta, rmax);
+    }
+    const bool first = ph == 0 || ph == 4;
+    // the factor's last product writes it where it belongs
+    double* out = ph == 4 || ph == 5 ? T.p[1] : ph == 6 || (orth && ph == 3) ? U : Y;
+    const int lo = ph == 4 || ph == 5 ? T.ld[1] : ph == 6 || (orth && ph == 3) ? T.ld[0] : ly;
+    const LrMat A1 = ph == 0 ? Mu : ph == 4 || ph == 5 ? Mv : (ph == 6 && !accum) ? Mu : My;
+    lr_rows<KB>(out, lo, A1, first ? (ph == 0 ? Mu2 : Mv2) : none, T.alpha, ph >= 5 ? S2 : S1, S2, k,
+                ph == 4 || ph == 5 ? n : m);
+  }
+  if (accum && !adapt) {  // U1 := Y
+    for (int e = threadIdx.x; e < m * k; e += NT) U[(size_t)(e / k) * T.ld[0] + e % k] = Y[(size_t)(e / k) * ly + e % k];
+  }
+  if (adapt && threadIdx.x == 0 && T.p[5]) T.p[5][0] = (double)rank;
   __syncthreads();
 }
 
-__device__ __noinline__ void dev_lrtrunc(const pp_task& T, double* smem) {
-  if (T.k <= 16) lrtrunc_impl<16>(T, smem);
-  else lrtrunc_impl<32>(T, smem);
+__device__ __forceinline__ void dev_lowrank(const pp_task& T) {
+  const int k = T.op == PP_OP_ORTH ? T.n : T.k;
+  if (k <= 16 && (T.op != PP_OP_ACCUM || T.l <= 16)) lowrank_impl<16>(T);
+  else lowrank_impl<32>(T);
 }
 
 __device__ __noinline__ void dev_kmul(const pp_task& T, double* smem);
-
-__device__ __noinline__ void dev_orth(double* Y, int m, int k, double* smem) {
-  if (k <= 16) orth_impl<16>(Y, m, k, smem);
-  else orth_impl<32>(Y, m, k, smem);
-}
 
 // C[m x n] := A[m x n]
 __device__ __noinline__ void dev_copy(double* C, int ldc, const double* A, int lda, int m, int n) {
@@ -2289,18 +2117,6 @@ __device__ __noinline__ void dev_copy(double* C, int ldc, const double* A, int l
     C[(size_t)r * ldc + c] = ldcg(&A[(size_t)r * lda + c]);
   }
   __syncthreads();
-}
-
-__device__ __noinline__ void dev_accum(const pp_task& T, double* smem) {
-  const int ny = T.m, k1 = T.k, k2 = T.l;
-  const bool on_chip = accum_y_on_chip(ny, k1, k2);
-  if (k1 <= 16 && k2 <= 16) {
-    if (on_chip) accum_impl<16, false>(T, smem);
-    else accum_impl<16, true>(T, smem);
-  } else {
-    if (on_chip) accum_impl<32, false>(T, smem);
-    else accum_impl<32, true>(T, smem);
-  }
 }
 
 // C[m x n] := beta C + sum_p T_p (p ascending), T_p the p-th m x n block of T
@@ -2366,8 +2182,7 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
     case PP_OP_GEMM4: break;
     case PP_OP_ACCUM:
       if (T.k > PP_VM_MAX_RANK || T.k < 1 || T.l > PP_VM_MAX_RANK || T.l < 0) return false;
-      dev_accum(T, smem);
-      return true;
+      break;
     case PP_OP_SUM:
       dev_sum(T.p[0], T.ld[0], T.p[1], T.ld[1], T.m, T.n, T.k, T.beta);
       return true;
@@ -2377,8 +2192,7 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
     case PP_OP_TRMV: return dev_trmv(T, smem);
     case PP_OP_ORTH:
       if (T.n < 1 || T.n > PP_VM_MAX_RANK || T.ld[0] != T.n) return false;
-      dev_orth(T.p[0], T.m, T.n, smem);
-      return true;
+      break;
     case PP_OP_COPY:
       dev_copy(T.p[0], T.ld[0], T.p[1], T.ld[1], T.m, T.n);
       return true;
@@ -2389,8 +2203,7 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
       return true;
     case PP_OP_LRTRUNC:
       if (T.k < 1 || T.k > PP_VM_MAX_RANK || T.m < T.k || T.n < T.k) return false;
-      dev_lrtrunc(T, smem);
-      return true;
+      break;
     case PP_OP_SHADOW:
       if (T.m < 32 || T.k < 64 || T.k % 64) return false;
       if (T.l < 0 || T.l > T.m || T.n < 0 || T.n > T.k) return false;
@@ -2401,7 +2214,8 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
       return true;
     default: return false;
   }
-  run_composite(T);
+  if (T.op == PP_OP_ACCUM || T.op == PP_OP_ORTH || T.op == PP_OP_LRTRUNC) dev_lowrank(T);
+  else run_composite(T);
   return true;
 }
 
@@ -3131,7 +2945,7 @@ __global__ void absmax2_kernel(const double* __restrict__ x, const double* __res
 // One ACCUM on caller buffers; its scratch (T.tmp) is the static array below.
 __global__ void __launch_bounds__(NT) accum_noalloc_kernel(pp_task T) {
   extern __shared__ __align__(16) double smem[];
-  dev_accum(T, smem);
+  dev_lowrank(T);
 }
 
 }  // namespace
@@ -3146,7 +2960,7 @@ static __device__ __align__(256) double g_accum_noalloc_scratch[PP_NOALLOC_SCRAT
 long long pp_accum_noalloc_capacity() { return PP_NOALLOC_SCRATCH_DOUBLES; }
 
 long long pp_accum_scratch_doubles(long long ny, int k1, int k2) {
-  // dev_accum keeps the ny x k1 sketch Y in shared memory while it fits beside the rest of the
+  // dev_lowrank keeps the ny x k1 sketch Y in shared memory while it fits beside the rest of the
   // 180 KB; only a larger Y goes to the task's scratch, and nothing else does
   return accum_y_on_chip(ny, k1, k2) ? 0 : ny * k1;
 }
