@@ -340,10 +340,6 @@ __device__ __forceinline__ void dev_gemm(double* __restrict__ C, int ldc, const 
   __syncthreads();
 }
 
-template <int NB, int RU, int TC>
-__device__ __noinline__ void trmv_impl(double* O, int ldo, const double* S, int lds, const double* M, int ldm, int m,
-                                       int n, int mode, int rbeg, int rows, double* smem);
-
 // ------------------------------------------------------------------------- tensor-core GEMM
 // Mixed-precision contraction on the 5th-generation tensor cores:
 //   C[m x n] (FP64) = beta C + alpha op(A) op(B),  op(A), op(B) rounded to TF32,
@@ -1376,92 +1372,110 @@ __device__ __forceinline__ void dev_tri(int op, double* B, int ldb, const double
   __syncthreads();
 }
 
-// ------------------------------------------------------------------------- TRINV / TRMV
-// Explicit inverses of a factored diagonal leaf (factor phase) and their application (solve
-// phase).  A solve then costs one triangular matrix-vector product per leaf, whose loads are
-// all independent, instead of a substitution whose steps form a chain.
-
-// Rows [r0, r0 + rows) of M S into O (row r at O row r - r0), M (m x m, m <= 32 TC) lower
-// (mode 0) or upper (mode 1) triangular or full (mode 2, then any number of rows), S (m x n);
-// O := beta O + alpha (M S) (alpha 1, beta 0 for the solves' inverses).  S is staged in shared memory first (so O may be S itself);
-// warp w takes RU rows at a time, lanes stride the columns, and every load of the RU rows is
-// issued before the first product; a warp reduction per row and right-hand side finishes the
-// dot products, so a row's result does not depend on which rows the call covers.
-template <int NB, int RU, int TC>
-__device__ __noinline__ void trmv_impl(double* O, int ldo, const double* S, int lds, const double* M, int ldm, int m,
-                                       int n, int mode, int rbeg, int rows, double* smem) {
-  // S staged as m rows of NB values, row stride NB + 1 for NB > 1: the lanes of a warp read
-  // consecutive rows, which then fall in distinct shared-memory banks
-  constexpr int SB = NB > 1 ? NB + 1 : 1;
-  double* Bs = smem;
-  for (int e = threadIdx.x; e < m * NB; e += NT) {
-    const int r = e / NB, q = e % NB;
-    Bs[r * SB + q] = q < n ? ldcg(&S[(size_t)r * lds + q]) : 0.0;
+// ------------------------------------------------------------------------- skinny products
+// Rows of a matrix times a few right-hand sides: rows [0, rows) of M S into O, M's row r at M + r ldm
+// (m columns), S m x n (n <= 16), O := beta O + alpha (M S).  tri 0: M lower triangular, tri 1: upper
+// (diagonal included; row r of the call is row r0 + r of the triangle), tri 2: full.  O may be S.
+// The explicit inverses of the leaves (TRMV) and the solves' products with a leaf or a low-rank
+// factor: S is staged in shared memory, a warp takes eight rows of M at a time straight from global
+// memory into FP64 tensor-core fragments, two columns per load (the k order is free: even columns in
+// one chain, odd ones in another), sixteen loads in flight per lane; nothing of a row depends on
+// which other rows the call covers.  Bound by one CTA's loads.  On a B200, hop of 2.5 us included
+// (before: warps along the columns, a shuffle reduction per row and right-hand side):
+//   TRMV 128 x 4, 64 rows  13 -> 6 us    94 x 1  13.5 -> 6 us    512 x 8, 64 rows  31 -> 12 us
+//   products 64 x 8 x 512  15 -> 12 us   61 x 4 x 64  5.5 -> 4 us  (the latter from the general routine)
+#define RW_U 8  /* steps of 8 columns whose loads go out together */
+__device__ __forceinline__ void dev_rows(double* O, int ldo, const double* M, int ldm, const double* S, int lds, int m,
+                                         int n, int rows, int tri, int r0, double alpha, double beta) {
+  extern __shared__ __align__(16) double vm_smem[];
+  const int tid = thread_index(), warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3;
+  const int ns = n <= 8 ? 8 : 16, ls = ns + 2, lm = (m + 7) & ~7;  // stride 2 mod 8: no bank conflicts
+#pragma unroll 4
+  for (int e = tid; e < lm * ns; e += NT) {
+    const int r = n <= 8 ? e >> 3 : e >> 4, q = e & (ns - 1);
+    vm_smem[r * ls + q] = ldcg_if(S + (size_t)r * lds + q, r < m && q < n);
   }
+  const bool wide = !((ldm | (int)(reinterpret_cast<uintptr_t>(M) >> 3)) & 1);
   __syncthreads();
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rend = rbeg + rows;
-  for (int r0 = rbeg + w * RU; r0 < rend; r0 += (NT / 32) * RU) {
-    double v[RU][TC];
+#pragma unroll 1
+  for (int t = 8 * warp; t < rows; t += 64) {
+    const int r = t + fa;
+    const bool rin = r < rows;
+    // columns the eight rows have entries in
+    const int cb = tri == 1 ? (r0 + t) & ~7 : 0, ce = tri == 0 ? min(m, r0 + t + 8) : m;
+    const double* row = M + (size_t)(rin ? r : 0) * ldm;
+    double acc[2][2][2];
 #pragma unroll
-    for (int u = 0; u < RU; ++u)
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int t = 0; t < TC; ++t) {
-        const int r = r0 + u, c = lane + 32 * t;
-        const bool in = r < rend && c < m && (mode == 2 || (mode == 1 ? c >= r : c <= r));
-        v[u][t] = in ? ldcg(&M[(size_t)r * ldm + c]) : 0.0;
+      for (int j = 0; j < 2; ++j) acc[h][j][0] = acc[h][j][1] = 0.0;
+    // a block of 64 columns in registers: even and odd columns of each step of 8
+    auto load = [&](int c0, double (&v)[RW_U][2]) {
+      const double* p = row + c0 + 2 * fb;
+      if (wide && c0 + 8 * RW_U <= m) {
+#pragma unroll
+        for (int u = 0; u < RW_U; ++u) {
+          const double2 x = __ldcg(reinterpret_cast<const double2*>(p + 8 * u));
+          v[u][0] = x.x;
+          v[u][1] = x.y;
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < RW_U; ++u) {
+          const int c = c0 + 8 * u + 2 * fb;
+          v[u][0] = ldcg_if(p + 8 * u, c < m);
+          v[u][1] = ldcg_if(p + 8 * u + 1, c + 1 < m);
+        }
       }
+    };
+    double v[RW_U][2], w[RW_U][2], old[2][2];
+    load(cb, v);
+    double* o = O + (size_t)r * ldo + 2 * fb;
 #pragma unroll
-    for (int u = 0; u < RU; ++u) {
-      double acc[NB];
+    for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int q = 0; q < NB; ++q) acc[q] = 0.0;
+      for (int e = 0; e < 2; ++e) old[j][e] = ldcg_if(o + 8 * j + e, rin && 8 * j + 2 * fb + e < n && beta != 0.0);
+#pragma unroll 1
+    for (int c0 = cb; c0 < ce; c0 += 8 * RW_U) {
+      if (c0 + 8 * RW_U < ce) load(c0 + 8 * RW_U, w);
+      if ((tri == 0 && c0 + 8 * RW_U > r0 + t) || (tri == 1 && c0 < r0 + t + 8)) {
+        // what lies outside the triangle is not used as a value
 #pragma unroll
-      for (int t = 0; t < TC; ++t) {
-        const int c = lane + 32 * t;
-        if (c < m) {
-#pragma unroll
-          for (int q = 0; q < NB; ++q) acc[q] = fma(v[u][t], Bs[c * SB + q], acc[q]);
+        for (int u = 0; u < RW_U; ++u) {
+          const int c = c0 + 8 * u + 2 * fb, d = r0 + r;
+          v[u][0] = (tri == 0 ? c <= d : c >= d) ? v[u][0] : 0.0;
+          v[u][1] = (tri == 0 ? c + 1 <= d : c + 1 >= d) ? v[u][1] : 0.0;
         }
       }
 #pragma unroll
-      for (int q = 0; q < NB; ++q) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+      for (int u = 0; u < RW_U; ++u) {
+        const double* b = vm_smem + min(c0 + 8 * u + 2 * fb, lm - 2) * ls + fa;
+        dmma(acc[0][0][0], acc[0][0][1], v[u][0], b[0]);
+        dmma(acc[1][0][0], acc[1][0][1], v[u][1], b[ls]);
+        if (n > 8) {
+          dmma(acc[0][1][0], acc[0][1][1], v[u][0], b[8]);
+          dmma(acc[1][1][0], acc[1][1][1], v[u][1], b[ls + 8]);
+        }
       }
-      const int r = r0 + u;
-      if (lane == 0 && r < rend) {
 #pragma unroll
-        for (int q = 0; q < NB; ++q)
-          if (q < n) {
-            O[(size_t)(r - rbeg) * ldo + q] = acc[q];
-          }
+      for (int u = 0; u < RW_U; ++u) {
+        v[u][0] = w[u][0];
+        v[u][1] = w[u][1];
       }
     }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        st_if(o + 8 * j + e, fma(alpha, acc[0][j][e] + acc[1][j][e], old[j][e]), rin && 8 * j + 2 * fb + e < n);
+      }
   }
   __syncthreads();
 }
 
 // TRMV: the whole product in place (l == 0) or rows [o, o + l) of it out of place (l > 0)
-__device__ __forceinline__ bool dev_trmv(const pp_task& T, double* smem) {
-  const int m = T.m, n = T.n;
-  if (m > PP_VM_INV || n < 1 || n > 16) return false;
-  const bool part = T.l > 0;
-  if (part && (T.o < 0 || T.o + T.l > m || !T.p[2])) return false;
-  const double* S = part ? T.p[2] : T.p[0];
-  const int lds = part ? T.ld[2] : T.ld[0], r0 = part ? T.o : 0, rows = part ? T.l : m;
-  if (m <= 256) {
-    if (n == 1) trmv_impl<1, 8, 8>(T.p[0], T.ld[0], S, lds, T.p[1], T.ld[1], m, n, T.ctrl, r0, rows, smem);
-    else if (n <= 4) trmv_impl<4, 4, 8>(T.p[0], T.ld[0], S, lds, T.p[1], T.ld[1], m, n, T.ctrl, r0, rows, smem);
-    else if (n <= 8) trmv_impl<8, 2, 8>(T.p[0], T.ld[0], S, lds, T.p[1], T.ld[1], m, n, T.ctrl, r0, rows, smem);
-    else trmv_impl<16, 2, 8>(T.p[0], T.ld[0], S, lds, T.p[1], T.ld[1], m, n, T.ctrl, r0, rows, smem);
-  } else {  // leaves of up to 512 rows: 16 columns per lane, half the rows per pass of loads
-    if (n == 1) trmv_impl<1, 4, 16>(T.p[0], T.ld[0], S, lds, T.p[1], T.ld[1], m, n, T.ctrl, r0, rows, smem);
-    else if (n <= 4) trmv_impl<4, 2, 16>(T.p[0], T.ld[0], S, lds, T.p[1], T.ld[1], m, n, T.ctrl, r0, rows, smem);
-    else if (n <= 8) trmv_impl<8, 2, 16>(T.p[0], T.ld[0], S, lds, T.p[1], T.ld[1], m, n, T.ctrl, r0, rows, smem);
-    else trmv_impl<16, 1, 16>(T.p[0], T.ld[0], S, lds, T.p[1], T.ld[1], m, n, T.ctrl, r0, rows, smem);
-  }
-  return true;
+__device__ __forceinline__ bool trmv_ok(const pp_task& T) {
+  return T.m <= PP_VM_INV && T.n >= 1 && T.n <= 16 && (T.l <= 0 || (T.o >= 0 && T.o + T.l <= T.m && T.p[2]));
 }
 
 // ------------------------------------------------------------------------- composite instructions
@@ -1596,48 +1610,6 @@ __device__ __forceinline__ bool tri_step(int op, double* B, int ldb, const doubl
     P.A = T + d;
   }
   return true;
-}
-
-__device__ __forceinline__ void run_composite(const pp_task& T) {
-  const bool product = T.op == PP_OP_GEMM || T.op == PP_OP_GEMM3 || T.op == PP_OP_GEMM4;
-  const bool free_order = T.op == PP_OP_GEMM && (T.flags & PP_FREE_ORDER);
-  int op = T.op, size = T.op == PP_OP_TRSMR ? T.n : T.m, lines = T.op == PP_OP_TRSMR ? T.m : T.n;
-  double* B = T.p[0];
-  const double* A = T.p[1];
-  const int ldb = T.ld[0], lda = T.ld[1];
-  if (T.op == PP_OP_TRINV) {
-    // columns [o, o + n) of L^-1 (ctrl 0) or U^-1 (1): identity columns, then the solve on the
-    // sub-triangle they need (rows o.. of L^-1 are the only nonzeros; rows ..o + n of U^-1)
-    const int w = T.n, c0 = T.o;
-    for (int e = threadIdx.x; e < T.m * w; e += NT) {
-      const int r = e / w, j = e % w;
-      B[(size_t)r * ldb + j] = r == c0 + j ? 1.0 : 0.0;
-    }
-    __syncthreads();
-    op = T.ctrl ? PP_OP_TRSMU : PP_OP_TRSML;
-    size = T.ctrl ? c0 + w : T.m - c0;
-    lines = w;
-    if (!T.ctrl) {
-      B += (size_t)c0 * ldb;
-      A += (size_t)c0 * lda + c0;
-    }
-  }
-#pragma unroll 1
-  for (int step = 0;; ++step) {
-    Product P;
-    if (product) {
-      if (!chain_step(T, step, P)) break;
-    } else {
-      int d = 0, len = 0;
-      if (!tri_step(op, B, ldb, A, lda, size, lines, step, d, len, P)) break;
-      if (!(step & 1)) {
-        double* Bd = B + (op == PP_OP_TRSMR ? (size_t)d : (size_t)d * ldb);
-        dev_tri(op, Bd, ldb, A + (size_t)d * lda + d, lda, len, lines, (T.flags & PP_PIVOT) ? T.p[2] : nullptr);
-        continue;
-      }
-    }
-    dev_gemm(P.C, P.ldc, P.A, P.lda, P.tA, P.B, P.ldb, P.tB, P.m, P.n, P.k, P.alpha, P.beta, free_order);
-  }
 }
 
 // ------------------------------------------------------------------------- low-rank instructions
@@ -2110,11 +2082,117 @@ __device__ __forceinline__ void dev_lowrank(const pp_task& T) {
 
 __device__ __noinline__ void dev_kmul(const pp_task& T, double* smem);
 
-// C[m x n] := A[m x n]
-__device__ __noinline__ void dev_copy(double* C, int ldc, const double* A, int lda, int m, int n) {
-  for (int e = threadIdx.x; e < m * n; e += NT) {
-    const int r = e / n, c = e % n;
-    C[(size_t)r * ldc + c] = ldcg(&A[(size_t)r * lda + c]);
+// C[m x n] (m <= 16, n <= 32) = beta C + alpha A^T B in free order, A: k x m, B: k x n as stored (the
+// solves' x^T V): every warp sums a slice of the rows, read straight into tensor-core fragments, and
+// the slices are added in order.
+__device__ __forceinline__ void dev_tn(double* C, int ldc, const double* A, int lda, const double* B, int ldb, int m, int n,
+                                       int k, double alpha, double beta) {
+  extern __shared__ __align__(16) double vm_smem[];
+  const int tid = thread_index(), warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3;
+  const int per = (((k + 7) >> 3) + 3) & ~3, l0 = min(k, warp * per), len = min(per, k - l0);
+#pragma unroll 1
+  for (int mi = 0; 8 * mi < m; ++mi) {
+    double acc[4][2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = 0.0;
+    const LrMat X{A + (size_t)l0 * lda, lda, 1, m}, W{B + (size_t)l0 * ldb, ldb, 1, n};
+    if (n > 16) lr_tn_tiles<4>(acc, X, W, mi, 0, len, fa, fb);
+    else lr_tn_tiles<2>(acc, X, W, mi, 0, len, fa, fb);
+    double* red = vm_smem + (mi * 8 + warp) * 256 + fa * 32 + 2 * fb;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      red[8 * j] = acc[j][0];
+      red[8 * j + 1] = acc[j][1];
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < m * n; e += NT) {
+    const int r = e / n, c = e - r * n;
+    const double* red = vm_smem + (r >> 3) * 2048 + (r & 7) * 32 + c;
+    double v = red[0];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) v += red[w * 256];
+    double* p = C + (size_t)r * ldc + c;
+    *p = beta != 0.0 ? fma(alpha, v, ldcg(p)) : alpha * v;
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ void run_composite(const pp_task& T) {
+  const bool product = T.op == PP_OP_GEMM || T.op == PP_OP_GEMM3 || T.op == PP_OP_GEMM4;
+  const bool free_order = T.op == PP_OP_GEMM && (T.flags & PP_FREE_ORDER), tA = T.flags & PP_T(1), tB = T.flags & PP_T(2);
+  // products of the solves, in free order: a leaf, its inverse or a low-rank factor times a few
+  // right-hand sides (columns that stage in shared memory), and a few right-hand sides' transposes
+  // times a low-rank factor (short k stays with the general product: 8 warps of 8 rows are not fewer
+  // steps than its one chunk)
+  if (T.op == PP_OP_TRMV || (free_order && !tA && !tB && T.n <= 16 && T.k <= 1024)) {
+    const bool trmv = T.op == PP_OP_TRMV, part = trmv && T.l > 0;
+    const int r0 = part ? T.o : 0;
+    const double* S = trmv ? (part ? T.p[2] : T.p[0]) : T.p[2];
+    const int lds = trmv ? (part ? T.ld[2] : T.ld[0]) : T.ld[2];
+    dev_rows(T.p[0], T.ld[0], T.p[1] + (size_t)r0 * T.ld[1], T.ld[1], S, lds, trmv ? T.m : T.k, T.n, part ? T.l : T.m,
+             !trmv ? 2 : T.ctrl == 1 ? 1 : T.ctrl == 0 ? 0 : 2, r0, trmv ? 1.0 : T.alpha, trmv ? 0.0 : T.beta);
+    return;
+  }
+  if (free_order && tA && !tB && T.m <= 16 && T.n <= 32 && T.k >= 64) {
+    dev_tn(T.p[0], T.ld[0], T.p[1], T.ld[1], T.p[2], T.ld[2], T.m, T.n, T.k, T.alpha, T.beta);
+    return;
+  }
+  int op = T.op, size = T.op == PP_OP_TRSMR ? T.n : T.m, lines = T.op == PP_OP_TRSMR ? T.m : T.n;
+  double* B = T.p[0];
+  const double* A = T.p[1];
+  const int ldb = T.ld[0], lda = T.ld[1];
+  if (T.op == PP_OP_TRINV) {
+    // columns [o, o + n) of L^-1 (ctrl 0) or U^-1 (1): identity columns, then the solve on the
+    // sub-triangle they need (rows o.. of L^-1 are the only nonzeros; rows ..o + n of U^-1)
+    const int w = T.n, c0 = T.o;
+    for (int e = threadIdx.x; e < T.m * w; e += NT) {
+      const int r = e / w, j = e % w;
+      B[(size_t)r * ldb + j] = r == c0 + j ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    op = T.ctrl ? PP_OP_TRSMU : PP_OP_TRSML;
+    size = T.ctrl ? c0 + w : T.m - c0;
+    lines = w;
+    if (!T.ctrl) {
+      B += (size_t)c0 * ldb;
+      A += (size_t)c0 * lda + c0;
+    }
+  }
+#pragma unroll 1
+  for (int step = 0;; ++step) {
+    Product P;
+    if (product) {
+      if (!chain_step(T, step, P)) break;
+    } else {
+      int d = 0, len = 0;
+      if (!tri_step(op, B, ldb, A, lda, size, lines, step, d, len, P)) break;
+      if (!(step & 1)) {
+        double* Bd = B + (op == PP_OP_TRSMR ? (size_t)d : (size_t)d * ldb);
+        dev_tri(op, Bd, ldb, A + (size_t)d * lda + d, lda, len, lines, (T.flags & PP_PIVOT) ? T.p[2] : nullptr);
+        continue;
+      }
+    }
+    dev_gemm(P.C, P.ldc, P.A, P.lda, P.tA, P.B, P.ldb, P.tB, P.m, P.n, P.k, P.alpha, P.beta, free_order);
+  }
+}
+
+// C[m x n] := A[m x n], eight loads in flight per thread
+__device__ __forceinline__ void dev_copy(double* C, int ldc, const double* A, int lda, int m, int n) {
+  const int tid = thread_index();
+#pragma unroll 1
+  for (int e0 = tid; e0 < m * n; e0 += 8 * NT) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int e = e0 + u * NT, r = e / n;
+      v[u] = ldcg_if(A + (size_t)r * lda + (e - r * n), e < m * n);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int e = e0 + u * NT, r = e / n;
+      st_if(C + (size_t)r * ldc + (e - r * n), v[u], e < m * n);
+    }
   }
   __syncthreads();
 }
@@ -2189,7 +2267,9 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
     case PP_OP_TRINV:
       if (T.m > PP_VM_INV || T.n < 1 || T.o < 0 || T.o + T.n > T.m) return false;
       break;
-    case PP_OP_TRMV: return dev_trmv(T, smem);
+    case PP_OP_TRMV:
+      if (!trmv_ok(T)) return false;
+      break;
     case PP_OP_ORTH:
       if (T.n < 1 || T.n > PP_VM_MAX_RANK || T.ld[0] != T.n) return false;
       break;

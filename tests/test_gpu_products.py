@@ -39,3 +39,14 @@ def test_product_free_order(pp, oracle, gctx, m, n, k, tA, tB, pad):
     """Two sums of the same k products differ by at most 2 k u times the sum of their magnitudes."""
     d, h, size = product(pp, oracle, gctx, m, n, k, tA, tB, 1, 1.0, 1.0, pad)
     assert np.abs(d - h).max() <= 2 * k * 2.0 ** -53 * size
+
+
+@pytest.mark.parametrize("pad", [0, 1])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (7, 8, 9), (8, 1, 64), (65, 9, 65), (200, 16, 130), (256, 4, 32), (64, 8, 512),
+                                   (40, 3, 1024), (40, 3, 1025)])
+def test_rows_times_few_columns(pp, oracle, gctx, m, n, k, pad):
+    """Free-order products with at most 16 columns (rows straight from global memory, the columns staged;
+    above k = 1024 the general product): within the rounding of two summation orders."""
+    for alpha, beta in ((-1.0, 1.0), (1.0, 0.0)):
+        d, h, size = product(pp, oracle, gctx, m, n, k, 0, 0, 1, alpha, beta, pad)
+        assert np.abs(d - h).max() <= 2 * k * 2.0 ** -53 * size
