@@ -50,9 +50,9 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
 __device__ __forceinline__ void st_release(int* p, int v) {
   asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ int atom_add_acq_rel(int* p, int v) {
+__device__ __forceinline__ int atom_add_relaxed(int* p, int v) {
   int old;
-  asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  asm volatile("atom.relaxed.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
   return old;
 }
 __device__ __forceinline__ int ld_relaxed(const int* p) {
@@ -1379,8 +1379,8 @@ __device__ __forceinline__ void dev_tri(int op, double* B, int ldb, const double
 // The explicit inverses of the leaves (TRMV) and the solves' products with a leaf or a low-rank
 // factor: S is staged in shared memory, a warp takes eight rows of M at a time straight from global
 // memory into FP64 tensor-core fragments, two columns per load (the k order is free: even columns in
-// one chain, odd ones in another), sixteen loads in flight per lane; nothing of a row depends on
-// which other rows the call covers.  Bound by one CTA's loads.  On a B200, hop of 2.5 us included
+// one chain, odd ones in another), the next 64 columns loading during the products; nothing of a row
+// depends on which other rows the call covers.  Bound by one CTA's loads.  On a B200, hop of 2.5 us included
 // (before: warps along the columns, a shuffle reduction per row and right-hand side):
 //   TRMV 128 x 4, 64 rows  13 -> 6 us    94 x 1  13.5 -> 6 us    512 x 8, 64 rows  31 -> 12 us
 //   products 64 x 8 x 512  15 -> 12 us   61 x 4 x 64  5.5 -> 4 us  (the latter from the general routine)
@@ -2326,9 +2326,11 @@ __global__ void __launch_bounds__(NT, 1)
     vm_kernel(const pp_task* __restrict__ tasks, int n_tasks, const int32_t* __restrict__ succ, int32_t* counters,
               int32_t* slots, pp_vm_state* st, long long wait_ns, unsigned long long* trace, int use_tc) {
   extern __shared__ __align__(16) double smem[];
-  __shared__ __align__(16) pp_task s_task;
+  __shared__ __align__(16) pp_task s_rec[2][4];  // this task's record, and those of its first successors
+  __shared__ int s_succ[32];                     // its first successors
+  __shared__ int s_pub[32], s_npub;              // successors ready but not run here
   __shared__ int s_id;
-  __shared__ int s_keep;  // position (in the successor list) of the successor run next
+  __shared__ int s_keep;  // position (in the successor list) of the successor run next, or -1
   __shared__ unsigned long long s_t0;
   __shared__ uint32_t s_tmem;
   __shared__ __align__(8) unsigned long long s_mbar;
@@ -2365,11 +2367,22 @@ __global__ void __launch_bounds__(NT, 1)
   // same CTA without a round trip through the queue; the others are pushed.  Queue slots
   // therefore number fewer than tasks, so a CTA waiting on a slot also leaves once every
   // task is done.
-  int next = -1;
+  //
+  // What a hop from a task to its successor costs is latency: a device-wide fence about 400 cycles
+  // behind stores, an atomic 690 (1570 with acquire and release folded in, which fences twice), a
+  // load 300 to 600.  So the successor list comes in while the task runs; after the task one CTA
+  // barrier collects its stores, warp 0 fences once, decrements the counters with relaxed atomics
+  // and fences again, while warps 1 to 4 fetch the records of the first four successors; and the
+  // ready successors that are not run here are pushed by the last warp beside the next task's loads.
+  // Between tasks of the critical path of the dense N = 1024 factor: 2.0 us before, 1.2 us so.
+  int next = -1, par = 0, slot = 0;
+  bool next_unfetched = false;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) s_npub = 0;
   for (;;) {
-    if (threadIdx.x == 0) {
-      int id = next;
-      if (id < 0) {
+    int id = next;
+    if (id < 0) {
+      if (threadIdx.x == 0) {
         const int idx = atomicAdd(&st->head, 1);
         if (idx < n_tasks) {
           const unsigned long long t_wait = gtimer_ns();
@@ -2387,53 +2400,82 @@ __global__ void __launch_bounds__(NT, 1)
             __nanosleep(32);
           }
         }
+        s_id = id;
       }
-      s_id = id;
-      if (trace) s_t0 = globaltimer_ns();
+      __syncthreads();
+      id = s_id;
+      if (id < 0) break;
+      slot = 0;
     }
-    __syncthreads();
-    const int id = s_id;
-    if (id < 0) break;
-    if (threadIdx.x < (int)(sizeof(pp_task) / 8))
-      reinterpret_cast<unsigned long long*>(&s_task)[threadIdx.x] =
-          __ldg(reinterpret_cast<const unsigned long long*>(&tasks[id]) + threadIdx.x);
-    if (threadIdx.x == 0) s_keep = NT;
-    __syncthreads();
+    pp_task& T = s_rec[par][slot];
+    if (next < 0 || next_unfetched) {
+      if (threadIdx.x < (int)(sizeof(pp_task) / 8))
+        reinterpret_cast<unsigned long long*>(&T)[threadIdx.x] =
+            __ldg(reinterpret_cast<const unsigned long long*>(&tasks[id]) + threadIdx.x);
+      __syncthreads();
+    }
+    if (trace && threadIdx.x == 0) s_t0 = globaltimer_ns();
+    const int nsucc = T.n_succ, sbeg = T.succ_begin;
+    if (warp == 7) {
+      // push what the previous task left ready, and fetch this task's successor list
+      const int count = s_npub;
+      if (count > 0) {
+        int base = 0;
+        if (lane == 0) base = atomicAdd(&st->tail, count);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (lane < count) st_release(&slots[base + lane], s_pub[lane]);
+      }
+      if (lane < nsucc)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&s_succ[lane])), "l"(&succ[sbeg + lane])
+                     : "memory");
+      cp_async_commit();
+    }
     int err = PP_VM_OK;
-    const bool ok = run_task(s_task, smem, tc, err);
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      if (!ok && atomicCAS(&st->error, 0, PP_VM_BAD_TASK) == 0) st->err_info = id;
-      if (err != PP_VM_OK && atomicCAS(&st->error, 0, err) == 0) st->err_info = id;
-      if (trace) {
-        trace[3 * (size_t)id] = s_t0;
-        trace[3 * (size_t)id + 1] = globaltimer_ns();
-        trace[3 * (size_t)id + 2] = smid() | ((unsigned long long)blockIdx.x << 32);
+    const bool ok = run_task(T, smem, tc, err);
+    if (warp == 7) cp_async_wait<0>();
+    __syncthreads();  // the task's stores, and the successor list
+    if (warp == 0) {
+      __threadfence();
+      if (lane == 0) {
+        if (!ok && atomicCAS(&st->error, 0, PP_VM_BAD_TASK) == 0) st->err_info = id;
+        if (err != PP_VM_OK && atomicCAS(&st->error, 0, err) == 0) st->err_info = id;
+        if (trace) {
+          trace[3 * (size_t)id] = s_t0;
+          trace[3 * (size_t)id + 1] = globaltimer_ns();
+          trace[3 * (size_t)id + 2] = smid() | ((unsigned long long)blockIdx.x << 32);
+        }
       }
-    }
-    // successors are released in parallel, one thread each (a serial loop costs one L2
-    // round trip per successor on the critical path)
-    const int nsucc = s_task.n_succ, sbeg = s_task.succ_begin;
-    int mine = -1;
-    for (int q = threadIdx.x; q < nsucc; q += NT) {
-      const int sq = succ[sbeg + q];
-      if (atom_add_acq_rel(&counters[sq], -1) == 1) {
-        if (q < NT) {
-          mine = sq;
-          atomicMin(&s_keep, q);
-        } else {
+      const int mine = lane < nsucc ? s_succ[lane] : -1;
+      const bool ready = mine >= 0 && atom_add_relaxed(&counters[mine], -1) == 1;
+      for (int q = lane + 32; q < nsucc; q += 32) {
+        const int sq = succ[sbeg + q];
+        if (atom_add_relaxed(&counters[sq], -1) == 1) {
+          __threadfence();
           st_release(&slots[atomicAdd(&st->tail, 1)], sq);
         }
       }
+      __threadfence();  // the other predecessors' stores are visible from here on
+      const unsigned all = __ballot_sync(0xffffffffu, ready);
+      const int keep = __ffs((int)all) - 1;
+      const unsigned rest = all & (all - 1);
+      if (ready && lane != keep) s_pub[__popc(rest & ((1u << lane) - 1))] = mine;
+      if (lane == 0) {
+        s_npub = __popc(rest);
+        s_keep = keep;
+        atomicAdd(&st->done, 1);
+      }
+    } else if (warp <= 4 && warp - 1 < nsucc) {
+      const pp_task* rec = &tasks[s_succ[warp - 1]];
+      if (lane < (int)(sizeof(pp_task) / 8))
+        reinterpret_cast<unsigned long long*>(&s_rec[par ^ 1][warp - 1])[lane] =
+            __ldg(reinterpret_cast<const unsigned long long*>(rec) + lane);
     }
     __syncthreads();
+    par ^= 1;
     const int keep = s_keep;
-    if (mine >= 0 && (int)threadIdx.x != keep) st_release(&slots[atomicAdd(&st->tail, 1)], mine);
-    if (threadIdx.x == 0) {
-      next = keep < NT ? succ[sbeg + keep] : -1;
-      atomicAdd(&st->done, 1);
-    }
+    next = keep >= 0 ? s_succ[keep] : -1;
+    next_unfetched = keep >= 4;
+    slot = keep >= 0 && keep < 4 ? keep : 0;
   }
   if (use_tc) {
     // an MMA group whose completion was never observed still owns the accumulators:
