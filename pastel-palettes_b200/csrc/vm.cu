@@ -146,7 +146,7 @@ __device__ __forceinline__ void copy_rows4(uint32_t& dst, const char*& src, int&
 // evicted by the tasks before it, so much of what a small product costs is fetching its code
 // (forms specialised by tile shape, ten times the code, ran small shapes at half the speed inside
 // the VM and faster outside of it).  The output is walked in CTA tiles of TM x TN (128 x 16,
-// 64 x 32, 128 x 32, 16 x 64, 64 x 64: the narrowest that covers it) of 16 x 16 warp tiles, one or
+// 64 x 32, 128 x 32, 16 x 128, 64 x 64: the narrowest that covers it) of 16 x 16 warp tiles, one or
 // two side by side per warp, k in chunks of GM_KC through a ring of GM_ST shared-memory stages over
 // (tile, chunk) pairs, so that the loads of the next chunks are in flight during the products.
 // Operands are staged as A[m][k] and B[k][n] whatever their storage, so that a fragment's address
@@ -163,7 +163,7 @@ __device__ __forceinline__ void copy_rows4(uint32_t& dst, const char*& src, int&
 #define GM_KC 64
 #define GM_LD (GM_KC + 4)
 #define GM_ST 2
-#define GM_STAGE (VM_SMEM_BYTES / 8 / GM_ST)  /* doubles: A 128 x 68 and B 64 x 36, or 64 x 68 and 64 x 68 */
+#define GM_STAGE (VM_SMEM_BYTES / 8 / GM_ST)  /* doubles: A 128 x 68 and B 64 x 36, 64 x 68 and 64 x 68, 16 x 68 and 64 x 132 */
 
 // v with its sign bit flipped where `mask` has it set (the factor alpha = -1, exactly: a
 // multiplication would take as long on the FP64 pipe as a product of fragments)
@@ -209,7 +209,7 @@ __device__ __forceinline__ void dev_gemm(double* __restrict__ C, int ldc, const 
   if (n <= 16) { lm = 7; ln = 4; r1 = 16 * warp; c1 = 0; }
   else if (n <= 32 && m <= 64) { lm = 6; ln = 5; r1 = 16 * (warp & 3); c1 = 16 * (warp >> 2); }
   else if (n <= 32) { lm = 7; ln = 5; r1 = 16 * warp; c1 = 0; wide_n = 1; }
-  else if (m <= 16) { lm = 4; ln = 6; r1 = 0; c1 = 16 * warp; }
+  else if (m <= 16) { lm = 4; ln = 7; r1 = 0; c1 = 16 * warp; }
   else { lm = 6; ln = 6; r1 = 16 * (warp & 3); c1 = 32 * (warp >> 2); wide_n = 1; }
   if (free_order && m <= 32 && n <= 32 && k >= 64) {
     const int wt = (m > 16 ? 1 : 0) + (n > 16 ? 1 : 0);  // 2^wt warp tiles

@@ -1,4 +1,4 @@
-"""The VM's product routine at the edges of its tile shapes (128 x 16, 64 x 32, 128 x 32, 16 x 64,
+"""The VM's product routine at the edges of its tile shapes (128 x 16, 64 x 32, 128 x 32, 16 x 128,
 64 x 64), of its k chunks (64) and passes (8), aligned and odd strides: bitwise equal to the oracle's
 ascending chain; free-order products of small outputs (k split over 2, 4 or 8 warps) within the
 rounding of two summation orders."""
@@ -50,3 +50,12 @@ def test_rows_times_few_columns(pp, oracle, gctx, m, n, k, pad):
     for alpha, beta in ((-1.0, 1.0), (1.0, 0.0)):
         d, h, size = product(pp, oracle, gctx, m, n, k, 0, 0, 1, alpha, beta, pad)
         assert np.abs(d - h).max() <= 2 * k * 2.0 ** -53 * size
+
+
+@pytest.mark.parametrize("pad", [0, 1])
+@pytest.mark.parametrize("tA,tB", [(0, 0), (0, 1)])
+@pytest.mark.parametrize("m,n,k", [(16, 128, 64), (16, 129, 64), (9, 300, 72), (1, 1000, 200)])
+def test_flat_product_bitwise(pp, oracle, gctx, m, n, k, tA, tB, pad):
+    """Outputs of at most 16 rows over several tiles: every warp stays inside its own tile."""
+    d, h, _ = product(pp, oracle, gctx, m, n, k, tA, tB, 0, 1.0, 1.0, pad)
+    assert np.array_equal(d, h)
