@@ -2628,72 +2628,8 @@ __device__ __noinline__ void dev_kmul(const pp_task& T, double* smem) {
   }
 }
 
-#define KR_THREADS 128
-#define KR_RPT 2                      /* rows per thread */
-#define KR_ROWS (KR_THREADS * KR_RPT)  /* rows per CTA */
-#define KR_COLS 256
-#define KR_SEG 128   /* columns per partial sum (small: enough CTAs to fill the SMs) */
-// matrix-free partial products of r = b - A x, A_ij = K(|p_i - p_j|) (+ shift on i == j):
-// CTA (row block, column segment) sums its KR_SEG columns (points and x staged through smem
-// in KR_COLS tiles; each thread carries KR_RPT rows, so every staged column feeds
-// independent chains) into part[seg][i]; residual_reduce adds the segments in order.  The
-// kernel, the dimension and the right-hand-side count are compile-time parameters.
-template <int KIND, int DIM, int NR>
-__global__ void __launch_bounds__(KR_THREADS) kernel_residual_part(double p0, double shift,
-                                                                   const double* __restrict__ pts, int n,
-                                                                   const double* __restrict__ x,
-                                                                   double* __restrict__ part, int nrhs) {
-  __shared__ double sp[KR_COLS * DIM];
-  __shared__ double sx[KR_COLS * NR];
-  const int seg = blockIdx.y, jb = seg * KR_SEG, je = min(n, jb + KR_SEG);
-  const double inv_p0 = 1.0 / p0;
-  int row[KR_RPT];
-  double pi[KR_RPT][DIM];
-  double acc[KR_RPT][NR];
-#pragma unroll
-  for (int t = 0; t < KR_RPT; ++t) {
-    row[t] = blockIdx.x * KR_ROWS + t * KR_THREADS + threadIdx.x;
-    const int i = min(row[t], n - 1);
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) pi[t][d] = pts[(size_t)i * DIM + d];
-#pragma unroll
-    for (int q = 0; q < NR; ++q) acc[t][q] = 0.0;
-  }
-  for (int j0 = jb; j0 < je; j0 += KR_COLS) {
-    const int nj = min(KR_COLS, je - j0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < nj * DIM; e += KR_THREADS) sp[e] = pts[(size_t)j0 * DIM + e];
-    for (int e = threadIdx.x; e < nj * NR; e += KR_THREADS) {
-      const int jj = e / NR, q = e % NR;
-      sx[e] = q < nrhs ? x[(size_t)(j0 + jj) * nrhs + q] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll 2
-    for (int j = 0; j < nj; ++j) {
-      double pj[DIM];
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) pj[d] = sp[j * DIM + d];
-#pragma unroll
-      for (int t = 0; t < KR_RPT; ++t) {
-        double d2 = 0.0;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-          const double u = pi[t][d] - pj[d];
-          d2 = fma(u, u, d2);
-        }
-        double a = kernel_eval_nr<KIND>(d2, p0, inv_p0);
-        if (j0 + j == row[t]) a += shift;
-#pragma unroll
-        for (int q = 0; q < NR; ++q) acc[t][q] = fma(a, sx[j * NR + q], acc[t][q]);
-      }
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < KR_RPT; ++t)
-    if (row[t] < n)
-      for (int q = 0; q < nrhs; ++q) part[((size_t)seg * n + row[t]) * nrhs + q] = acc[t][q];
-}
-
+#define KR_SEG 128   /* columns per partial sum of the one-column products */
+#define KW_SEG 256   /* and of the wider ones (kernel_residual_wide) */
 // Jobs of one batched residual launch, passed by value (kernel parameter space): job j owns
 // the launch's work items [first, next job's first) — tile pairs of the residual kernel,
 // elements of the update and reduction kernels.
@@ -2891,6 +2827,150 @@ __global__ void __launch_bounds__(KR_SEG) kernel_residual_sym(const __grid_const
   }
 }
 
+// The symmetric form for two and more right-hand sides, eight at a time (blockIdx.y: the group of
+// eight): a CTA takes the tile pair (I, J), I <= J, of KW_SEG x KW_SEG tiles and evaluates each entry
+// once; both products run on the FP64 tensor cores.  In an 8 x 8 block lane (a, b) = (l / 4, l % 4)
+// evaluates entries (a, b) and (a, b + 4): as they are, they are the A fragments of E X_J, whose sums
+// stay in the warp's registers; turned by four shuffles they are those of E^T X_I.  A warp owns 32
+// rows, whose points, right-hand sides and sums it keeps in registers, and walks the columns in
+// blocks of 32; in each of 8 phases the warps are on different blocks, so that the column sums are
+// added in shared memory by one warp at a time and in a fixed order.  Every (segment, row) partial is
+// written once, by one CTA: deterministic, no atomics.
+// Bound by the FP64 pipe: 15 operations per entry and, with eight columns, 4 tensor instructions per
+// 64 entries, as much again.  On a B200, 3-D Laplace: N = 65536,
+// 8 columns 9.7 -> 5.8 ms (before: a row-block form that evaluated every entry twice), 3 columns 20.8 ->
+// 5.6 ms (before: column sums of every entry read and written in shared memory).
+#define KW_LDX 10  /* doubles between the rows of a staged right-hand side block: 2 mod 8 */
+template <int KIND>
+__device__ __forceinline__ double kernel_eval_wide(double d2, double p0, double cp0, double inv_p0) {
+  // d2 comes with 1e-300 added (nothing to a distance above 1e-140), which keeps the estimate finite;
+  // an overflowed one is brought down to 2^1023 by an integer select (the FP64 pipe is the full one)
+  const int hi = __double2hiint(d2);
+  d2 = __hiloint2double(hi == 0x7ff00000 ? 0x7fe00000 : hi, __double2loint(d2));
+  const double y0 = rsqrt_est(d2), s0 = d2 * y0, e = fma(-s0, y0, 1.0);
+  const double d = fma(s0 * e, fma(0.375, e, 0.5), s0);
+  if (KIND <= 1) {
+    constexpr double c = KIND == 1 ? 4.0 * 3.14159265358979323846 : 1.0;
+    const double x = fma(c, d, cp0);
+    return rcp_refine(x, rcp_est(x));
+  }
+  if (KIND == 2) return exp(-d * inv_p0);
+  const double s = 1.7320508075688772 * d * inv_p0;
+  return (1.0 + s) * exp(-s);
+}
+template <int KIND, int DIM>
+__global__ void __launch_bounds__(KW_SEG) kernel_residual_wide(const __grid_constant__ ResidLaunch L) {
+  extern __shared__ __align__(16) double kw_smem[];
+  double* xj = kw_smem;                    // KW_SEG x KW_LDX: right-hand sides of the columns
+  double* col = xj + KW_SEG * KW_LDX;      // KW_SEG x KW_LDX: column sums
+  double* pj = col + KW_SEG * KW_LDX;      // KW_SEG x DIM: points of the columns
+  const ResidLaunch::Job& jb = L.job[resid_job_of(L, (long long)blockIdx.x)];
+  const double* __restrict__ pts = jb.pts;
+  const double* __restrict__ x = jb.x;
+  double* __restrict__ part = jb.part;
+  const int n = jb.n, nrhs = jb.nrhs, T = jb.T, q0 = 8 * blockIdx.y;
+  if (q0 >= nrhs) return;
+  const double p0 = jb.p0, cp0 = (KIND == 1 ? 4.0 * 3.14159265358979323846 : 1.0) * p0, inv_p0 = 1.0 / p0;
+  // (I, J) of the job's pair index over the upper triangle, row by row (as kernel_residual_sym)
+  const long long b = (long long)blockIdx.x - jb.first;
+  const double tt = 2.0 * T + 1.0;
+  int I = (int)floor((tt - sqrt(tt * tt - 8.0 * (double)b)) * 0.5);
+  auto row_start = [&](int r) { return (long long)r * T - (long long)r * (r - 1) / 2; };
+  while (I > 0 && row_start(I) > b) --I;
+  while (row_start(I + 1) <= b) ++I;
+  const int J = I + (int)(b - row_start(I));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3;
+  const int i0 = I * KW_SEG + 32 * warp, j0 = J * KW_SEG;
+  for (int e = tid; e < KW_SEG * DIM; e += KW_SEG) pj[e] = j0 + e / DIM < n ? pts[(size_t)j0 * DIM + e] : 0.0;
+  for (int e = tid; e < KW_SEG * 8; e += KW_SEG) {
+    const int r = e >> 3, q = e & 7;
+    xj[r * KW_LDX + q] = (j0 + r < n && q0 + q < nrhs) ? x[(size_t)(j0 + r) * nrhs + q0 + q] : 0.0;
+    col[r * KW_LDX + q] = 0.0;
+  }
+  double pi[4][DIM], xi[4][2], acc[4][2];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const int i = min(i0 + 8 * t + fa, n - 1);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) pi[t][d] = pts[(size_t)i * DIM + d];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = i0 + 8 * t + 4 * h + fb;
+      xi[t][h] = (r < n && q0 + fa < nrhs) ? x[(size_t)r * nrhs + q0 + fa] : 0.0;
+      acc[t][h] = 0.0;
+    }
+  }
+  const bool offdiag = I != J;
+#pragma unroll 1
+  for (int ph = 0; ph < 8; ++ph) {
+    __syncthreads();
+    const int cb = 32 * ((warp + ph) & 7);
+#pragma unroll 1
+    for (int c0 = cb; c0 < cb + 32; c0 += 8) {
+      if (j0 + c0 >= n) break;
+      double p[2][DIM];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) p[h][d] = pj[(c0 + 4 * h + fb) * DIM + d];
+      const double x0 = xj[(c0 + fb) * KW_LDX + fa], x1 = xj[(c0 + 4 + fb) * KW_LDX + fa];
+      double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        double e[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          double d2 = 1e-300;
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) {
+            const double u = pi[t][d] - p[h][d];
+            d2 = fma(u, u, d2);
+          }
+          e[h] = kernel_eval_wide<KIND>(d2, p0, cp0, inv_p0);
+        }
+        dmma(acc[t][0], acc[t][1], e[0], x0);
+        dmma(acc[t][0], acc[t][1], e[1], x1);
+        if (offdiag) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            // entry (4 h + fb, fa) of the block: lane (4 h + fb, fa % 4), its first or second entry
+            const int src = (4 * h + fb) * 4 + (fa & 3);
+            const double v0 = __shfl_sync(0xffffffffu, e[0], src), v1 = __shfl_sync(0xffffffffu, e[1], src);
+            dmma(s0, s1, fa < 4 ? v0 : v1, xi[t][h]);
+          }
+        }
+      }
+      if (offdiag) {
+        double* c = col + (c0 + fa) * KW_LDX + 2 * fb;
+        c[0] += s0;
+        c[1] += s1;
+      }
+    }
+  }
+  // the diagonal entries' shift, and the row sums
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const int i = i0 + 8 * t + fa;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int q = q0 + 2 * fb + h;
+      if (i < n && q < nrhs) {
+        const double v = offdiag ? acc[t][h] : fma(jb.shift, x[(size_t)i * nrhs + q], acc[t][h]);
+        part[((size_t)J * n + i) * nrhs + q] = v;
+      }
+    }
+  }
+  if (offdiag) {
+    __syncthreads();
+    for (int e = tid; e < KW_SEG * 8; e += KW_SEG) {
+      const int r = e >> 3, q = e & 7;
+      if (j0 + r < n && q0 + q < nrhs) part[((size_t)I * n + j0 + r) * nrhs + q0 + q] = col[r * KW_LDX + q];
+    }
+  }
+}
+template <int DIM>
+constexpr size_t kw_smem_bytes() { return sizeof(double) * (2 * KW_SEG * KW_LDX + KW_SEG * DIM); }
+
 // r = b - (sum of the job's segments in order), one thread per (row, rhs) element
 __global__ void residual_reduce(const __grid_constant__ ResidLaunch L) {
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2913,14 +2993,9 @@ __global__ void residual_update(const __grid_constant__ ResidLaunch L) {
 
 template <int KIND, int DIM>
 cudaError_t launch_residual_sym(const ResidLaunch& L, unsigned pairs, int nr, bool lowp, cudaStream_t s) {
-  if (lowp) {
-    if (nr == 1) kernel_residual_sym<KIND, DIM, 1, true><<<pairs, KR_SEG, 0, s>>>(L);
-    else kernel_residual_sym<KIND, DIM, 4, true><<<pairs, KR_SEG, 0, s>>>(L);
-  } else if (nr == 1) {
-    kernel_residual_sym<KIND, DIM, 1, false><<<pairs, KR_SEG, 0, s>>>(L);
-  } else {
-    kernel_residual_sym<KIND, DIM, 4, false><<<pairs, KR_SEG, 0, s>>>(L);
-  }
+  if (!lowp) kernel_residual_sym<KIND, DIM, 1, false><<<pairs, KR_SEG, 0, s>>>(L);
+  else if (nr == 1) kernel_residual_sym<KIND, DIM, 1, true><<<pairs, KR_SEG, 0, s>>>(L);
+  else kernel_residual_sym<KIND, DIM, 4, true><<<pairs, KR_SEG, 0, s>>>(L);
   return cudaGetLastError();
 }
 
@@ -2933,24 +3008,22 @@ cudaError_t launch_residual_sym_dim(int dim, const ResidLaunch& L, unsigned pair
 }
 
 template <int KIND, int DIM>
-cudaError_t launch_residual_part(const pp_resid_job& j, cudaStream_t s) {
-  const int segs = (j.n + KR_SEG - 1) / KR_SEG;
-  const dim3 grid((j.n + KR_ROWS - 1) / KR_ROWS, segs);
-  if (j.nrhs <= 8)
-    kernel_residual_part<KIND, DIM, 8><<<grid, KR_THREADS, 0, s>>>(j.p0, j.shift, j.pts, j.n, j.x, j.part, j.nrhs);
-  else
-    kernel_residual_part<KIND, DIM, 16><<<grid, KR_THREADS, 0, s>>>(j.p0, j.shift, j.pts, j.n, j.x, j.part, j.nrhs);
+cudaError_t launch_residual_wide(const ResidLaunch& L, unsigned pairs, int nrhs, cudaStream_t s) {
+  kernel_residual_wide<KIND, DIM><<<dim3(pairs, (nrhs + 7) / 8), KW_SEG, kw_smem_bytes<DIM>(), s>>>(L);
   return cudaGetLastError();
 }
 
 template <int KIND>
-cudaError_t launch_residual_part_dim(const pp_resid_job& j, cudaStream_t s) {
-  if (j.dim == 1) return launch_residual_part<KIND, 1>(j, s);
-  if (j.dim == 2) return launch_residual_part<KIND, 2>(j, s);
-  return launch_residual_part<KIND, 3>(j, s);
+cudaError_t launch_residual_wide_dim(int dim, const ResidLaunch& L, unsigned pairs, int nrhs, cudaStream_t s) {
+  if (dim == 1) return launch_residual_wide<KIND, 1>(L, pairs, nrhs, s);
+  if (dim == 2) return launch_residual_wide<KIND, 2>(L, pairs, nrhs, s);
+  return launch_residual_wide<KIND, 3>(L, pairs, nrhs, s);
 }
 
-ResidLaunch::Job resid_job(const pp_resid_job& j) {
+// whether a job's product takes kernel_residual_wide: two and more right-hand sides in FP64
+bool resid_wide(const pp_resid_job& j, bool lowp) { return j.nrhs > 4 || (j.nrhs > 1 && !lowp); }
+
+ResidLaunch::Job resid_job(const pp_resid_job& j, bool lowp) {
   ResidLaunch::Job o{};
   o.pts = j.pts;
   o.x = j.x;
@@ -2962,19 +3035,19 @@ ResidLaunch::Job resid_job(const pp_resid_job& j) {
   o.shift = j.shift;
   o.n = j.n;
   o.nrhs = j.nrhs;
-  o.T = (j.n + KR_SEG - 1) / KR_SEG;
+  o.T = resid_wide(j, lowp) ? (j.n + KW_SEG - 1) / KW_SEG : (j.n + KR_SEG - 1) / KR_SEG;
   return o;
 }
 
 // element-wise launch (update or reduction) over jobs[sel] in chunks of KR_LAUNCH_JOBS
 template <typename F>
-cudaError_t launch_elementwise(const pp_resid_job* jobs, const std::vector<int>& sel, F kernel, cudaStream_t s) {
+cudaError_t launch_elementwise(const pp_resid_job* jobs, const std::vector<int>& sel, F kernel, bool lowp, cudaStream_t s) {
   for (size_t c = 0; c < sel.size(); c += KR_LAUNCH_JOBS) {
     ResidLaunch L;
     L.njobs = (int)std::min<size_t>(KR_LAUNCH_JOBS, sel.size() - c);
     long long total = 0;
     for (int q = 0; q < L.njobs; ++q) {
-      L.job[q] = resid_job(jobs[sel[c + q]]);
+      L.job[q] = resid_job(jobs[sel[c + q]], lowp);
       L.job[q].first = total;
       total += (long long)L.job[q].n * L.job[q].nrhs;
     }
@@ -3135,11 +3208,12 @@ cudaError_t preload(F f) {
 template <int KIND, int DIM>
 cudaError_t preload_residual() {
   cudaError_t e = preload(kernel_residual_sym<KIND, DIM, 1, false>);
-  if (e == cudaSuccess) e = preload(kernel_residual_sym<KIND, DIM, 4, false>);
   if (e == cudaSuccess) e = preload(kernel_residual_sym<KIND, DIM, 1, true>);
   if (e == cudaSuccess) e = preload(kernel_residual_sym<KIND, DIM, 4, true>);
-  if (e == cudaSuccess) e = preload(kernel_residual_part<KIND, DIM, 8>);
-  if (e == cudaSuccess) e = preload(kernel_residual_part<KIND, DIM, 16>);
+  if (e == cudaSuccess) e = preload(kernel_residual_wide<KIND, DIM>);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel_residual_wide<KIND, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kw_smem_bytes<DIM>());
   return e;
 }
 template <int KIND>
@@ -3196,7 +3270,7 @@ cudaError_t pp_kernel_residual_batch(const pp_resid_job* jobs, int njobs, cudaSt
     all.push_back(q);
     if (j.dx) upd.push_back(q);
   }
-  cudaError_t e = launch_elementwise(jobs, upd, residual_update, s);
+  cudaError_t e = launch_elementwise(jobs, upd, residual_update, lowp, s);
   if (e != cudaSuccess) return e;
   // tile-pair launches, one per (kernel, dimension, right-hand-side width) group
   for (int kern = 0; kern < 4; ++kern)
@@ -3211,32 +3285,39 @@ cudaError_t pp_kernel_residual_batch(const pp_resid_job* jobs, int njobs, cudaSt
           L.njobs = (int)std::min<size_t>(KR_LAUNCH_JOBS, sel.size() - c);
           long long pairs = 0;
           for (int q = 0; q < L.njobs; ++q) {
-            L.job[q] = resid_job(jobs[sel[c + q]]);
+            L.job[q] = resid_job(jobs[sel[c + q]], lowp);
             L.job[q].first = pairs;
             pairs += (long long)L.job[q].T * (L.job[q].T + 1) / 2;
           }
           if (pairs >= (1LL << 31)) return cudaErrorInvalidValue;
+          const bool wide = nr > 1 && !lowp;
           switch (kern) {
-            case 0: e = launch_residual_sym_dim<0>(dim, L, (unsigned)pairs, nr, lowp, s); break;
-            case 1: e = launch_residual_sym_dim<1>(dim, L, (unsigned)pairs, nr, lowp, s); break;
-            case 2: e = launch_residual_sym_dim<2>(dim, L, (unsigned)pairs, nr, lowp, s); break;
-            default: e = launch_residual_sym_dim<3>(dim, L, (unsigned)pairs, nr, lowp, s); break;
+            case 0: e = wide ? launch_residual_wide_dim<0>(dim, L, (unsigned)pairs, nr, s) : launch_residual_sym_dim<0>(dim, L, (unsigned)pairs, nr, lowp, s); break;
+            case 1: e = wide ? launch_residual_wide_dim<1>(dim, L, (unsigned)pairs, nr, s) : launch_residual_sym_dim<1>(dim, L, (unsigned)pairs, nr, lowp, s); break;
+            case 2: e = wide ? launch_residual_wide_dim<2>(dim, L, (unsigned)pairs, nr, s) : launch_residual_sym_dim<2>(dim, L, (unsigned)pairs, nr, lowp, s); break;
+            default: e = wide ? launch_residual_wide_dim<3>(dim, L, (unsigned)pairs, nr, s) : launch_residual_sym_dim<3>(dim, L, (unsigned)pairs, nr, lowp, s); break;
           }
           if (e != cudaSuccess) return e;
         }
       }
-  // wider right-hand-side blocks: per-job row-block partial products
+  // wider right-hand-side blocks: a launch per job
   for (int q = 0; q < njobs; ++q) {
     if (jobs[q].nrhs <= 4) continue;
+    ResidLaunch L;
+    L.njobs = 1;
+    L.job[0] = resid_job(jobs[q], lowp);
+    L.job[0].first = 0;
+    const long long pairs = (long long)L.job[0].T * (L.job[0].T + 1) / 2;
+    if (pairs >= (1LL << 31)) return cudaErrorInvalidValue;
     switch (jobs[q].kernel) {
-      case 0: e = launch_residual_part_dim<0>(jobs[q], s); break;
-      case 1: e = launch_residual_part_dim<1>(jobs[q], s); break;
-      case 2: e = launch_residual_part_dim<2>(jobs[q], s); break;
-      default: e = launch_residual_part_dim<3>(jobs[q], s); break;
+      case 0: e = launch_residual_wide_dim<0>(jobs[q].dim, L, (unsigned)pairs, jobs[q].nrhs, s); break;
+      case 1: e = launch_residual_wide_dim<1>(jobs[q].dim, L, (unsigned)pairs, jobs[q].nrhs, s); break;
+      case 2: e = launch_residual_wide_dim<2>(jobs[q].dim, L, (unsigned)pairs, jobs[q].nrhs, s); break;
+      default: e = launch_residual_wide_dim<3>(jobs[q].dim, L, (unsigned)pairs, jobs[q].nrhs, s); break;
     }
     if (e != cudaSuccess) return e;
   }
-  return launch_elementwise(jobs, all, residual_reduce, s);
+  return launch_elementwise(jobs, all, residual_reduce, lowp, s);
 }
 
 cudaError_t pp_kernel_residual(int kernel, double p0, double p1, double diag_shift, const double* pts, int dim, int n,
