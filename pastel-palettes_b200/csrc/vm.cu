@@ -541,14 +541,6 @@ __device__ __noinline__ bool dev_gemm_tc(double* __restrict__ C, int ldc, const 
 // K-major, M = 128 (bits 24-28 = M >> 4); N (bits 17-22 = N >> 3) is added per task
 constexpr uint32_t kIdescBf16Base = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 4) << 24);
 
-__device__ __forceinline__ uint32_t bf16_bits(double x) {
-  // round to nearest even through FP32 (finite values; NaN stays a quiet NaN)
-  uint32_t u = __float_as_uint(__double2float_rn(x));
-  if ((u & 0x7F800000u) == 0x7F800000u) return (u >> 16) | ((u & 0xFFFFu) ? 0x40u : 0u);
-  u += 0x7FFFu + ((u >> 16) & 1u);
-  return u >> 16;
-}
-
 // byte offset of element (r, c) of an R x K operand in the tiled layout with chunks of cr rows
 // (32, 64 or 128) and 64 columns
 __device__ __forceinline__ size_t tiled_at(int r, int c, int K, int cr) {
@@ -559,92 +551,83 @@ __device__ __forceinline__ size_t tiled_at(int r, int c, int K, int cr) {
 }
 
 // S := the tiled BF16 shadow of X (m x k, padded with zeros beyond the source's mr rows and nc
-// columns), X(r, c) = A[r lda + c] or A[c lda + r] (tA).  Each thread converts 8 consecutive
-// columns of a row and stores them as one 16-byte word, lanes along the rows (the stores of 32
-// consecutive rows fill 512 contiguous bytes).  With tA the loads are coalesced as they stand
-// (four words per thread at a time: 32 loads in flight); otherwise 128 x 64 blocks of X are
-// staged in shared memory with coalesced loads, 32 per thread in flight, the loads of the next
-// block issued before the current one is converted.  A split shadow (split = PP_SPLIT_*, k = nseg
-// segments of ks columns) writes each word once per segment: bf16(x), or the residual
-// bf16(x - bf16(x)) in the segments of the low mask.
-__device__ __forceinline__ void shadow_word(uint8_t* S, int r, int c, int k, int ks, int cr, int split,
-                                            const double* x) {
-  uint32_t h[8], l[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    h[q] = bf16_bits(x[q]);
-    l[q] = split ? bf16_bits(x[q] - (double)__uint_as_float(h[q] << 16)) : 0u;
-  }
-  uint4 vh, vl;
-  vh.x = h[0] | (h[1] << 16);
-  vh.y = h[2] | (h[3] << 16);
-  vh.z = h[4] | (h[5] << 16);
-  vh.w = h[6] | (h[7] << 16);
-  if (!split) {
-    *reinterpret_cast<uint4*>(S + tiled_at(r, c, k, cr)) = vh;
-    return;
-  }
-  vl.x = l[0] | (l[1] << 16);
-  vl.y = l[2] | (l[3] << 16);
-  vl.z = l[4] | (l[5] << 16);
-  vl.w = l[6] | (l[7] << 16);
-  const int nseg = split >> 8;
-  for (int sg = 0; sg < nseg; ++sg)
-    *reinterpret_cast<uint4*>(S + tiled_at(r, c + sg * ks, k, cr)) = ((split >> sg) & 1) ? vl : vh;
-}
+// columns), X(r, c) = A[r lda + c] or A[c lda + r] (tA).  Each thread converts 8 consecutive columns
+// of a row and stores them as one 16-byte word, lanes along the rows of a chunk (the words of 32
+// consecutive rows fill 512 contiguous bytes), four words per thread at a time: 32 values in flight.
+// With tA the loads are coalesced as they stand; otherwise a thread reads its 64 bytes as two whole
+// sectors (one by one where they are not aligned).  A split shadow (split =
+// PP_SPLIT_*, k = nseg segments of ks columns) writes each word once per segment: bf16(x), or the
+// residual bf16(x - bf16(x)) in the segments of the low mask.
+// Bound by the loads a CTA has in flight and by the conversions (15 per clock and SM).  512 x 512 on a
+// B200: 104 -> 63 us, split 172 -> 90 us (before: 128 x 64 blocks staged through shared memory, and a
+// rounding with a branch per element, which alone cost 25 us).
 
-__device__ __noinline__ void dev_shadow(uint8_t* S, const double* A, int lda, bool tA, int m, int k, int mr, int nc,
-                                       int cr, int split, double* smem) {
-  const int ks = split ? k / (split >> 8) : k;  // source columns (one segment)
-  if (tA) {
-    constexpr int W = 4;
-    const int units = m * (ks >> 3);
-    for (int u0 = threadIdx.x; u0 < units; u0 += W * NT) {
+// two doubles to BF16, to nearest even through FP32, packed (x in the low half)
+__device__ __forceinline__ uint32_t bf16_pair(double x, double y) {
+  uint32_t v;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(__double2float_rn(y)), "f"(__double2float_rn(x)));
+  return v;
+}
+__device__ __forceinline__ uint4 bf16_word(const double (&x)[8], bool low) {
+  uint32_t h[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    h[q] = bf16_pair(x[2 * q], x[2 * q + 1]);
+    if (low)
+      h[q] = bf16_pair(x[2 * q] - (double)__uint_as_float(h[q] << 16),
+                       x[2 * q + 1] - (double)__uint_as_float(h[q] & 0xFFFF0000u));
+  }
+  return make_uint4(h[0], h[1], h[2], h[3]);
+}
+__device__ __forceinline__ void dev_shadow(uint8_t* S, const double* A, int lda, bool tA, int m, int k, int mr, int nc,
+                                           int cr, int split) {
+  constexpr int W = 4;
+  const int tid = thread_index(), ks = split ? k / (split >> 8) : k;  // source columns (one segment)
+  const int lc = 31 - __clz(cr), rr = tid & (cr - 1), cstep = 8 * (NT >> lc);
+  const bool wide = !tA && nc >= 8 && ((lda & 3) == 0) && ((reinterpret_cast<uintptr_t>(A) & 31) == 0);
+#pragma unroll 1
+  for (int r0 = 0; r0 < m; r0 += cr) {
+    const int r = r0 + rr;
+#pragma unroll 1
+    for (int cb = 8 * (tid >> lc); cb < ks; cb += W * cstep) {
       double x[W][8];
 #pragma unroll
       for (int j = 0; j < W; ++j) {
-        const int u = u0 + j * NT, r = u % m, c = (u / m) << 3;
+        const int c = cb + j * cstep;
+        const bool row = r < mr && c < ks;
+        if (wide) {  // words past the source's edge are read anew below
+          const double* p = A + (size_t)(row ? r : 0) * lda + (row && c + 8 <= nc ? c : 0);
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          x[j][q] = (u < units && r < mr && c + q < nc) ? ldcg(&A[(size_t)(c + q) * lda + r]) : 0.0;
+          for (int h = 0; h < 2; ++h)
+            asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                         : "=d"(x[j][4 * h]), "=d"(x[j][4 * h + 1]), "=d"(x[j][4 * h + 2]), "=d"(x[j][4 * h + 3])
+                         : "l"(p + 4 * h)
+                         : "memory");
+        } else {
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            x[j][q] = ldcg_if(tA ? &A[(size_t)(c + q) * lda + r] : &A[(size_t)r * lda + c + q], row && c + q < nc);
+        }
       }
 #pragma unroll
       for (int j = 0; j < W; ++j) {
-        const int u = u0 + j * NT, r = u % m, c = (u / m) << 3;
-        if (u >= units) break;
-        shadow_word(S, r, c, k, ks, cr, split, x[j]);
-      }
-    }
-  } else {
-    constexpr int BR = 128, BC = 64, LD = BC + 1, PER = BR * BC / NT;
-    const int nbc = ks / BC, nb = ((m + BR - 1) / BR) * nbc;
-    double v[PER];
-    auto fetch = [&](int b) {
-      const int r0 = (b / nbc) * BR, c0 = (b % nbc) * BC;
+        const int c = cb + j * cstep;
+        if (c >= ks) break;
+        if (wide && !(r < mr && c + 8 <= nc)) {
 #pragma unroll
-      for (int p = 0; p < PER; ++p) {
-        const int e = threadIdx.x + p * NT, r = r0 + e / BC, c = c0 + e % BC;
-        v[p] = (r < m && r < mr && c < nc) ? ldcg(&A[(size_t)r * lda + c]) : 0.0;
+          for (int q = 0; q < 8; ++q) x[j][q] = ldcg_if(&A[(size_t)r * lda + c + q], r < mr && c + q < nc);
+        }
+        const uint4 high = bf16_word(x[j], false);
+        if (!split) {
+          *reinterpret_cast<uint4*>(S + tiled_at(r, c, k, cr)) = high;
+        } else {
+          const uint4 low = bf16_word(x[j], true);
+          const int nseg = split >> 8;
+#pragma unroll 1
+          for (int sg = 0; sg < nseg; ++sg)
+            *reinterpret_cast<uint4*>(S + tiled_at(r, c + sg * ks, k, cr)) = ((split >> sg) & 1) ? low : high;
+        }
       }
-    };
-    fetch(0);
-    for (int b = 0; b < nb; ++b) {
-      const int r0 = (b / nbc) * BR, c0 = (b % nbc) * BC, rows = min(BR, m - r0);
-#pragma unroll
-      for (int p = 0; p < PER; ++p) {
-        const int e = threadIdx.x + p * NT;
-        smem[(e / BC) * LD + e % BC] = v[p];
-      }
-      __syncthreads();
-      if (b + 1 < nb) fetch(b + 1);
-      for (int u = threadIdx.x; u < rows * (BC >> 3); u += NT) {
-        const int rr = u % rows, cg = (u / rows) << 3;
-        double x[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) x[q] = smem[rr * LD + cg + q];
-        shadow_word(S, r0 + rr, c0 + cg, k, ks, cr, split, x);
-      }
-      __syncthreads();
     }
   }
   // the shadow is read by bulk copies (the async proxy) of other CTAs
@@ -2290,7 +2273,7 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
       if (!(T.ctrl == 0 || T.ctrl == 32 || T.ctrl == 64 || T.ctrl == 128) || T.m % (T.ctrl ? T.ctrl : 128)) return false;
       if (T.o != 0 && (T.o >> 8 != 3 || (T.o & ~0x7FF) || T.k % (64 * 3) || T.n > T.k / 3)) return false;
       dev_shadow(reinterpret_cast<uint8_t*>(T.p[0]), T.p[1], T.ld[1], T.flags & PP_T(1), T.m, T.k,
-                 T.l > 0 ? T.l : T.m, T.n > 0 ? T.n : (T.o ? T.k / 3 : T.k), T.ctrl ? T.ctrl : 128, T.o, smem);
+                 T.l > 0 ? T.l : T.m, T.n > 0 ? T.n : (T.o ? T.k / 3 : T.k), T.ctrl ? T.ctrl : 128, T.o);
       return true;
     default: return false;
   }
