@@ -51,6 +51,8 @@ struct VmPlan {
   double dag_ms = 0;       // wall time of the DAG build alone
   int dag_on_device = 0;   // 1: built by build_dag_device
   int grid = 0;
+  bool by_class = false;  // ready tasks queued by priority class
+  pp_vm_classes classes{};
   int use_tc = 0;  // holds TF32 contractions (tensor memory per CTA)
   unsigned long long* d_trace = nullptr;  // per-task (start, end, sm | cta << 32) when tracing
   std::vector<int64_t> work_off, scratch_off, rhs_off;  // per instance (batched plans)
@@ -275,8 +277,31 @@ pp_status plan_to_device_multi(pp_context* ctx, const std::vector<pp_hmatrix*>& 
   }
   std::vector<pp_task> tasks;
   std::vector<int32_t> succ, indeg, ready;
-  plan.prog.encode(bases, tasks, succ, indeg, ready);
+  plan.prog.encode(bases, plan.prog.path_ns, tasks, succ, indeg, ready);
   plan.n_ready = (int)ready.size();
+  // Priority classes, sixteenths of the longest path still ahead of a task, where the program has
+  // enough work beside its critical path for ready tasks to queue up: from 0.3 of what the CTAs
+  // could do in that path's time.  Below that a task hardly ever waits for a CTA, and the one queue
+  // hands it over sooner (one atomic instead of three).  On a B200, one queue against classes: factor of
+  // a mixed-precision matrix with N = 32768 (0.7) 106 -> 95 ms, of 32 with 8192 unknowns (1.2) 10.8 -> 10.1
+  // ms, of 8192 unknowns in FP64 (0.5) 37.2 -> 36.1 ms, of 16 adaptive ones (0.4) 4.0 ms either way.
+  int64_t longest = 1;
+  for (int64_t b : plan.prog.path_ns) longest = std::max(longest, b);
+  plan.by_class = n < (1 << PP_VM_ID_BITS) && (double)plan.prog.work_ns >= 0.3 * (double)longest * ctx->sm_count;
+  if (plan.by_class) {
+    auto cls = [&](int32_t t) {
+      return PP_VM_CLASSES - 1 - (int)std::min<int64_t>(PP_VM_CLASSES - 1, plan.prog.path_ns[t] * PP_VM_CLASSES / longest);
+    };
+    pp_vm_classes& c = plan.classes;
+    c = pp_vm_classes{};
+    for (int32_t t = 0; t < n; ++t) ++c.base[cls(t) + 1];
+    for (int32_t t : ready) ++c.first[cls(t) + 1];  // most urgent first already
+    for (int q = 0; q < PP_VM_CLASSES; ++q) {
+      c.base[q + 1] += c.base[q];
+      c.first[q + 1] += c.first[q];
+    }
+    for (int32_t& s : succ) s |= cls(s) << PP_VM_ID_BITS;
+  }
   plan.use_tc = 0;
   for (const auto& t : tasks)
     if (t.prec == PP_PREC_TF32 || t.prec == PP_PREC_BF16) plan.use_tc = 1;
@@ -285,7 +310,7 @@ pp_status plan_to_device_multi(pp_context* ctx, const std::vector<pp_hmatrix*>& 
   PP_CUDA(alloc((void**)&plan.d_indeg, sizeof(int32_t) * n));
   PP_CUDA(alloc((void**)&plan.d_ready, sizeof(int32_t) * ready.size()));
   PP_CUDA(alloc((void**)&plan.d_counters, sizeof(int32_t) * n));
-  PP_CUDA(alloc((void**)&plan.d_slots, sizeof(int32_t) * n));
+  PP_CUDA(alloc((void**)&plan.d_slots, sizeof(int32_t) * (n + 3 * PP_VM_CLASSES)));
   PP_CUDA(alloc((void**)&plan.d_state, sizeof(pp_vm_state)));
   PP_CUDA(h2d(plan.d_tasks, tasks.data(), sizeof(pp_task) * n));
   if (!succ.empty()) PP_CUDA(h2d(plan.d_succ, succ.data(), sizeof(int32_t) * succ.size()));
@@ -317,6 +342,7 @@ pp_status launch_plan(pp_context* ctx, VmPlan& plan, cudaStream_t s, int grid_ca
   L.wait_ns = ctx->cfg.spin_limit * 1000;
   L.grid = grid_cap > 0 ? std::min(plan.grid, grid_cap) : plan.grid;
   L.trace = plan.d_trace;
+  L.classes = plan.by_class ? &plan.classes : nullptr;
   L.use_tc = plan.use_tc;
   PP_CUDA(pp_vm_run(L, s));
   return PP_OK;
@@ -878,7 +904,7 @@ pp_status pp_hmatrix_encode_program(pp_hmatrix* h, int which, int nrhs, double* 
   std::vector<double*> b(bases, bases + pp::PP_ARENAS);
   std::vector<pp_task> t;
   std::vector<int32_t> s, d, r;
-  plan->prog.encode(b, t, s, d, r);
+  plan->prog.encode(b, plan->prog.blevel, t, s, d, r);
   std::memcpy(tasks, t.data(), sizeof(pp_task) * t.size());
   if (succ && !s.empty()) std::memcpy(succ, s.data(), sizeof(int32_t) * s.size());
   std::memcpy(indeg, d.data(), sizeof(int32_t) * d.size());

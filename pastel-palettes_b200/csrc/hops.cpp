@@ -220,15 +220,55 @@ void Program::build_dag() {
   finish_dag();
 }
 
+// Estimated time of one instruction on a B200 (nanoseconds; within a third of what the instructions of
+// a factorization and a solve take).  It only orders tasks on the device: which successor a CTA goes on
+// with, and how urgent a ready task is.  By operation counts (blevel) the small serial instructions of
+// the critical path weigh nothing against the large products beside it: list-scheduling the measured
+// tasks of a mixed-precision factorization (N = 32768) by times instead ends 6% earlier.
+static int64_t task_ns(const pp_task& t) {
+  const int64_t m = t.m, n = t.n, k = t.k, l = t.l;
+  auto solve = [](int64_t d, int64_t passes) { return 2000 + passes * (90 * d + d * d / 2); };
+  switch (t.op) {
+    case PP_OP_GETRF: return 3000 + 270 * std::min(m, n);
+    case PP_OP_TRSML:
+    case PP_OP_TRSMRT:
+    case PP_OP_TRSMU: return solve(m, (n + 63) / 64);
+    case PP_OP_TRSMR: return solve(n, (m + 63) / 64) + n * n / 3;
+    case PP_OP_TRINV: return solve(t.ctrl ? t.o + n : m - t.o, (n + 63) / 64);
+    case PP_OP_GEMM:
+      if (t.prec != PP_PREC_FP64) return 10000 + m * n / 4 + m * n * (k + l) / 4096;
+      return 2500 + 10 * k + m * n / 3 + m * n * k / 81;
+    case PP_OP_GEMM3: return 5000 + (m * l * k + m * n * l) / 64;
+    case PP_OP_GEMM4: return 5000 + (m * k * l + m * l * t.o + m * n * t.o) / 64;
+    case PP_OP_ACCUM: return 5000 + 72 * k * k + (m + n) * k * std::max<int64_t>(l, k) / 4;
+    case PP_OP_LRTRUNC: return 5000 + 72 * k * k + (m + n) * k * k / 8;
+    case PP_OP_ORTH: return 3000 + m * n * n / 5;
+    case PP_OP_SUM: return 1500 + m * n * k / 8;
+    case PP_OP_COPY: return 1500 + m * n * 3 / 8;
+    case PP_OP_TRMV: return 2500 + (l > 0 ? l : m) * m * ((n + 7) / 8) / 3;
+    case PP_OP_SHADOW: return 4000 + (t.o ? m * k / 9 : m * k / 4);
+    case PP_OP_KMUL: return 3000 + m * n * (10 + k) / 1000;
+    default: return 1000;
+  }
+}
+
 void Program::finish_dag() {
   const int n = (int)tasks.size();
   deps_.clear();
   deps_built_ = false;
   blevel.assign(n, 0);
+  path_ns.assign(n, 0);
+  work_ns = 0;
   for (int t = n - 1; t >= 0; --t) {
-    int64_t b = 0;
-    for (int s : succ[t]) b = std::max(b, blevel[s]);
+    int64_t b = 0, p = 0;
+    for (int s : succ[t]) {
+      b = std::max(b, blevel[s]);
+      p = std::max(p, path_ns[s]);
+    }
     blevel[t] = b + std::max<int64_t>(tasks[t].flops, 1 << 14);
+    const int64_t ns = task_ns(tasks[t].t);
+    path_ns[t] = p + ns;
+    work_ns += ns;
   }
 }
 
@@ -252,7 +292,7 @@ h_ops_dag Program::to_dag() const {
   return d;
 }
 
-void Program::encode(const std::vector<double*>& bases, std::vector<pp_task>& out, std::vector<int32_t>& succ_out,
+void Program::encode(const std::vector<double*>& bases, const std::vector<int64_t>& level, std::vector<pp_task>& out, std::vector<int32_t>& succ_out,
                      std::vector<int32_t>& indeg_out, std::vector<int32_t>& ready_out) const {
   const int n = (int)tasks.size();
   out.resize(n);
@@ -278,7 +318,7 @@ void Program::encode(const std::vector<double*>& bases, std::vector<pp_task>& ou
       x.tmp = nullptr;
     }
     s = succ[t];
-    std::stable_sort(s.begin(), s.end(), [&](int a, int b) { return blevel[a] > blevel[b]; });
+    std::stable_sort(s.begin(), s.end(), [&](int a, int b) { return level[a] > level[b]; });
     x.succ_begin = (int32_t)succ_out.size();
     x.n_succ = (int32_t)s.size();
     succ_out.insert(succ_out.end(), s.begin(), s.end());
@@ -286,7 +326,7 @@ void Program::encode(const std::vector<double*>& bases, std::vector<pp_task>& ou
     if (pred[t].empty()) ready_out.push_back(t);
     out[t] = x;
   }
-  std::stable_sort(ready_out.begin(), ready_out.end(), [&](int a, int b) { return blevel[a] > blevel[b]; });
+  std::stable_sort(ready_out.begin(), ready_out.end(), [&](int a, int b) { return level[a] > level[b]; });
 }
 
 void Program::merge(const Program& o) {
@@ -309,14 +349,17 @@ void Program::merge(const Program& o) {
   succ.resize(tasks.size());
   pred.resize(tasks.size());
   blevel.resize(tasks.size());
+  path_ns.resize(tasks.size());
   pred_bits.resize(tasks.size());
   for (size_t t = 0; t < o.tasks.size(); ++t) {
     for (int x : o.succ[t]) succ[task0 + t].push_back(x + task0);
     for (int x : o.pred[t]) pred[task0 + t].push_back(x + task0);
     if (t < o.pred_bits.size()) pred_bits[task0 + t] = o.pred_bits[t];
     blevel[task0 + t] = o.blevel[t];
+    path_ns[task0 + t] = o.path_ns[t];
   }
   deps_built_ = false;
+  work_ns += o.work_ns;
   edges += o.edges;
 }
 

@@ -86,6 +86,8 @@ class Program {
   // the typed edges as the reference's dependency_table (rts/dependency.h), built on request
   const dependency_table& dep_table();
   std::vector<int64_t> blevel;  // FLOP-weighted longest path to an exit
+  std::vector<int64_t> path_ns; // the same in estimated nanoseconds: the order the device runs by
+  int64_t work_ns = 0;          // the tasks' estimated nanoseconds in all
   int64_t edges = 0;
  private:
   dependency_table deps_;
@@ -112,8 +114,9 @@ class Program {
   void finish_dag();
   h_ops_dag to_dag() const;
   // Pointer binding and device-table encoding.  bases[arena id] = base address.
-  void encode(const std::vector<double*>& bases, std::vector<pp_task>& out, std::vector<int32_t>& succ_out,
-              std::vector<int32_t>& indeg_out, std::vector<int32_t>& ready_out) const;
+  // successors and initially ready tasks are sorted by `level` (blevel or path_ns), descending
+  void encode(const std::vector<double*>& bases, const std::vector<int64_t>& level, std::vector<pp_task>& out,
+              std::vector<int32_t>& succ_out, std::vector<int32_t>& indeg_out, std::vector<int32_t>& ready_out) const;
   // Append all tasks of `other` (another instance's program); arenas are renumbered.
   void merge(const Program& other);
 

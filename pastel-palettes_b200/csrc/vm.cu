@@ -2282,12 +2282,31 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
   return true;
 }
 
+// Counters of the priority classes' queues, behind the slots: tasks available, taken and pushed
+#define VM_AVAIL 0
+#define VM_HEAD PP_VM_CLASSES
+#define VM_TAIL (2 * PP_VM_CLASSES)
+
 __global__ void vm_init(const int32_t* __restrict__ indeg, const int32_t* __restrict__ ready, int n_ready, int n,
-                        int32_t* counters, int32_t* slots, pp_vm_state* st) {
+                        int32_t* counters, int32_t* slots, pp_vm_state* st, int by_class,
+                        const __grid_constant__ pp_vm_classes cls) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
     counters[i] = indeg[i];
-    slots[i] = i < n_ready ? ready[i] : -1;
+    int at = i, count = n_ready;
+    if (by_class) {
+      int q = 0;
+      while (q < PP_VM_CLASSES - 1 && i >= cls.base[q + 1]) ++q;
+      at = cls.first[q] + (i - cls.base[q]);
+      count = cls.first[q + 1];
+    }
+    slots[i] = at < count ? ready[at] : -1;
+  }
+  if (by_class && i < PP_VM_CLASSES) {
+    const int first = cls.first[i + 1] - cls.first[i];
+    slots[n + VM_AVAIL + i] = first;
+    slots[n + VM_HEAD + i] = 0;
+    slots[n + VM_TAIL + i] = first;
   }
   if (i == 0) {
     st->head = 0;
@@ -2305,12 +2324,68 @@ __device__ __forceinline__ unsigned smid() {
   return s;
 }
 
+// Ready tasks by priority class (warp-wide).  A program with much work beside its critical path keeps
+// many tasks ready, and in one queue a task of that path waits for all of them: 37 of the 116 ms of a
+// mixed-precision factorization (N = 32768).  A push takes its slot with the class's tail, stores the
+// task and then counts it as available; a take first secures one of the most urgent class that shows
+// any (the count would go below zero otherwise: given back), then its slot.  A secured slot is filled,
+// or about to be: its push holds an earlier count or a slot already taken.
+__device__ __forceinline__ void push_by_class(int32_t* slots, int n, const pp_vm_classes& cls, int entry, int lane) {
+  const int q = entry >= 0 ? entry >> PP_VM_ID_BITS : -1;
+  const unsigned same = __match_any_sync(0xffffffffu, q);
+  const int leader = __ffs((int)same) - 1, rank = __popc(same & ((1u << lane) - 1));
+  int pos = 0;
+  if (q >= 0 && lane == leader) pos = atom_add_relaxed(&slots[n + VM_TAIL + q], __popc(same));
+  pos = __shfl_sync(0xffffffffu, pos, leader);
+  if (q >= 0) st_release(&slots[cls.base[q] + pos + rank], entry & ((1 << PP_VM_ID_BITS) - 1));
+  __syncwarp();
+  if (q >= 0 && lane == leader)
+    asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(&slots[n + VM_AVAIL + q]), "r"(__popc(same)) : "memory");
+}
+// -1: every task is done, or the run has failed
+__device__ __forceinline__ int take_by_class(int32_t* slots, int n, const pp_vm_classes& cls, pp_vm_state* st,
+                                             long long wait_ns, int lane) {
+  const unsigned long long t0 = gtimer_ns();
+  int slot = -1;  // of the secured task
+  for (;;) {
+    if (slot < 0) {
+      const int avail = lane < PP_VM_CLASSES ? ld_relaxed(&slots[n + VM_AVAIL + lane]) : 0;
+      const bool over = __any_sync(0xffffffffu, ld_relaxed(&st->error) != 0 || ld_relaxed(&st->done) >= n);
+      const unsigned some = __ballot_sync(0xffffffffu, avail > 0);
+      if (some) {
+        const int q = __ffs((int)some) - 1;
+        if (lane == 0) {
+          if (atom_add_relaxed(&slots[n + VM_AVAIL + q], -1) > 0)
+            slot = cls.base[q] + atom_add_relaxed(&slots[n + VM_HEAD + q], 1);
+          else
+            atom_add_relaxed(&slots[n + VM_AVAIL + q], 1);
+        }
+        slot = __shfl_sync(0xffffffffu, slot, 0);
+      } else if (over) {
+        return -1;
+      } else {
+        __nanosleep(32);
+      }
+    }
+    if (slot >= 0) {
+      const int id = __shfl_sync(0xffffffffu, ld_acquire(&slots[slot]), 0);
+      if (id >= 0) return id;
+    }
+    // bounded in time, as a wait on the one queue is
+    if (__any_sync(0xffffffffu, (long long)(gtimer_ns() - t0) > wait_ns)) {
+      if (lane == 0 && atomicCAS(&st->error, 0, PP_VM_TIMEOUT) == 0) st->err_info = slot >= 0 ? slot : ld_relaxed(&st->done);
+      return -1;
+    }
+  }
+}
+
 __global__ void __launch_bounds__(NT, 1)
     vm_kernel(const pp_task* __restrict__ tasks, int n_tasks, const int32_t* __restrict__ succ, int32_t* counters,
-              int32_t* slots, pp_vm_state* st, long long wait_ns, unsigned long long* trace, int use_tc) {
+              int32_t* slots, pp_vm_state* st, long long wait_ns, unsigned long long* trace, int use_tc, int by_class,
+              const __grid_constant__ pp_vm_classes cls) {
   extern __shared__ __align__(16) double smem[];
   __shared__ __align__(16) pp_task s_rec[2][4];  // this task's record, and those of its first successors
-  __shared__ int s_succ[32];                     // its first successors
+  __shared__ int s_succ[2][32];                  // its first successors, and the previous task's
   __shared__ int s_pub[32], s_npub;              // successors ready but not run here
   __shared__ int s_id;
   __shared__ int s_keep;  // position (in the successor list) of the successor run next, or -1
@@ -2358,6 +2433,7 @@ __global__ void __launch_bounds__(NT, 1)
   // and fences again, while warps 1 to 4 fetch the records of the first four successors; and the
   // ready successors that are not run here are pushed by the last warp beside the next task's loads.
   // Between tasks of the critical path of the dense N = 1024 factor: 2.0 us before, 1.2 us so.
+  const int id_mask = by_class ? (1 << PP_VM_ID_BITS) - 1 : 0x7FFFFFFF;
   int next = -1, par = 0, slot = 0;
   bool next_unfetched = false;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -2365,7 +2441,12 @@ __global__ void __launch_bounds__(NT, 1)
   for (;;) {
     int id = next;
     if (id < 0) {
-      if (threadIdx.x == 0) {
+      if (by_class) {
+        if (warp == 0) {
+          id = take_by_class(slots, n_tasks, cls, st, wait_ns, lane);
+          if (lane == 0) s_id = id;
+        }
+      } else if (threadIdx.x == 0) {
         const int idx = atomicAdd(&st->head, 1);
         if (idx < n_tasks) {
           const unsigned long long t_wait = gtimer_ns();
@@ -2402,14 +2483,16 @@ __global__ void __launch_bounds__(NT, 1)
     if (warp == 7) {
       // push what the previous task left ready, and fetch this task's successor list
       const int count = s_npub;
-      if (count > 0) {
+      if (count > 0 && by_class) {
+        push_by_class(slots, n_tasks, cls, lane < count ? s_pub[lane] : -1, lane);
+      } else if (count > 0) {
         int base = 0;
         if (lane == 0) base = atomicAdd(&st->tail, count);
         base = __shfl_sync(0xffffffffu, base, 0);
         if (lane < count) st_release(&slots[base + lane], s_pub[lane]);
       }
       if (lane < nsucc)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&s_succ[lane])), "l"(&succ[sbeg + lane])
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&s_succ[par][lane])), "l"(&succ[sbeg + lane])
                      : "memory");
       cp_async_commit();
     }
@@ -2428,14 +2511,14 @@ __global__ void __launch_bounds__(NT, 1)
           trace[3 * (size_t)id + 2] = smid() | ((unsigned long long)blockIdx.x << 32);
         }
       }
-      const int mine = lane < nsucc ? s_succ[lane] : -1;
-      const bool ready = mine >= 0 && atom_add_relaxed(&counters[mine], -1) == 1;
-      for (int q = lane + 32; q < nsucc; q += 32) {
-        const int sq = succ[sbeg + q];
-        if (atom_add_relaxed(&counters[sq], -1) == 1) {
-          __threadfence();
-          st_release(&slots[atomicAdd(&st->tail, 1)], sq);
-        }
+      const int mine = lane < nsucc ? s_succ[par][lane] : -1;
+      const bool ready = mine >= 0 && atom_add_relaxed(&counters[mine & id_mask], -1) == 1;
+      for (int q = 32; q < nsucc; q += 32) {
+        const int sq = q + lane < nsucc ? succ[sbeg + q + lane] : -1;
+        const bool now = sq >= 0 && atom_add_relaxed(&counters[sq & id_mask], -1) == 1;
+        if (now) __threadfence();
+        if (by_class) push_by_class(slots, n_tasks, cls, now ? sq : -1, lane);
+        else if (now) st_release(&slots[atomicAdd(&st->tail, 1)], sq);
       }
       __threadfence();  // the other predecessors' stores are visible from here on
       const unsigned all = __ballot_sync(0xffffffffu, ready);
@@ -2448,15 +2531,15 @@ __global__ void __launch_bounds__(NT, 1)
         atomicAdd(&st->done, 1);
       }
     } else if (warp <= 4 && warp - 1 < nsucc) {
-      const pp_task* rec = &tasks[s_succ[warp - 1]];
+      const pp_task* rec = &tasks[s_succ[par][warp - 1] & id_mask];
       if (lane < (int)(sizeof(pp_task) / 8))
         reinterpret_cast<unsigned long long*>(&s_rec[par ^ 1][warp - 1])[lane] =
             __ldg(reinterpret_cast<const unsigned long long*>(rec) + lane);
     }
     __syncthreads();
-    par ^= 1;
     const int keep = s_keep;
-    next = keep >= 0 ? s_succ[keep] : -1;
+    next = keep >= 0 ? s_succ[par][keep] & id_mask : -1;  // while the last warp fetches the next list
+    par ^= 1;
     next_unfetched = keep >= 4;
     slot = keep >= 0 && keep < 4 ? keep : 0;
   }
@@ -3226,10 +3309,12 @@ cudaError_t pp_vm_prepare() {
 cudaError_t pp_vm_run(const pp_vm_launch& L, cudaStream_t s) {
   if (L.n_tasks <= 0) return cudaSuccess;
   const int ib = 256;
+  const pp_vm_classes cls = L.classes ? *L.classes : pp_vm_classes{};
+  const int by_class = L.classes != nullptr;
   vm_init<<<(L.n_tasks + ib - 1) / ib, ib, 0, s>>>(L.indeg, L.ready, L.n_ready, L.n_tasks, L.counters, L.slots,
-                                                  L.state);
+                                                  L.state, by_class, cls);
   vm_kernel<<<L.grid, NT, pp_vm_smem_bytes(), s>>>(L.tasks, L.n_tasks, L.succ, L.counters, L.slots, L.state,
-                                                   L.wait_ns, L.trace, L.use_tc);
+                                                   L.wait_ns, L.trace, L.use_tc, by_class, cls);
   return cudaGetLastError();
 }
 

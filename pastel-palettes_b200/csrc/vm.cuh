@@ -22,6 +22,15 @@ typedef struct pp_vm_state {
   int pad[3];
 } pp_vm_state;
 
+/* Priority classes of ready tasks, the most urgent first: class q has the queue slots
+ * [base[q], base[q + 1]) and the entries [first[q], first[q + 1]) of the initially ready tasks.
+ * A successor entry holds the task id in its low PP_VM_ID_BITS and the task's class above them. */
+#define PP_VM_CLASSES 16
+#define PP_VM_ID_BITS 27
+struct pp_vm_classes {
+  int32_t base[PP_VM_CLASSES + 1], first[PP_VM_CLASSES + 1];
+};
+
 struct pp_vm_launch {
   const pp_task* tasks;
   int n_tasks;
@@ -36,6 +45,9 @@ struct pp_vm_launch {
                             before the kernel gives up */
   int grid;              /* CTAs (persistent)                                       */
   unsigned long long* trace = nullptr;  /* optional: 3 words per task (start ns, end ns, sm | cta << 32) */
+  /* null: one queue in order of readiness.  Otherwise the classes' queues; `slots` then has 3 x
+   * PP_VM_CLASSES counters behind the n_tasks slots */
+  const pp_vm_classes* classes = nullptr;
   int use_tc = 0;        /* the program holds TF32 tasks: tensor memory + an mbarrier per CTA */
 };
 
