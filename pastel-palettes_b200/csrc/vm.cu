@@ -114,6 +114,12 @@ __device__ __forceinline__ void st_if(double* p, double v, bool in) {
                : "memory");
 }
 
+__device__ __forceinline__ void sts_if(double* p, double v, bool in) {
+  asm volatile("{\n .reg .pred a;\n setp.ne.s32 a, %2, 0;\n @a st.shared.f64 [%1], %0;\n}\n" ::"d"(v), "r"(smem_u32(p)),
+               "r"((int)in)
+               : "memory");
+}
+
 __host__ __device__ constexpr int log2_of(int v) { return v <= 1 ? 0 : 1 + log2_of(v / 2); }
 
 // Four copies of one thread (16 bytes of `valid`, or 8), rows r, r + step, ... below `rows`, the
@@ -879,15 +885,15 @@ __device__ __noinline__ bool dev_gemm_bf16(double* __restrict__ C, int ldc, cons
 // back to divisions then.  Compared with `/` on 2^32 random pairs: no difference.
 __device__ __forceinline__ double rcp_seed(double v) {
   double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+  asm volatile("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
   return y;
 }
-__device__ __forceinline__ double reciprocal(double t) {
-  double y = rcp_seed(t);
+__device__ __forceinline__ double reciprocal(double t, double y) {  // y: rcp_seed(t)
   const double e = fma(-t, y, 1.0);
   y = fma(y, fma(e, e, e), y);
   return fma(fma(-t, y, 1.0), y, y);
 }
+__device__ __forceinline__ double reciprocal(double t) { return reciprocal(t, rcp_seed(t)); }
 __device__ __forceinline__ double quotient(double x, double t, double y) {
   double q = x * y;
   q = fma(fma(-q, t, x), y, q);
@@ -902,109 +908,147 @@ __device__ __forceinline__ int quotient_unsafe(double x, double t) {  // without
 }
 
 // ------------------------------------------------------------------------- GETRF
-// A[m x n] := L\U in place (m, n <= TL), like kernel.cu:104-147: step i divides the entries
-// below the pivot by a_ii and applies a_rc = fma(a_ic, -l_r, a_rc) to the trailing block.
-// Thread t = 16 ty + tx holds rows ty + 16 a and columns tx + 16 b (a, b < 4).  The pivot
-// row and the raw pivot column of step i are published to shared memory (double buffered)
-// by their owners at the end of step i - 1, so a step needs one CTA barrier; lanes tx < 4
-// of each half-warp form the multipliers of the half-warp's rows (one division each) and
-// share them by shuffles.  The steps run in four blocks of sixteen whose block index is a
-// compile-time constant: register selection, the shrinking trailing region and most
-// bounds tests then cost nothing at run time.
-struct GetrfState {
-  double x[4][4];
-  double* prow;  // [2][TL]
-  double* pcol;  // [2][TL]
-  int tx, ty, lane, m;
-};
-
-template <int JB>
-__device__ __forceinline__ void getrf_publish(GetrfState& S, int j, int buf) {
-  const int jj = j & 15;
-  if (S.ty == jj) {
-#pragma unroll
-    for (int b = JB; b < 4; ++b) S.prow[buf * TL + S.tx + 16 * b] = S.x[JB][b];
-  }
-  if (S.tx == jj) {
-#pragma unroll
-    for (int a = JB; a < 4; ++a) S.pcol[buf * TL + S.ty + 16 * a] = S.x[a][JB];
-  }
-}
-
-template <int IB>
-__device__ __forceinline__ void getrf_step(GetrfState& S, int i, int i_end, int mn) {
-  const int ii = i & 15, buf = i & 1;
+#define GETRF_LD (TL + 3)  /* odd: lanes along rows and fragments both nearly free of bank conflicts */
+// the whole block with divisions, for values out of the quotients' range
+__device__ __noinline__ void getrf_by_division(double* A, int lda, int m, int n) {
+  extern __shared__ __align__(16) double vm_smem[];
+  double* S = vm_smem;
+  const int tid = threadIdx.x;
+  for (int e = tid; e < m * n; e += NT) S[(e / n) * GETRF_LD + e % n] = ldcg(&A[(size_t)(e / n) * lda + e % n]);
   __syncthreads();
-  const double piv = S.prow[buf * TL + i];
-  double lm = 0.0;
-  if (S.tx >= IB && S.tx < 4) {
-    const int r = S.ty + 16 * S.tx;
-    if (r > i && r < S.m) lm = S.pcol[buf * TL + r] / piv;
-  }
-  double l[4], u[4];
-#pragma unroll
-  for (int a = IB; a < 4; ++a) l[a] = __shfl_sync(0xffffffffu, lm, (S.lane & 16) | a);
-#pragma unroll
-  for (int b = IB; b < 4; ++b) u[b] = S.prow[buf * TL + S.tx + 16 * b];
-  const bool row_below = S.ty > ii, col_right = S.tx > ii;
-#pragma unroll
-  for (int a = IB; a < 4; ++a)
-#pragma unroll
-    for (int b = IB; b < 4; ++b) {
-      const bool live = (a > IB || row_below) && (b > IB || col_right);
-      if (live) S.x[a][b] = fma(u[b], -l[a], S.x[a][b]);
+  for (int i = 0; i < min(m, n); ++i) {
+    const double* u = S + i * GETRF_LD;
+    for (int r = i + 1 + tid; r < m; r += NT) S[r * GETRF_LD + i] = S[r * GETRF_LD + i] / u[i];
+    __syncthreads();
+    for (int e = tid; e < (m - i - 1) * (n - i - 1); e += NT) {
+      double* x = S + (i + 1 + e / (n - i - 1)) * GETRF_LD;
+      const int c = i + 1 + e % (n - i - 1);
+      x[c] = fma(u[c], -x[i], x[c]);
     }
-  if (S.tx == ii) {  // column i keeps its multipliers (the L part)
-#pragma unroll
-    for (int a = IB; a < 4; ++a)
-      if (a > IB || row_below) S.x[a][IB] = l[a];
+    __syncthreads();
   }
-  if (i + 1 < i_end) getrf_publish<IB>(S, i + 1, buf ^ 1);
-  else if constexpr (IB < 3) {
-    if (i + 1 < mn) getrf_publish<IB + 1>(S, i + 1, buf ^ 1);
-  }
+  for (int e = tid; e < m * n; e += NT) A[(size_t)(e / n) * lda + e % n] = S[(e / n) * GETRF_LD + e % n];
 }
 
-template <int IB>
-__device__ __forceinline__ void getrf_block(GetrfState& S, int mn) {
-  const int i_end = min(mn, 16 * IB + 16);
-  if (i_end == 16 * IB + 16) {
-#pragma unroll
-    for (int t = 0; t < 16; ++t) getrf_step<IB>(S, 16 * IB + t, i_end, mn);
-  } else {
+// A[m x n] := L\U in place (m, n <= TL), like kernel.cu:104-147: step i divides the entries below the
+// pivot by a_ii and applies a_rc = fma(a_ic, -l_r, a_rc) to the trailing block.
+//
+// The block stays in shared memory, eight columns per warp.  When a panel of eight is factored, the warp
+// of the next one applies it to its columns and factors them, two rows per lane, while the warps
+// further right solve their eight rows against it and update the rows below on the FP64 tensor cores (a
+// chain of fma in ascending i, see dmma): one CTA barrier per eight steps.  A lane's row moves one place
+// to the left in its registers with each step, so that the steps are one loop: beside SMs that load the
+// memory system, what the instruction costs is its code's way here (the unrolled form before, with
+// a barrier and a division per step: 20 us alone, 56 us beside the products of a mixed-precision
+// factorization).  What bounds it is a step's chain: shuffle, reciprocal, quotient, update.
+// 64 x 64 on a B200, hop included: 20.4 -> 18.2 us alone, 56 -> 21 us there.
+__device__ __forceinline__ void dev_getrf(double* A, int lda, int m, int n) {
+  extern __shared__ __align__(16) double vm_smem[];
+  double* S = vm_smem;  // TL x GETRF_LD (and a panel's width of reads past its end)
+  const int tid = thread_index(), warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3;
+  const int mn = min(m, n), panels = (mn + 7) >> 3, cg = 8 * warp;
+  int bad = 0;
+  {
+    const int c = tid & 63;
+    if (c < n) {
+#pragma unroll 4
+      for (int r = tid >> 6; r < m; r += NT / 64) cp_async8(smem_u32(S + r * GETRF_LD + c), A + (size_t)r * lda + c, 8u);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+  }
+  __syncthreads();
 #pragma unroll 1
-    for (int i = 16 * IB; i < i_end; ++i) getrf_step<IB>(S, i, i_end, mn);
+  for (int J = -1; J < panels; ++J) {
+    const int c0 = 8 * J;
+    const bool next = warp == J + 1 && warp < panels;
+    if (J >= 0 && cg < n && warp > J && !next) {
+      // rows c0 .. c0 + 7 of these columns: solve against the panel's unit lower triangle
+      double* u = S + (c0 + fa) * GETRF_LD;
+      double x0 = u[cg + 2 * fb], x1 = u[cg + 2 * fb + 1], c = u[c0];
+#pragma unroll 1
+      for (int i = 0; i < 7; ++i) {
+        const double v0 = __shfl_sync(0xffffffffu, x0, 4 * i + fb), v1 = __shfl_sync(0xffffffffu, x1, 4 * i + fb);
+        const double y0 = fma(v0, -c, x0), y1 = fma(v1, -c, x1);
+        c = u[c0 + i + 1];
+        x0 = fa > i ? y0 : x0;
+        x1 = fa > i ? y1 : x1;
+      }
+      u[cg + 2 * fb] = x0;
+      u[cg + 2 * fb + 1] = x1;
+      __syncwarp();
+      const double b0 = S[(c0 + fb) * GETRF_LD + cg + fa], b1 = S[(c0 + 4 + fb) * GETRF_LD + cg + fa];
+#pragma unroll 4
+      for (int t = c0 + 8; t < m; t += 8) {  // tiles of eight rows; rows past m stay inside S
+        double* p = S + (t + fa) * GETRF_LD;
+        double y0 = p[cg + 2 * fb], y1 = p[cg + 2 * fb + 1];
+        dmma(y0, y1, -p[c0 + fb], b0);
+        dmma(y0, y1, -p[c0 + 4 + fb], b1);
+        p[cg + 2 * fb] = y0;
+        p[cg + 2 * fb + 1] = y1;
+      }
+      __syncwarp();
+    }
+    if (next) {  // the next panel, in rows: this panel's steps applied to it, then its own
+      const int w = min(8, n - cg), steps = min(8, mn - cg), r0 = max(c0, 0), off = cg - r0;
+      const int ra = min(r0 + lane, TL - 1), rb = min(r0 + lane + 32, TL - 1);
+      double x[2][8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        x[0][c] = S[ra * GETRF_LD + cg + c];
+        x[1][c] = S[rb * GETRF_LD + cg + c];
+      }
+      double la = S[ra * GETRF_LD + r0], lb = S[rb * GETRF_LD + r0];
+#pragma unroll 1
+      for (int i = 0; i < off; ++i) {
+        double* row = S + (r0 + i) * GETRF_LD + cg;  // becomes a row of U
+#pragma unroll
+        for (int c = 0; c < 8; ++c) sts_if(row + c, x[0][c], lane == i && c < w);
+        __syncwarp();
+        double u[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) u[c] = row[c];
+        const double na = -la, nb = -lb;
+        la = S[ra * GETRF_LD + r0 + i + 1];
+        lb = S[rb * GETRF_LD + r0 + i + 1];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {  // lanes up to i have their row of U in place: of no consequence
+          x[0][c] = fma(u[c], na, x[0][c]);
+          x[1][c] = fma(u[c], nb, x[1][c]);
+        }
+      }
+#pragma unroll 1
+      for (int i = 0; i < steps; ++i) {
+        double* row = S + (cg + i) * GETRF_LD + cg + i;
+        const double p = __shfl_sync(0xffffffffu, x[0][0], off + i), seed = rcp_seed(p);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) sts_if(row + c, x[0][c], lane == off + i && c < w - i);
+        __syncwarp();
+        double u[8];
+#pragma unroll
+        for (int c = 1; c < 8; ++c) u[c] = row[c];  // past the panel: of no consequence
+        const double y = reciprocal(p, seed);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = r0 + lane + 32 * h, below = (int)(lane + 32 * h > off + i) & (int)(r < m);
+          const double l = quotient(x[h][0], p, y);
+          bad |= below & quotient_unsafe(x[h][0], p);
+          sts_if(S + (h ? rb : ra) * GETRF_LD + cg + i, l, below);
+#pragma unroll
+          for (int c = 1; c < 8; ++c) x[h][c - 1] = fma(u[c], -l, x[h][c]);
+        }
+      }
+    }
+    __syncthreads();
   }
-}
-
-__device__ __noinline__ void dev_getrf(double* A, int lda, int m, int n, double* smem) {
-  GetrfState S;
-  S.prow = smem;
-  S.pcol = smem + 2 * TL;
-  S.tx = threadIdx.x & 15;
-  S.ty = threadIdx.x >> 4;
-  S.lane = threadIdx.x & 31;
-  S.m = m;
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int r = S.ty + 16 * a, c = S.tx + 16 * b;
-      S.x[a][b] = (r < m && c < n) ? ldcg(&A[(size_t)r * lda + c]) : 0.0;
-    }
-  const int mn = min(m, n);
-  if (mn > 0) getrf_publish<0>(S, 0, 0);
-  getrf_block<0>(S, mn);
-  getrf_block<1>(S, mn);
-  getrf_block<2>(S, mn);
-  getrf_block<3>(S, mn);
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int r = S.ty + 16 * a, c = S.tx + 16 * b;
-      if (r < m && c < n) A[(size_t)r * lda + c] = S.x[a][b];
-    }
+  if (__syncthreads_or(bad)) {
+    getrf_by_division(A, lda, m, n);
+  } else {
+    const int c = tid & 63;
+    if (c < n)
+#pragma unroll 4
+      for (int r = tid >> 6; r < m; r += NT / 64) A[(size_t)r * lda + c] = S[r * GETRF_LD + c];
+  }
   __syncthreads();
 }
 
@@ -1019,8 +1063,7 @@ __device__ __noinline__ void dev_getrf(double* A, int lda, int m, int n, double*
 // FP64 tensor cores (a chain of fma in ascending i, see dmma); the next group's warp goes on to
 // factor it while the others still update.  One CTA barrier per eight steps; the instructions of
 // the one warp that factors bound it.  64 x 64, hop included: 80 -> 41 us (before: the whole block
-// in shared memory with four CTA barriers per step).  Without pivoting the routine above is as fast.
-#define GETRF_LD (TL + 4)
+// in shared memory with four CTA barriers per step).
 // the pivot of step ci among the rows at positions >= ci (a lane's two rows: values v0, v1 at
 // positions pos): lane pl, half ph; swaps the positions of the pivot row and of the row at ci
 __device__ __forceinline__ void getrf_pivot(double v0, double v1, int (&pos)[2], int ci, int m, int& pl, int& ph) {
@@ -2202,7 +2245,7 @@ __device__ bool run_task(const pp_task& T, double* smem, TcCtx& tc, int& err) {
         if (!T.p[1]) return false;
         dev_getrf_piv(T.p[0], T.ld[0], T.m, T.n, T.p[1]);
       } else {
-        dev_getrf(T.p[0], T.ld[0], T.m, T.n, smem);
+        dev_getrf(T.p[0], T.ld[0], T.m, T.n);
       }
       return true;
     case PP_OP_TRSML:
