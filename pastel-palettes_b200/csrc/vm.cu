@@ -3,10 +3,11 @@
 // Replaces the reference's `kernel_dynamic` (Pastel-Palettes src/kernel.cu:1375-1526).
 // The reference gives each thread block a fixed, statically scheduled instruction
 // stream and makes blocks spin on per-instruction flags in global memory.  Here every
-// CTA of a persistent grid pops the next READY task from a device queue; finishing a
-// task decrements its successors' dependency counters (acq_rel atomics) and pushes the
-// ones that reach zero.  Waits are bounded: a CTA that polls an empty slot for
-// longer than its time limit (globaltimer) records PP_VM_TIMEOUT and every CTA returns.
+// CTA of a persistent grid takes the next READY task from a device queue (one queue, or one per
+// priority class); finishing a task decrements its successors' dependency counters, and of those
+// that reach zero the CTA runs the first and pushes the others.  Waits are bounded: a CTA that
+// finds nothing for longer than its time limit (globaltimer) records PP_VM_TIMEOUT and every CTA
+// returns.
 //
 // Arithmetic contract (FP64 path): every matrix element receives its updates in the
 // order the reference's routines apply them, one fma per product with the same
@@ -16,11 +17,18 @@
 //   TRSMR  kernel.cu:185-226   x_ri = b_ri / u_ii; b_rc = fma(-x_ri, u_ic, b_rc)
 //   TRSMRT kernel.cu:229-285   x_ic = v_ic * (1 / u_ii); v_rc = fma(-u_ir, x_ic, v_rc)
 //   GEMM   kernel.cu:288-664   c_ij = fma(alpha a_ik, b_kj, c_ij), k ascending from beta c_ij
-// Work distribution does not touch that order: GEMM tiles are shaped to the operands
-// (square, skinny, single column, small output with a long k), the triangular routines
-// keep each column (or row) in registers across four lanes of a warp and broadcast the
-// finished pivot entry with a shuffle, so they need no CTA barrier per step.
-// All global loads of data other CTAs may have written use ld.global.cg (L2), never L1.
+// Work distribution does not touch that order: an FP64 tensor-core product (dmma) gives the bits of
+// the same chain of fma, and the routines feed it in ascending k.  Only products marked free-order
+// (the solves', whose sums no contract fixes) are split over lanes and warps.
+// Data other CTAs have written is loaded past L1 (ld.global.cg, cp.async.cg) or through it (8-byte
+// cp.async, SHADOW's 32-byte loads): a task starts behind a gpu-scope acquire of its CTA, which
+// invalidates that SM's L1.
+//
+// What an instruction costs inside the VM is often its code: its lines have been evicted by the tasks
+// before, a scheduler holds two warps, a taken branch costs one about 30 cycles, and beside SMs that
+// load the memory system a fetch costs several times as much.  So each routine is one compact
+// piece of code, inlined once (a call spills more than it saves), loops are rolled where the body
+// is long enough, and conditions on lanes are predicates, not branches.
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -34,7 +42,6 @@
 
 #define NT PP_VM_THREADS
 #define TL PP_VM_TILE
-#define LDS (PP_VM_TILE + 1)   /* padded smem row stride (doubles) */
 #define VM_SMEM_BYTES 184320   /* 180 KB, one CTA per SM: ACCUM keeps its ny x k1 sketch on chip;
                                   the BF16 GEMM holds 3 stages of 48 KB + its epilogue's buffers */
 
@@ -109,6 +116,13 @@ __device__ __forceinline__ double ldcg_if(const double* p, bool in) {
                : "memory");
   return v;
 }
+__device__ __forceinline__ void ldcg2_if(double& x, double& y, const double* p, bool in) {  // 16-byte aligned
+  asm volatile("{\n .reg .pred a;\n setp.ne.s32 a, %3, 0;\n mov.f64 %0, 0d0000000000000000;\n mov.f64 %1, %0;\n"
+               " @a ld.global.cg.v2.f64 {%0, %1}, [%2];\n}\n"
+               : "=&d"(x), "=&d"(y)
+               : "l"(p), "r"((int)in)
+               : "memory");
+}
 __device__ __forceinline__ void st_if(double* p, double v, bool in) {
   asm volatile("{\n .reg .pred a;\n setp.ne.s32 a, %2, 0;\n @a st.global.f64 [%1], %0;\n}\n" ::"d"(v), "l"(p), "r"((int)in)
                : "memory");
@@ -161,11 +175,10 @@ __device__ __forceinline__ void copy_rows4(uint32_t& dst, const char*& src, int&
 // What bounds it: the loads' latency and the staging's instructions for small products, the FP64
 // tensor rate (2.1 M cycles for 512^3) and the staging that is not overlapped with it for large ones.
 // Time per instruction on a B200, hop to the next task included (before: SIMT tiles by shape, whose
-// operand loads were waited for before each chunk's products; hop 2.5 us):
-//   64 x 64 x 64     16.5 -> 9.1 us     64 x 16 x 64      15.9 -> 5.5 us
-//   64 x 64 x 256    42   -> 17.6 us    16 x 16 x 512     25   -> 10.8 us (k over 8 warps)
-//   512 x 512 x 512  2630 -> 1655 us    512 x 32 x 512    327  -> 105 us
-//   64 x 8 x 512     43   -> 15.3 us    256 x 1 x 256     48   -> 19 us
+// operand loads were waited for before each chunk's products):
+//   64 x 64 x 64     17 -> 7.3 us        64 x 16 x 64      16 -> 5.1 us
+//   64 x 64 x 256    42 -> 17 us         16 x 16 x 512     25 -> 7.4 us (k over 8 warps)
+//   512 x 512 x 512  2640 -> 1655 us     512 x 32 x 512    327 -> 105 us
 #define GM_KC 64
 #define GM_LD (GM_KC + 4)
 #define GM_ST 2
@@ -1295,9 +1308,9 @@ __device__ __noinline__ double2 tri_by_division(double x0, double x1, double tii
 // every kind runs forward), a warp takes eight lines and needs no other warp from there on.  Eight
 // positions at a time: the sum over the earlier positions on the FP64 tensor cores (a chain of fma
 // in ascending i, see dmma), then the eight against each other with shuffles (about 40 cycles a
-// position, 140 with a quotient), which bounds it.  On a B200, hop of 2.5 us included (before: a
+// position, 140 with a quotient), which bounds it.  On a B200, hop to the next task included (before: a
 // shuffled sweep over all 64 positions, unrolled, its coefficients fetched step by step):
-//   64 x 64: TRSML 18 -> 11 us, TRSMR 22.8 -> 14.5 us;  TRSML 256 x 64: 149 -> 63 us
+//   64 x 64: TRSML 18 -> 10.5 us, TRSMR 22.5 -> 14 us;  TRSML 256 x 64: 148 -> 61 us
 #define TRI_LDX 12  /* doubles between positions of a warp's lines: 4 mod 8, no bank conflicts */
 __device__ __forceinline__ void dev_tri(int op, double* B, int ldb, const double* T, int ldt, int len, int lines,
                                         const double* perm) {
@@ -1405,11 +1418,13 @@ __device__ __forceinline__ void dev_tri(int op, double* B, int ldb, const double
 // The explicit inverses of the leaves (TRMV) and the solves' products with a leaf or a low-rank
 // factor: S is staged in shared memory, a warp takes eight rows of M at a time straight from global
 // memory into FP64 tensor-core fragments, two columns per load (the k order is free: even columns in
-// one chain, odd ones in another), the next 64 columns loading during the products; nothing of a row
-// depends on which other rows the call covers.  Bound by one CTA's loads.  On a B200, hop of 2.5 us included
-// (before: warps along the columns, a shuffle reduction per row and right-hand side):
-//   TRMV 128 x 4, 64 rows  13 -> 6 us    94 x 1  13.5 -> 6 us    512 x 8, 64 rows  31 -> 12 us
-//   products 64 x 8 x 512  15 -> 12 us   61 x 4 x 64  5.5 -> 4 us  (the latter from the general routine)
+// one chain, odd ones in another); nothing of a row depends on which other rows the call covers.  Bound
+// by one CTA's loads and by the instructions around them: with the next 64 columns loading during the
+// products it is no faster (10.4 k cycles either way at 64 x 8 x 512), and those registers cost every
+// instruction of the VM 1% in spills.  On a B200, time of the task (before: warps along the columns, a
+// shuffle reduction per row and right-hand side):
+//   TRMV 128 x 4, 64 rows  11.5 -> 3.3 us   512 x 8, 64 rows  29 -> 7.5 us
+//   products 64 x 8 x 512  42 -> 10.2 us   256 x 4 x 32  17 -> 4.9 us
 #define RW_U 8  /* steps of 8 columns whose loads go out together */
 __device__ __forceinline__ void dev_rows(double* O, int ldo, const double* M, int ldm, const double* S, int lds, int m,
                                          int n, int rows, int tri, int r0, double alpha, double beta) {
@@ -1454,7 +1469,7 @@ __device__ __forceinline__ void dev_rows(double* O, int ldo, const double* M, in
         }
       }
     };
-    double v[RW_U][2], w[RW_U][2], old[2][2];
+    double v[RW_U][2], old[2][2];
     load(cb, v);
     double* o = O + (size_t)r * ldo + 2 * fb;
 #pragma unroll
@@ -1463,7 +1478,6 @@ __device__ __forceinline__ void dev_rows(double* O, int ldo, const double* M, in
       for (int e = 0; e < 2; ++e) old[j][e] = ldcg_if(o + 8 * j + e, rin && 8 * j + 2 * fb + e < n && beta != 0.0);
 #pragma unroll 1
     for (int c0 = cb; c0 < ce; c0 += 8 * RW_U) {
-      if (c0 + 8 * RW_U < ce) load(c0 + 8 * RW_U, w);
       if ((tri == 0 && c0 + 8 * RW_U > r0 + t) || (tri == 1 && c0 < r0 + t + 8)) {
         // what lies outside the triangle is not used as a value
 #pragma unroll
@@ -1483,11 +1497,7 @@ __device__ __forceinline__ void dev_rows(double* O, int ldo, const double* M, in
           dmma(acc[1][1][0], acc[1][1][1], v[u][1], b[ls + 8]);
         }
       }
-#pragma unroll
-      for (int u = 0; u < RW_U; ++u) {
-        v[u][0] = w[u][0];
-        v[u][1] = w[u][1];
-      }
+      if (c0 + 8 * RW_U < ce) load(c0 + 8 * RW_U, v);
     }
 #pragma unroll
     for (int j = 0; j < 2; ++j)
@@ -1495,6 +1505,101 @@ __device__ __forceinline__ void dev_rows(double* O, int ldo, const double* M, in
       for (int e = 0; e < 2; ++e) {
         st_if(o + 8 * j + e, fma(alpha, acc[0][j][e] + acc[1][j][e], old[j][e]), rin && 8 * j + 2 * fb + e < n);
       }
+  }
+  __syncthreads();
+}
+
+// The same for one right-hand side, with FMAs: 4 columns per lane (adjacent, or a row's width apart where
+// pairs are not aligned), 4 to 32 lanes along a row or along 128 columns of it, eight rows per lane at a
+// time, from global memory; the eight sums are exchanged so that each lane ends with one (or two).  The
+// tensor-core form above spends seven eighths of its work on columns that are not there, and its
+// instructions are what such a product costs (about five cycles each, fetched for this task).  O may be
+// S: it is read once, before a barrier, or kept in shared memory where it has more than 128 rows.  Cycles on a B200, the form above -> this one:
+//   256 x 16  6100 -> 1650   111 x 24  3500 -> 1630   94 x 94 triangle  5600 -> 4400   111 x 111  6600 -> 4600
+//   64 x 256  3200 -> 2500   256 x 256  18000 -> 15200
+__device__ __forceinline__ void dev_column(double* O, int ldo, const double* M, int ldm, const double* S, int sr, int m,
+                                           int rows, int tri, int r0, double alpha, double beta) {
+  extern __shared__ __align__(16) double vm_smem[];
+  const int tid = thread_index(), warp = tid >> 5, lane = tid & 31;
+  const int lg = m <= 16 ? 2 : m <= 32 ? 3 : m <= 64 ? 4 : 5;  // log2 of the lanes per row
+  const int cl = lane & ((1 << lg) - 1), rl = lane >> lg, step = 32 >> lg;
+  const bool wide = !((ldm | m | (int)(reinterpret_cast<uintptr_t>(M) >> 3)) & 1), once = m <= 128, inplace = O == S;
+  const int cs = wide ? 1 : 1 << lg;  // this lane's columns: c + e cs
+  const int fin = 4 * (cl & 1) + (cl & 2) + (lg > 2 ? (cl >> 2) & 1 : 0);  // the first of the eight sums that stays here
+  const bool staged = inplace && !once;
+  if (staged) {
+    for (int e = tid; e < m; e += NT) vm_smem[e] = ldcg(S + (size_t)e * sr);
+    __syncthreads();
+  }
+  double s[4];
+  bool first = true;
+#pragma unroll 1
+  for (int t = 8 * step * warp; t < rows || (first && inplace && once); t += 64 * step) {
+    double v[8], old[2];
+    const int r = t + rl + fin * step, end = once || tri != 0 ? m : min(m, r0 + t + 8);
+    double* o = O + (size_t)r * ldo;
+    old[0] = ldcg_if(o, beta != 0.0 && r < rows && cl < 8);
+    old[1] = ldcg_if(o + (size_t)step * ldo, beta != 0.0 && lg == 2 && r + step < rows);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = 0.0;
+#pragma unroll 1
+    for (int c0 = once || tri != 1 ? 0 : (r0 + t) & ~127; c0 < end; c0 += 128) {
+      const int c = c0 + (wide ? 4 * cl : cl);
+      const double* p = M + (size_t)(t + rl) * ldm + c;
+      double x[8][4];
+      if (!once || first) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (staged) s[e] = c + e * cs < m ? vm_smem[c + e * cs] : 0.0;
+          else s[e] = ldcg_if(S + (size_t)(c + e * cs) * sr, c + e * cs < m);
+        }
+      }
+      if (wide) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const bool in = t + rl + i * step < rows;
+          ldcg2_if(x[i][0], x[i][1], p, in && c < end);
+          ldcg2_if(x[i][2], x[i][3], p + 2, in && c + 2 < end);
+          p += (size_t)step * ldm;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const bool in = t + rl + i * step < rows;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[i][e] = ldcg_if(p + e * cs, in && c + e * cs < end);
+          p += (size_t)step * ldm;
+        }
+      }
+      if (first && inplace && once) __syncthreads();  // every thread has its part of S
+      first = false;
+      if (tri != 2) {  // what lies outside the triangle is not used as a value
+        const int k = c - (r0 + t + rl);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[i][e] = (tri == 0 ? k + e * cs <= i * step : k + e * cs >= i * step) ? x[i][e] : 0.0;
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = fma(x[i][e], s[e], v[i]);
+    }
+#pragma unroll
+    for (int h = 4; h > 0; h >>= 1) {  // halves exchanged with the lane 4 / h away
+      if (h > 1 || lg > 2) {
+        const bool up = cl & (4 / h);
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+          const double other = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + h], 4 / h);
+          v[i] = (up ? v[i + h] : v[i]) + other;
+        }
+      }
+    }
+    if (lg > 3) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 8);
+    if (lg > 4) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
+    st_if(o, fma(alpha, v[0], old[0]), r < rows && cl < 8);
+    st_if(o + (size_t)step * ldo, fma(alpha, v[1], old[1]), lg == 2 && r + step < rows);
   }
   __syncthreads();
 }
@@ -2150,14 +2255,20 @@ __device__ __forceinline__ void run_composite(const pp_task& T) {
   // products of the solves, in free order: a leaf, its inverse or a low-rank factor times a few
   // right-hand sides (columns that stage in shared memory), and a few right-hand sides' transposes
   // times a low-rank factor (short k stays with the general product: 8 warps of 8 rows are not fewer
-  // steps than its one chunk)
-  if (T.op == PP_OP_TRMV || (free_order && !tA && !tB && T.n <= 16 && T.k <= 1024)) {
+  // steps than its one chunk; so do several transposed columns: 94 x 16 x 16 took 3.05 us instead of 2.8)
+  if (T.op == PP_OP_TRMV || (free_order && !tA && T.n <= (tB ? 1 : 16) && T.k <= 1024)) {
     const bool trmv = T.op == PP_OP_TRMV, part = trmv && T.l > 0;
     const int r0 = part ? T.o : 0;
     const double* S = trmv ? (part ? T.p[2] : T.p[0]) : T.p[2];
     const int lds = trmv ? (part ? T.ld[2] : T.ld[0]) : T.ld[2];
-    dev_rows(T.p[0], T.ld[0], T.p[1] + (size_t)r0 * T.ld[1], T.ld[1], S, lds, trmv ? T.m : T.k, T.n, part ? T.l : T.m,
-             !trmv ? 2 : T.ctrl == 1 ? 1 : T.ctrl == 0 ? 0 : 2, r0, trmv ? 1.0 : T.alpha, trmv ? 0.0 : T.beta);
+    const int m = trmv ? T.m : T.k, rows = part ? T.l : T.m, tri = !trmv ? 2 : T.ctrl == 1 ? 1 : T.ctrl == 0 ? 0 : 2;
+    const double* M = T.p[1] + (size_t)r0 * T.ld[1];
+    const double alpha = trmv ? 1.0 : T.alpha, beta = trmv ? 0.0 : T.beta;
+    // one column: with FMAs; more of them: on the tensor cores
+    if (T.n == 1 && m > 0)
+      dev_column(T.p[0], T.ld[0], M, T.ld[1], S, !trmv && tB ? 1 : lds, m, rows, tri, r0, alpha, beta);
+    else
+      dev_rows(T.p[0], T.ld[0], M, T.ld[1], S, lds, m, T.n, rows, tri, r0, alpha, beta);
     return;
   }
   if (free_order && tA && !tB && T.m <= 16 && T.n <= 32 && T.k >= 64) {
