@@ -1425,19 +1425,39 @@ __device__ __forceinline__ void dev_tri(int op, double* B, int ldb, const double
 // shuffle reduction per row and right-hand side):
 //   TRMV 128 x 4, 64 rows  11.5 -> 3.3 us   512 x 8, 64 rows  29 -> 7.5 us
 //   products 64 x 8 x 512  42 -> 10.2 us   256 x 4 x 32  17 -> 4.9 us
+// A fragment's zeros outside the triangle, or past the last column, would make NaN of an infinity or a
+// NaN in S: with one there the product is summed entry by entry (rows_exact).
 #define RW_U 8  /* steps of 8 columns whose loads go out together */
+__device__ __noinline__ void rows_exact(double* O, int ldo, const double* M, int ldm, int ls, int m, int n, int rows,
+                                        int tri, int r0, double alpha, double beta) {
+  extern __shared__ __align__(16) double vm_smem[];
+  for (int e = threadIdx.x; e < rows * n; e += NT) {
+    const int r = e / n, q = e - r * n, end = tri == 0 ? r0 + r + 1 : m;
+    double sum = 0.0;
+    for (int c = tri == 1 ? r0 + r : 0; c < end; ++c) sum = fma(ldcg(&M[(size_t)r * ldm + c]), vm_smem[c * ls + q], sum);
+    double* o = O + (size_t)r * ldo + q;
+    *o = beta != 0.0 ? fma(alpha, sum, ldcg(o)) : alpha * sum;
+  }
+  __syncthreads();
+}
 __device__ __forceinline__ void dev_rows(double* O, int ldo, const double* M, int ldm, const double* S, int lds, int m,
                                          int n, int rows, int tri, int r0, double alpha, double beta) {
   extern __shared__ __align__(16) double vm_smem[];
   const int tid = thread_index(), warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3;
   const int ns = n <= 8 ? 8 : 16, ls = ns + 2, lm = (m + 7) & ~7;  // stride 2 mod 8: no bank conflicts
+  int special = 0;
 #pragma unroll 4
   for (int e = tid; e < lm * ns; e += NT) {
     const int r = n <= 8 ? e >> 3 : e >> 4, q = e & (ns - 1);
-    vm_smem[r * ls + q] = ldcg_if(S + (size_t)r * lds + q, r < m && q < n);
+    const double v = ldcg_if(S + (size_t)r * lds + q, r < m && q < n);
+    special |= (int)((__double2hiint(v) & 0x7FF00000) == 0x7FF00000);
+    vm_smem[r * ls + q] = v;
   }
   const bool wide = !((ldm | (int)(reinterpret_cast<uintptr_t>(M) >> 3)) & 1);
-  __syncthreads();
+  if (__syncthreads_or(special)) {
+    rows_exact(O, ldo, M, ldm, ls, m, n, rows, tri, r0, alpha, beta);
+    return;
+  }
 #pragma unroll 1
   for (int t = 8 * warp; t < rows; t += 64) {
     const int r = t + fa;
@@ -1573,17 +1593,14 @@ __device__ __forceinline__ void dev_column(double* O, int ldo, const double* M, 
       }
       if (first && inplace && once) __syncthreads();  // every thread has its part of S
       first = false;
-      if (tri != 2) {  // what lies outside the triangle is not used as a value
-        const int k = c - (r0 + t + rl);
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) x[i][e] = (tri == 0 ? k + e * cs <= i * step : k + e * cs >= i * step) ? x[i][e] : 0.0;
-      }
+      const int k = c - (r0 + t + rl);
 #pragma unroll
       for (int e = 0; e < 4; ++e)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = fma(x[i][e], s[e], v[i]);
+        for (int i = 0; i < 8; ++i) {  // what lies outside the triangle, or the matrix, is not used
+          const double y = fma(x[i][e], s[e], v[i]);
+          v[i] = (tri == 2 || (tri == 0 ? k + e * cs <= i * step : k + e * cs >= i * step)) ? y : v[i];
+        }
     }
 #pragma unroll
     for (int h = 4; h > 0; h >>= 1) {  // halves exchanged with the lane 4 / h away

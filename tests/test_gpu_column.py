@@ -58,3 +58,21 @@ def test_triangle(pp, gctx, m, upper, part):
     out = dev(np.full((n, 1), 7.0))
     launch(pp, gctx, op=TRMV, m=m, n=1, o=o, l=n, ctrl=upper, p=[out, dev(A), dev(x)], ld=[1, m + pad, 1])
     assert (np.abs(out.cpu().numpy()[:, 0] - want[o : o + n]) <= bound[o : o + n]).all()
+
+
+@pytest.mark.parametrize("n", [1, 2, 9])
+@pytest.mark.parametrize("tri", [0, 1, 2])
+@pytest.mark.parametrize("m", [5, 30, 94, 200])
+def test_infinite_entry_stays_in_its_rows(pp, gctx, m, n, tri):
+    """An infinity in the right-hand side reaches the rows whose coefficients meet it, and no other."""
+    rng = np.random.default_rng(m)
+    A, x = rng.uniform(1, 2, (m, m)), rng.uniform(1, 2, (m, n))
+    T = [np.tril, np.triu, np.array][tri](A)
+    x[m // 2, 0] = np.inf
+    out = dev(np.zeros((m, n)))
+    if tri == 2:
+        launch(pp, gctx, op=GEMM, flags=1, m=m, n=n, k=m, alpha=1.0, beta=0.0, p=[out, dev(A), dev(x)], ld=[n, m, n])
+    else:
+        launch(pp, gctx, op=TRMV, m=m, n=n, o=0, l=m, ctrl=tri, p=[out, dev(A), dev(x)], ld=[n, m, n])
+    got, meets = out.cpu().numpy(), T[:, m // 2] != 0
+    assert np.isposinf(got[meets, 0]).all() and np.isfinite(got[~meets, 0]).all() and np.isfinite(got[:, 1:]).all()
