@@ -1932,8 +1932,9 @@ __device__ __forceinline__ void lr_rows(double* Y, int ly, const LrMat& A1, cons
 }
 
 // Cholesky of a Gram matrix G = Y^T Y (k x k, zero-padded) of a Y of m rows, G (+ shift) = C^T C:
-// S1 := C^-T, so that Y C^-1 = Y S1^T (one Cholesky-QR pass), or S1 := C itself (factor); G is
-// overwritten.  Elimination of [G | I] without pivoting, eight rows at a time: one warp eliminates
+// S1 := C^-T, so that Y C^-1 = Y S1^T (one Cholesky-QR pass), or (factor) S1 := C times the power of two
+// that brings the trace of C^T C near 1: what the truncation decides is relative, and its squares of
+// squares then stay in range whatever the norm of Y.  G is overwritten.  Elimination of [G | I] without pivoting, eight rows at a time: one warp eliminates
 // them against each other (a column of G and one of the right half per lane, the eight rows in
 // registers, multipliers by shuffles), then all warps update the rows below on the FP64 tensor cores.
 // A non-positive pivot marks a rank-deficient column, which becomes zero.  The chain of one pivot's
@@ -1950,7 +1951,7 @@ __device__ __forceinline__ void lr_chol(double* G, double* S1, double* misc, int
   // `reciprocal`
   const int ex = (__double2hiint(tr) >> 20) & 0x7FF;
   const int half = ex > 0 && ex < 0x7FF ? (ex - 1023) >> 1 : 0;
-  const double down = __hiloint2double((1023 - half) << 20, 0), up = __hiloint2double((1023 + half) << 20, 0);
+  const double down = __hiloint2double((1023 - half) << 20, 0);
   const double down2 = down * down;
   // shift of shifted CholeskyQR3: 11 (m k + k (k + 1)) u ||Y||_F^2, u = 2^-53
   const double sh = shifted ? 11.0 * ((double)m * k + (double)k * (k + 1)) * 1.1102230246251565e-16 * (tr * down2) : 0.0;
@@ -2015,13 +2016,13 @@ __device__ __forceinline__ void lr_chol(double* G, double* S1, double* misc, int
     }
     __syncthreads();
   }
-  for (int e = tid; e < KB * LD; e += NT) S1[e] = factor ? (e % LD >= e / LD ? G[e] * up : 0.0) : S1[e] * down;
+  for (int e = tid; e < KB * LD; e += NT) S1[e] = factor ? (e % LD >= e / LD ? G[e] : 0.0) : S1[e] * down;
   __syncthreads();
 }
 
 // Singular directions of a matrix V from the Cholesky factor C (k x k, k rows of B, stride LD,
-// zero-padded) of its Gram matrix, V^T V = C^T C: one-sided Jacobi makes the rows of C orthogonal,
-// their norms are then V's singular values and the rows themselves, normalized, its right singular
+// zero-padded) of its Gram matrix, V^T V ~ C^T C scaled to a trace near 1: one-sided Jacobi makes the rows
+// of C orthogonal, their norms are then V's singular values, scaled, and the rows themselves, normalized, its right singular
 // vectors.  Then the rank decision: rows in decreasing order of norm, r = #{ norm_i > tol norm_0 }, at
 // most rmax, and S[i] = the i-th direction for i < r (zero rows beyond), so that a row of V times S^T
 // is its coordinates in the kept directions.  Returns r.
