@@ -1947,10 +1947,10 @@ __device__ __forceinline__ void lr_chol(double* G, double* S1, double* misc, int
   double tr = lane < k ? G[lane * LD + lane] : 0.0;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
-  // an even power of two brings the trace near 1: every live pivot is then within the range of
-  // `reciprocal`
+  // an even power of two brings the trace near 1, or a subnormal trace to 2^-52 at least: every live
+  // pivot is then within the range of `reciprocal`, whose estimate takes no subnormal number
   const int ex = (__double2hiint(tr) >> 20) & 0x7FF;
-  const int half = ex > 0 && ex < 0x7FF ? (ex - 1023) >> 1 : 0;
+  const int half = ex < 0x7FF ? (max(ex, 1) - 1023) >> 1 : 0;
   const double down = __hiloint2double((1023 - half) << 20, 0);
   const double down2 = down * down;
   // shift of shifted CholeskyQR3: 11 (m k + k (k + 1)) u ||Y||_F^2, u = 2^-53
