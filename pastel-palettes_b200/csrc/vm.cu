@@ -1764,8 +1764,9 @@ __device__ __forceinline__ bool tri_step(int op, double* B, int ldb, const doubl
 // ACCUM, ORTH and LRTRUNC, made of four pieces with one copy of code each (see dev_gemm for why):
 //   tn    S = X^T [W1 W2], small outputs over many rows, on the FP64 tensor cores
 //   rows  Y = A1 S1^T + alpha A2 S2^T row by row, on the FP64 tensor cores
-//   chol  Cholesky G = C^T C of a Gram matrix: C itself, or S1 = C^-T with Y C^-1 = Y S1^T
-//   svd   one-sided Jacobi on C and the rank decision: the matrix S2 of kept singular directions
+//   chol  Cholesky G = C^T C of a Gram matrix: S1 = C^-T with Y C^-1 = Y S1^T
+//   svd   pivoted factor C of a Gram matrix, one-sided Jacobi on C and the rank decision: the matrix S2 of
+//         kept singular directions
 // ACCUM: U1 V1^T := Q Q^T (U1 V1^T + alpha U2 V2^T), Q spanning (U1 V1^T + alpha U2 V2^T) R, the
 // reference's randomized accumulation (kernel.cu:1255-1280) with Q from shifted CholeskyQR3 (three
 // Gram passes) in place of the reference's Givens sweeps; m = ny, n = nx, k = k1 (target rank),
@@ -1931,28 +1932,32 @@ __device__ __forceinline__ void lr_rows(double* Y, int ly, const LrMat& A1, cons
   __syncthreads();
 }
 
-// Cholesky of a Gram matrix G = Y^T Y (k x k, zero-padded) of a Y of m rows, G (+ shift) = C^T C:
-// S1 := C^-T, so that Y C^-1 = Y S1^T (one Cholesky-QR pass), or (factor) S1 := C times the power of two
-// that brings the trace of C^T C near 1: what the truncation decides is relative, and its squares of
-// squares then stay in range whatever the norm of Y.  G is overwritten.  Elimination of [G | I] without pivoting, eight rows at a time: one warp eliminates
-// them against each other (a column of G and one of the right half per lane, the eight rows in
-// registers, multipliers by shuffles), then all warps update the rows below on the FP64 tensor cores.
-// A non-positive pivot marks a rank-deficient column, which becomes zero.  The chain of one pivot's
-// reciprocal after the other bounds it (a form with every thread on its own entries and a barrier
-// per row took three times as long).
-template <int KB>
-__device__ __forceinline__ void lr_chol(double* G, double* S1, double* misc, int k, int m, bool shifted, bool factor) {
-  constexpr int LD = LrSmem<KB>::LD;
-  const int tid = thread_index(), warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3, col = lane & (KB - 1);
-  double tr = lane < k ? G[lane * LD + lane] : 0.0;
+// The power of two, 2^-half, that brings a Gram matrix's trace near 1 (a subnormal one to 2^-52 at
+// least) when it is applied twice: every live pivot is then within the range of `reciprocal`, whose
+// estimate takes no subnormal number.  `mine`: the lane's diagonal entry; tr: the trace.
+__device__ __forceinline__ double lr_scale(double mine, double& tr) {
+  tr = mine;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
-  // an even power of two brings the trace near 1, or a subnormal trace to 2^-52 at least: every live
-  // pivot is then within the range of `reciprocal`, whose estimate takes no subnormal number
   const int ex = (__double2hiint(tr) >> 20) & 0x7FF;
   const int half = ex < 0x7FF ? (max(ex, 1) - 1023) >> 1 : 0;
-  const double down = __hiloint2double((1023 - half) << 20, 0);
-  const double down2 = down * down;
+  return __hiloint2double((1023 - half) << 20, 0);
+}
+
+// Cholesky of a Gram matrix G = Y^T Y (k x k, zero-padded) of a Y of m rows, G (+ shift) = C^T C:
+// S1 := C^-T, so that Y C^-1 = Y S1^T (one Cholesky-QR pass); G is overwritten.  Elimination of
+// [G | I] without pivoting, eight rows at a time: one warp eliminates them against each other (a
+// column of G and one of the right half per lane, the eight rows in registers, multipliers by
+// shuffles), then all warps update the rows below on the FP64 tensor cores.  A non-positive pivot
+// marks a rank-deficient column, which becomes zero.  The chain of one pivot's reciprocal after the
+// other bounds it (a form with every thread on its own entries and a barrier per row took three times
+// as long).
+template <int KB>
+__device__ __forceinline__ void lr_chol(double* G, double* S1, int k, int m, bool shifted) {
+  constexpr int LD = LrSmem<KB>::LD;
+  const int tid = thread_index(), warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3, col = lane & (KB - 1);
+  double tr;
+  const double down = lr_scale(lane < k ? G[lane * LD + lane] : 0.0, tr), down2 = down * down;
   // shift of shifted CholeskyQR3: 11 (m k + k (k + 1)) u ||Y||_F^2, u = 2^-53
   const double sh = shifted ? 11.0 * ((double)m * k + (double)k * (k + 1)) * 1.1102230246251565e-16 * (tr * down2) : 0.0;
   const double tiny = 1e-28 * (tr * down2);
@@ -2016,12 +2021,62 @@ __device__ __forceinline__ void lr_chol(double* G, double* S1, double* misc, int
     }
     __syncthreads();
   }
-  for (int e = tid; e < KB * LD; e += NT) S1[e] = factor ? (e % LD >= e / LD ? G[e] : 0.0) : S1[e] * down;
+  for (int e = tid; e < KB * LD; e += NT) S1[e] *= down;
   __syncthreads();
 }
 
-// Singular directions of a matrix V from the Cholesky factor C (k x k, k rows of B, stride LD,
-// zero-padded) of its Gram matrix, V^T V ~ C^T C scaled to a trace near 1: one-sided Jacobi makes the rows
+// C^T C = G P times a power of two for the Gram matrix G of a factor to be truncated: rows of C, k of them
+// at most (zero beyond; k x k, zero-padded), by elimination with the largest remaining diagonal entry as the
+// pivot.  A column whose remaining entry is at most k u of what it was is noise and gets no row: dividing by
+// its root would spread that noise over the others (an exactly rank-deficient G without pivoting: errors
+// up to 2e-5 of G, and a rank beyond its own at tolerances of 1e-7 in a third of the cases), while all that
+// is left then errs by k u sqrt(g_ii g_jj), as G's own rounding does.  The norms of the rows come out
+// decreasing by and large, which also saves the Jacobi below one sweep or two.
+// One warp, a column per lane: row s is pivot p's row of G minus the rows before it, times their
+// entries in p; pivots by their upper 27 bits and lane in one integer reduction.  The chain of pivots
+// bounds it: reduction, reciprocal root, update of the diagonal.
+template <int KB>
+__device__ __forceinline__ void lr_factor(const double* G, double* C, int k) {
+  constexpr int LD = LrSmem<KB>::LD;
+  const int tid = thread_index(), lane = tid & 31, col = lane & (KB - 1);
+  for (int e = tid; e < KB * LD; e += NT) C[e] = 0.0;
+  __syncthreads();
+  if (tid < 32) {
+    const double mine = lane < k ? G[lane * LD + lane] : 0.0;
+    double tr;
+    const double down = lr_scale(mine, tr), down2 = down * down;
+    double left = mine * down2;  // of the lane's diagonal entry; 0 once it has been the pivot
+    const double noise = (double)k * 1.1102230246251565e-16 * left;
+    bool done = false;
+#pragma unroll 1
+    for (int s = 0; s < k; ++s) {
+      const unsigned key = left > noise ? ((unsigned)__double2hiint(left) & ~31u) | (31u - lane) : 0u;
+      const unsigned best = __reduce_max_sync(0xffffffffu, key);
+      if (best < 32u) break;
+      const int p = 31 - (int)(best & 31u);
+      const double d = __shfl_sync(0xffffffffu, left, p), r = rsqrt(d);
+      double x = G[p * LD + col] * down2, y = 0.0;
+      const double *cp = C + p, *cc = C + col;
+#pragma unroll 1
+      for (int t = 0; t < s; t += 4) {  // rows past s are zero
+#pragma unroll
+        for (int u = 0; u < 4; u += 2) {
+          x = fma(-cp[(t + u) * LD], cc[(t + u) * LD], x);
+          y = fma(-cp[(t + u + 1) * LD], cc[(t + u + 1) * LD], y);
+        }
+      }
+      const double c = done ? 0.0 : lane == p ? d * r : (x + y) * r;
+      done |= lane == p;
+      left = done ? 0.0 : fma(-c, c, left);
+      if (lane < KB) C[s * LD + lane] = c;
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+}
+
+// Singular directions of a matrix V from a factor C (k x k, k rows of B, stride LD, zero-padded) of its
+// Gram matrix, V^T V ~ C^T C scaled to a trace near 1 (lr_factor): one-sided Jacobi makes the rows
 // of C orthogonal, their norms are then V's singular values, scaled, and the rows themselves, normalized, its right singular
 // vectors.  Then the rank decision: rows in decreasing order of norm, r = #{ norm_i > tol norm_0 }, at
 // most rmax, and S[i] = the i-th direction for i < r (zero rows beyond), so that a row of V times S^T
@@ -2205,7 +2260,8 @@ __device__ __forceinline__ void lowrank_impl(const pp_task& T) {
       const LrMat W2 = ph == 0 ? Mv2 : ph == 4 ? Mu2 : none;
       const bool gram = ph != 0 && ph != 4;
       lr_tn<KB>(X, W1, W2, ph == 0 || ph == 5 ? n : m, gram ? G : S1, S2);
-      if (ph >= 1 && ph != 4) lr_chol<KB>(G, S1, misc, k, m, ph == 1, ph == 5);
+      if (ph >= 1 && ph <= 3) lr_chol<KB>(G, S1, k, m, ph == 1);
+      if (ph == 5) lr_factor<KB>(G, S1, k);
       if (ph == 5) rank = lr_svd<KB>(S1, S2, misc, k, T.beta, rmax);
     }
     const bool first = ph == 0 || ph == 4;
