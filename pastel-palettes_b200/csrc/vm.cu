@@ -2242,14 +2242,8 @@ __device__ __forceinline__ void lowrank_impl(const pp_task& T) {
     for (int e = threadIdx.x; e < m * k; e += NT) Y[(e / k) * ly + e % k] = ldcg(&U[e]);
     __syncthreads();
   }
-  // without a tolerance or a smaller limit there is nothing to truncate
   const int rmax = (!accum && T.o > 0) ? min(T.o, k) : k;
   int rank = k;
-  if (!accum && !orth && T.beta <= 0.0 && rmax == k) {
-    if (threadIdx.x == 0 && T.p[5]) T.p[5][0] = (double)rank;
-    __syncthreads();
-    return;
-  }
   // phases: 0 the sketch, 1-3 the Cholesky-QR passes, 4 the projection, 5 the truncation of V and
   // 6 of the orthonormal factor
 #pragma unroll 1
