@@ -2082,12 +2082,13 @@ __device__ __forceinline__ void lr_factor(const double* G, double* C, int k) {
 // most rmax, and S[i] = the i-th direction for i < r (zero rows beyond), so that a row of V times S^T
 // is its coordinates in the kept directions.  Returns r.
 //
-// The factor of a graded Gram matrix is close to row-orthogonal already: 7 or 8 sweeps where the
+// The pivoted factor of a graded Gram matrix is close to row-orthogonal already: 5 or 6 sweeps where the
 // two-sided Jacobi on the Gram matrix took 12 (its limit), a third of the shared-memory traffic, and
 // the directions are orthogonal to rounding however small their singular value.  Round-robin order,
 // k/2 disjoint pairs at once, eight lanes of the first four warps per pair, which all compute its
-// rotation; one barrier of those warps per step.  A pair is rotated while |b_p . b_q| > 1e-13 |b_p| |b_q| and the smaller norm counts for the
-// rank (> 1e-2 tol of the largest); a sweep whose rotations were all below 1e-8 is the last (the next
+// rotation; one barrier of those warps per step.  A pair is rotated while |b_p . b_q| > 1e-15 |b_p| |b_q|
+// (a few u: what is left bounds the directions' products) and the smaller norm counts for the rank
+// (> 1e-2 tol of the largest); a sweep whose rotations were all below 1e-8 is the last (the next
 // would find products of such angles), and at most 14 are made.  The rotation is the symmetric
 // Schur decomposition of the pair's 2 x 2 Gram matrix (Golub & Van Loan, sym.schur2), t = tan(theta)
 // written as 2 a sgn(d) / (|d| + h), d = |b_q|^2 - |b_p|^2, h = sqrt(d^2 + 4 a^2): cos = r / s,
@@ -2171,7 +2172,7 @@ __device__ __forceinline__ int lr_svd(double* B, double* S, double* misc, int k,
         const double rr = fma(v, rsqrt_seed(v), fabs(d)), s2 = fma(rr, rr, gg), y0 = rsqrt_seed(s2);
         const double e = fma(-s2 * y0, y0, 1.0), w = fma(y0 * e, fma(0.375, e, 0.5), y0);
         const double a2 = a * a, both = app * aqq;
-        const int rot = (int)(a2 > 1e-26 * both) & (int)(fmin(app, aqq) > floor2) & (int)(v > 1e-280) &
+        const int rot = (int)(a2 > 1e-30 * both) & (int)(fmin(app, aqq) > floor2) & (int)(v > 1e-280) &
                         (int)(s2 < 1e280) & (int)(pair < np);
         if (rot) {
           const double c = rr * w, sn = g2 * w;
