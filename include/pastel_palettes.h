@@ -272,6 +272,8 @@ pp_status pp_dense_residual_dev(pp_context* ctx, const double* A, int lda, int n
                                 double* r, int nrhs, void* stream);
 /* r := b - A x, A_ij = K(|p_i - p_j|) + shift * (i == j) evaluated on the fly.
  * kernel: 0 = 1/(r+p0), 1 = 1/(4 pi (r+p0)), 2 = exp(-r/p0), 3 = Matern-3/2 length p0.
+ * A squared distance that overflows counts as 2^1023.  With p0 = 0 (kernels 0 and 1 take it) an entry
+ * at distance zero, the diagonal among them, is not finite.
  * Partial sums go through a context-owned buffer, grown on the first call of a larger size
  * (make that call before capturing a CUDA graph); calls on different streams must not
  * overlap. */
@@ -280,9 +282,9 @@ pp_status pp_kernel_residual_dev(pp_context* ctx, int kernel, double p0, double 
                                  void* stream);
 /* The dense blocks of an uploaded H-matrix assembled on the device from its points (device,
  * n x dim, in the H-matrix's cluster order): entry (i, j) = K(|p_i - p_j|) with the kernels of
- * pp_kernel_residual_dev, plus `shift` on the matrix diagonal, with the same entry evaluation as
- * the residual.  Low-rank blocks are left as they are.  No reference counterpart (the
- * reference's matrices come from a separate Java compressor). */
+ * pp_kernel_residual_dev, plus `shift` on the matrix diagonal, with the entry evaluation of the
+ * one-column residual (the wider ones' entries are a few ulps apart).  Low-rank blocks are left as
+ * they are.  No reference counterpart (the reference's matrices come from a separate Java compressor). */
 pp_status pp_hmatrix_assemble_dense_dev(pp_hmatrix* h, int kernel, double p0, double shift, const double* pts_dev,
                                         int dim, void* stream);
 /* Builds the whole H-matrix on the device from its points (device, n x dim, in the H-matrix's

@@ -2823,18 +2823,28 @@ __device__ __forceinline__ double rcp_refine(double a, double y0) {
   const double e = fma(-a, y0, 1.0);
   return fma(y0, fma(e, e, e), y0);
 }
-// Entry K(d) of the kernel matrix at squared distance d2.  The distance: y0 estimates
-// 1 / sqrt(max(d2, 1e-300)), s0 = d2 y0 and e = 1 - s0 y0 = 1 - d2 y0^2; then
-// sqrt(d2) = s0 (1 - e)^(-1/2) = s0 (1 + e/2 + 3e^2/8 + O(e^3)) (binomial series, truncated
-// terms below 2^-58 relative for |e| < 2^-19).  Exact zero on the diagonal and for coincident
-// points, an absolute error below 1e-150 for 0 < d2 < 1e-300, a few ulps elsewhere.
-template <int KIND>
-__device__ __forceinline__ double kernel_eval_nr(double d2, double p0, double inv_p0) {
-  constexpr double c = KIND == 1 ? 4.0 * 3.14159265358979323846 : 1.0;
-  const double y0 = rsqrt_est(fmax(d2, 1e-300));
+// The distance of a squared one: y0 estimates 1 / sqrt(max(d2, 1e-300)), s0 = d2 y0 and
+// e = 1 - s0 y0 = 1 - d2 y0^2; then sqrt(d2) = s0 (1 - e)^(-1/2) = s0 (1 + e/2 + 3e^2/8 + O(e^3))
+// (binomial series, truncated terms below 2^-58 relative for |e| < 2^-19).  Exact zero on the
+// diagonal and for coincident points, an absolute error below 1e-150 for 0 < d2 < 1e-300, a few ulps
+// elsewhere; no number stays none.
+__device__ __forceinline__ double distance_from(double d2, double y0) {
   const double s0 = d2 * y0;
   const double e = fma(-s0, y0, 1.0);
-  const double d = fma(s0 * e, fma(0.375, e, 0.5), s0);
+  return fma(s0 * e, fma(0.375, e, 0.5), s0);
+}
+// An overflowed d2 counts as 2^1023.  Both bounds are put on the upper word, by which the estimate goes: the
+// FP64 pipe is the full one in the residual kernels (one column, 32 jobs of 8192: 4% of a refined
+// batch; with a comparison in FP64 the product of 8 columns takes 8% longer).
+__device__ __forceinline__ double distance_of(double d2) {
+  const int up = __double2hiint(d2), hi = up == 0x7ff00000 ? 0x7fe00000 : up, lo = __double2loint(d2);
+  // 0x01a56e1f: upper word of 1e-300
+  return distance_from(__hiloint2double(hi, lo), rsqrt_est(__hiloint2double(max(hi, 0x01a56e1f), lo)));
+}
+// Entry of the kernel matrix at distance d.
+template <int KIND>
+__device__ __forceinline__ double kernel_at(double d, double p0, double inv_p0) {
+  constexpr double c = KIND == 1 ? 4.0 * 3.14159265358979323846 : 1.0;
   if (KIND <= 1) {
     const double x = c * (d + p0);
     return rcp_refine(x, rcp_est(x));
@@ -2863,7 +2873,9 @@ __device__ __forceinline__ float kernel_eval_f32(float d2, float p0, float inv_p
 
 // C[m x k] = K(P_I, P_J) B (PP_OP_KMUL): a thread per row of C, the columns j of the kernel
 // matrix in chunks of KM_JC whose points and B rows are staged in shared memory (read by all
-// threads as broadcasts); points padded to three coordinates with zeros
+// threads as broadcasts); points padded to three coordinates with zeros.  The distance is bounded below in
+// FP64 and not above: distance_of here, a few instructions longer or shorter, shifts the VM's code and made
+// every other instruction 2 to 5% slower.
 #define KM_JC 128
 template <int KIND>
 __device__ __noinline__ void kmul_impl(const pp_task& T, double* smem) {
@@ -2897,7 +2909,7 @@ __device__ __noinline__ void kmul_impl(const pp_task& T, double* smem) {
       for (int j = 0; j < jc; ++j) {
         const double u0 = pr[0] - sp[3 * j], u1 = pr[1] - sp[3 * j + 1], u2 = pr[2] - sp[3 * j + 2];
         const double d2 = fma(u2, u2, fma(u1, u1, u0 * u0));
-        const double a = kernel_eval_nr<KIND>(d2, p0, inv_p0);
+        const double a = kernel_at<KIND>(distance_from(d2, rsqrt_est(fmax(d2, 1e-300))), p0, inv_p0);
 #pragma unroll
         for (int c = 0; c < PP_VM_MAX_RANK; ++c) acc[c] = fma(a, sb[j * PP_VM_MAX_RANK + c], acc[c]);
       }
@@ -2972,7 +2984,7 @@ __device__ __forceinline__ void residual_steps(const double* sp, const double* s
       const double u = pi[d] - sp[jj * DIM + d];
       d2 = fma(u, u, d2);
     }
-    const double ak = kernel_eval_nr<KIND>(d2, p0, inv_p0);
+    const double ak = kernel_at<KIND>(distance_of(d2), p0, inv_p0);
     const double a = live ? ak : 0.0;
 #pragma unroll
     for (int q = 0; q < NR; ++q) acc[q] = fma(a, sx[jj * NR + q], acc[q]);
@@ -3130,14 +3142,10 @@ __global__ void __launch_bounds__(KR_SEG) kernel_residual_sym(const __grid_const
 // 8 columns 9.7 -> 5.8 ms (before: a row-block form that evaluated every entry twice), 3 columns 20.8 ->
 // 5.6 ms (before: column sums of every entry read and written in shared memory).
 #define KW_LDX 10  /* doubles between the rows of a staged right-hand side block: 2 mod 8 */
+// kernel_at(distance_of(d2)) with c (d + p0) as c d + c p0: a few ulps apart, one operation less
 template <int KIND>
 __device__ __forceinline__ double kernel_eval_wide(double d2, double p0, double cp0, double inv_p0) {
-  // d2 comes with 1e-300 added (nothing to a distance above 1e-140), which keeps the estimate finite;
-  // an overflowed one is brought down to 2^1023 by an integer select (the FP64 pipe is the full one)
-  const int hi = __double2hiint(d2);
-  d2 = __hiloint2double(hi == 0x7ff00000 ? 0x7fe00000 : hi, __double2loint(d2));
-  const double y0 = rsqrt_est(d2), s0 = d2 * y0, e = fma(-s0, y0, 1.0);
-  const double d = fma(s0 * e, fma(0.375, e, 0.5), s0);
+  const double d = distance_of(d2);
   if (KIND <= 1) {
     constexpr double c = KIND == 1 ? 4.0 * 3.14159265358979323846 : 1.0;
     const double x = fma(c, d, cp0);
@@ -3209,7 +3217,7 @@ __global__ void __launch_bounds__(KW_SEG) kernel_residual_wide(const __grid_cons
         double e[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          double d2 = 1e-300;
+          double d2 = 0.0;
 #pragma unroll
           for (int d = 0; d < DIM; ++d) {
             const double u = pi[t][d] - p[h][d];
@@ -3350,8 +3358,9 @@ cudaError_t launch_elementwise(const pp_resid_job* jobs, const std::vector<int>&
 // Dense blocks of an H-matrix assembled in place from its points (the first step of building it
 // on the device): entry (i, j) of the block at rows [r0, r0 + m), columns [c0, c0 + n) is
 // K(|p_{r0+i} - p_{c0+j}|), plus the shift on the matrix diagonal, with the residual kernel's
-// distance and entry evaluation (the same bits as the matrix the refinement applies).  One CTA
-// per AS_ROWS rows of a block; blocks passed by value, up to AS_LAUNCH_JOBS per launch.
+// distance and entry evaluation (the bits of the matrix that the one-column product applies, a few ulps
+// from those of the wider one).  One CTA per AS_ROWS rows of a block; blocks passed by value, up to
+// AS_LAUNCH_JOBS per launch.
 #define AS_LAUNCH_JOBS 64
 #define AS_ROWS 16
 struct AssembleLaunch {
@@ -3385,7 +3394,7 @@ __global__ void __launch_bounds__(256) assemble_dense_kernel(const __grid_consta
       const double u = L.pts[(size_t)gi * DIM + d] - L.pts[(size_t)gj * DIM + d];
       d2 = fma(u, u, d2);
     }
-    double a = kernel_eval_nr<KIND>(d2, L.p0, inv_p0);
+    double a = kernel_at<KIND>(distance_of(d2), L.p0, inv_p0);
     if (gi == gj) a += L.shift;
     jb.a[(size_t)i * jb.ld + j] = a;
   }
