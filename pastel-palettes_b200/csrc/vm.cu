@@ -3178,7 +3178,9 @@ __global__ void __launch_bounds__(KW_SEG) kernel_residual_wide(const __grid_cons
   const int J = I + (int)(b - row_start(I));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, fa = lane >> 2, fb = lane & 3;
   const int i0 = I * KW_SEG + 32 * warp, j0 = J * KW_SEG;
-  for (int e = tid; e < KW_SEG * DIM; e += KW_SEG) pj[e] = j0 + e / DIM < n ? pts[(size_t)j0 * DIM + e] : 0.0;
+  // places past the last point take that point: an entry there is one of the matrix, so its product with a
+  // zero of x or of xi is zero wherever the sums it goes to are numbers
+  for (int e = tid; e < KW_SEG * DIM; e += KW_SEG) pj[e] = pts[(size_t)min(j0 + e / DIM, n - 1) * DIM + e % DIM];
   for (int e = tid; e < KW_SEG * 8; e += KW_SEG) {
     const int r = e >> 3, q = e & 7;
     xj[r * KW_LDX + q] = (j0 + r < n && q0 + q < nrhs) ? x[(size_t)(j0 + r) * nrhs + q0 + q] : 0.0;

@@ -52,3 +52,18 @@ def test_no_parameter_is_no_number_on_the_diagonal(pp, gctx, kernel):
     pts, x, b = rng.uniform(0, 1, (300, 2)), rng.standard_normal((300, 8)), rng.standard_normal((300, 8))
     for q in (1, 2, 8):
         assert not np.isfinite(residual(pp, gctx, kernel, 0.0, pts, x[:, :q].copy(), b[:, :q].copy())).any()
+
+
+@pytest.mark.parametrize("n", [5, 257, 300])
+@pytest.mark.parametrize("nrhs", NRHS)
+def test_places_past_the_last_point_are_of_no_account(pp, gctx, n, nrhs):
+    """Points far from the origin and a kernel that grows with the distance (a negative length is accepted):
+    an entry between a point and the origin would overflow, and nothing of it may reach a sum."""
+    rng = np.random.default_rng(n)
+    pts = 1000.0 + 0.01 * rng.uniform(0, 1, (n, 3))
+    x, b = rng.standard_normal((n, nrhs)), rng.standard_normal((n, nrhs))
+    d = np.sqrt(((pts[:, None, :] - pts[None, :, :]) ** 2).sum(-1))
+    A = np.exp(d / 0.05) + 0.5 * np.eye(n)
+    r = residual(pp, gctx, "exp", -0.05, pts, x, b)
+    # entries to 8 u and their argument's 6 u; the coordinates' differences are exact
+    assert (np.abs(r - (b - A @ x)) <= 2 * (n + 16) * 2.0 ** -53 * (np.abs(A) @ np.abs(x) + np.abs(b))).all()
