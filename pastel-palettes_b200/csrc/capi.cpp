@@ -358,6 +358,9 @@ pp_status launch_plan(pp_hmatrix* h, VmPlan& plan, cudaStream_t s, int grid_cap)
 pp_status vm_state_status(pp_context* ctx, const pp_vm_state& s, int n_tasks) {
   if (s.error == PP_VM_TIMEOUT)
     return fail(ctx, PP_TIMEOUT, "VM: ready-queue slot " + std::to_string(s.err_info) + " never filled");
+  if (s.error == PP_VM_IDLE)
+    return fail(ctx, PP_TIMEOUT, "VM: no task became ready within the time limit (" + std::to_string(s.err_info) + " of " +
+                                     std::to_string(n_tasks) + " done)");
   if (s.error == PP_VM_MMA_TIMEOUT)
     return fail(ctx, PP_TIMEOUT, "VM: tensor-core completion of task " + std::to_string(s.err_info) + " not observed");
   if (s.error == PP_VM_BAD_TASK)

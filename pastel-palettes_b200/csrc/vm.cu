@@ -6,8 +6,8 @@
 // CTA of a persistent grid takes the next READY task from a device queue (one queue, or one per
 // priority class); finishing a task decrements its successors' dependency counters, and of those
 // that reach zero the CTA runs the first and pushes the others.  Waits are bounded: a CTA that
-// finds nothing for longer than its time limit (globaltimer) records PP_VM_TIMEOUT and every CTA
-// returns.
+// finds nothing for longer than its time limit (globaltimer) records PP_VM_TIMEOUT or PP_VM_IDLE and
+// every CTA returns.
 //
 // Arithmetic contract (FP64 path): every matrix element receives its updates in the
 // order the reference's routines apply them, one fma per product with the same
@@ -2596,7 +2596,8 @@ __device__ __forceinline__ int take_by_class(int32_t* slots, int n, const pp_vm_
     }
     // bounded in time, as a wait on the one queue is
     if (__any_sync(0xffffffffu, (long long)(gtimer_ns() - t0) > wait_ns)) {
-      if (lane == 0 && atomicCAS(&st->error, 0, PP_VM_TIMEOUT) == 0) st->err_info = slot >= 0 ? slot : ld_relaxed(&st->done);
+      if (lane == 0 && atomicCAS(&st->error, 0, slot >= 0 ? PP_VM_TIMEOUT : PP_VM_IDLE) == 0)
+        st->err_info = slot >= 0 ? slot : ld_relaxed(&st->done);
       return -1;
     }
   }

@@ -11,14 +11,15 @@
 #define PP_VM_INV 512          /* largest leaf of a TRINV / TRMV task (explicit inverses)       */
 #define PP_VM_MAX_RANK 32      /* largest k1 of ACCUM (register-resident reductions)    */
 
-enum pp_vm_error { PP_VM_OK = 0, PP_VM_TIMEOUT = 1, PP_VM_BAD_TASK = 2, PP_VM_MMA_TIMEOUT = 3 };
+/* PP_VM_TIMEOUT: a queue slot was not filled in time; PP_VM_IDLE: by priority class, no task became ready in time */
+enum pp_vm_error { PP_VM_OK = 0, PP_VM_TIMEOUT = 1, PP_VM_BAD_TASK = 2, PP_VM_MMA_TIMEOUT = 3, PP_VM_IDLE = 4 };
 
 typedef struct pp_vm_state {
   int head;      /* next ready-slot index to pop                  */
   int tail;      /* next ready-slot index to fill                 */
   int done;      /* tasks completed                               */
   int error;     /* pp_vm_error                                   */
-  int err_info;  /* slot index (timeout) or task id (bad task)    */
+  int err_info;  /* slot index (timeout), tasks completed (idle) or task id (the others) */
   int pad[3];
 } pp_vm_state;
 
