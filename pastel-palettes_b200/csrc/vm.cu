@@ -887,6 +887,19 @@ __device__ __noinline__ bool dev_gemm_bf16(double* __restrict__ C, int ldc, cons
   return ok;
 }
 
+// Estimates from the special-function unit: PTX rsqrt.approx.ftz.f64 / rcp.approx.ftz.f64
+// (computed from the upper word of the double, about single-precision accuracy, full double
+// exponent range; zero gives infinity).
+__device__ __forceinline__ double rsqrt_est(double v) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+  return y;
+}
+__device__ __forceinline__ double rcp_est(double v) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+  return y;
+}
 // ------------------------------------------------------------------------- quotients
 // A division takes 128 cycles of dependent work on this chip, and the triangular routines have one
 // per row on their critical path.  These are the same correctly rounded quotients from published
@@ -896,17 +909,12 @@ __device__ __noinline__ bool dev_gemm_bf16(double* __restrict__ C, int ldc, cons
 // q = RN(x y), the residual exact in an fma, leave RN(x / t), as long as nothing over- or underflows.
 // quotient_unsafe: exponents for which that may not hold (a positive zero is fine); the routines fall
 // back to divisions then.  Compared with `/` on 2^32 random pairs: no difference.
-__device__ __forceinline__ double rcp_seed(double v) {
-  double y;
-  asm volatile("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
-  return y;
-}
-__device__ __forceinline__ double reciprocal(double t, double y) {  // y: rcp_seed(t)
+__device__ __forceinline__ double reciprocal(double t, double y) {  // y: rcp_est(t)
   const double e = fma(-t, y, 1.0);
   y = fma(y, fma(e, e, e), y);
   return fma(fma(-t, y, 1.0), y, y);
 }
-__device__ __forceinline__ double reciprocal(double t) { return reciprocal(t, rcp_seed(t)); }
+__device__ __forceinline__ double reciprocal(double t) { return reciprocal(t, rcp_est(t)); }
 __device__ __forceinline__ double quotient(double x, double t, double y) {
   double q = x * y;
   q = fma(fma(-q, t, x), y, q);
@@ -1033,7 +1041,7 @@ __device__ __forceinline__ void dev_getrf(double* A, int lda, int m, int n) {
 #pragma unroll 1
       for (int i = 0; i < steps; ++i) {
         double* row = S + (cg + i) * GETRF_LD + cg + i;
-        const double p = __shfl_sync(0xffffffffu, x[0][0], off + i), seed = rcp_seed(p);
+        const double p = __shfl_sync(0xffffffffu, x[0][0], off + i), seed = rcp_est(p);
 #pragma unroll
         for (int c = 0; c < 8; ++c) sts_if(row + c, x[0][c], lane == off + i && c < w - i);
         __syncwarp();
@@ -2095,11 +2103,6 @@ __device__ __forceinline__ void lr_factor(const double* G, double* C, int k) {
 // sin = 2 a sgn(d) / s with r = |d| + h, s = sqrt(r^2 + 4 a^2).  h only steers the angle and comes
 // from an estimate of the reciprocal root; 1 / s, which makes the rotation orthogonal, is corrected
 // to full precision (y (1 + e/2 + 3 e^2/8), e = 1 - s^2 y^2, binomial series).
-__device__ __forceinline__ double rsqrt_seed(double v) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
-  return y;
-}
 __device__ __forceinline__ void round_robin(int kk, int r, int jp, int& p, int& q) {
   // positions of pair jp in step r: 1 + (pos - 1 + r) mod (kk - 1); position 0 stays
   int ua = jp - 1 + r, ub = kk - 2 - jp + r;
@@ -2169,7 +2172,7 @@ __device__ __forceinline__ int lr_svd(double* B, double* S, double* misc, int k,
         for (int i = 0; i < NE; ++i) dot = fma(x[i], y[i], dot);
         const double app = n2[p], aqq = n2[q], a = sum8(dot);
         const double d = aqq - app, g2 = d >= 0.0 ? 2.0 * a : -2.0 * a, gg = g2 * g2, v = fma(d, d, gg);
-        const double rr = fma(v, rsqrt_seed(v), fabs(d)), s2 = fma(rr, rr, gg), y0 = rsqrt_seed(s2);
+        const double rr = fma(v, rsqrt_est(v), fabs(d)), s2 = fma(rr, rr, gg), y0 = rsqrt_est(s2);
         const double e = fma(-s2 * y0, y0, 1.0), w = fma(y0 * e, fma(0.375, e, 0.5), y0);
         const double a2 = a * a, both = app * aqq;
         const int rot = (int)(a2 > 1e-30 * both) & (int)(fmin(app, aqq) > floor2) & (int)(v > 1e-280) &
@@ -2620,7 +2623,7 @@ __global__ void __launch_bounds__(NT, 1)
   __shared__ int s_abort;
   TcCtx tc{0u, 0u, 0u, wait_ns, 0, 0, 0u, 0u, 0u, &s_abort};
   if (use_tc) {
-    // TF32 tasks: 64 TMEM columns (128 lanes x 64 FP32 accumulators) and one mbarrier per CTA
+    // TF32 and BF16 tasks: all 512 TMEM columns (TF32 uses 64, BF16 two accumulators of 256) and mbarriers
     if ((threadIdx.x >> 5) == 0) {
       asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
                    "r"(TC_TMEM_COLS)
@@ -2803,19 +2806,6 @@ __global__ void dense_residual_kernel(const double* __restrict__ A, int lda, int
   }
 }
 
-// Estimates from the special-function unit: PTX rsqrt.approx.ftz.f64 / rcp.approx.ftz.f64
-// (computed from the upper word of the double, about single-precision accuracy, full double
-// exponent range; zero gives infinity).
-__device__ __forceinline__ double rsqrt_est(double v) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
-  return y;
-}
-__device__ __forceinline__ double rcp_est(double v) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
-  return y;
-}
 // One third-order correction of an estimate y0 of 1/a: with e = 1 - a y0,
 // 1/a = y0 (1 - e)^-1 = y0 (1 + e + e^2 + O(e^3)) (geometric series).  For |e| < 2^-19 the
 // truncated terms are below 2^-57 relative: the result is within a few ulps of double, the
@@ -3484,7 +3474,7 @@ cudaError_t pp_accum_noalloc_launch(const pp_task& T, long long scratch_doubles,
   if (g_noalloc_err[dev] != cudaSuccess) return g_noalloc_err[dev];
   pp_task t = T;
   t.tmp = g_noalloc_addr[dev];
-  // 160 KB of dynamic shared memory, as the VM's ACCUM has; pp_vm_prepare (run at context
+  // 180 KB of dynamic shared memory, as the VM's ACCUM has; pp_vm_prepare (run at context
   // creation on this device) raised the kernel's limit to that
   accum_noalloc_kernel<<<1, NT, VM_SMEM_BYTES, s>>>(t);
   return cudaGetLastError();
