@@ -34,13 +34,13 @@ C3_NAME = "laplace3d-n65536-leaf512-eta1-rank32tol1e-8-8rhs-bf16schur-fp64ir1e-1
 WORKLOAD = dict(n=8192, dim=2, kernel="inv", p0=1e-3, leaf=256, rank=16, admissibility=0, seed=1234, tol=1e-10)
 WORKLOAD_NAME = "hodlr-inv2d-n8192-leaf256-rank16-fp64-ir1e-10"
 # DRAM bytes (read + write) of one job's factor work inside the batched HODLR factor launch, from
-# one ncu capture of the batch-4 launch (dram__bytes.sum.per_second x gpu__time_duration.sum / 4);
-# the jobs touch disjoint arenas, so the launch's traffic scales with the batch
-FACTOR_DRAM_BYTES_PER_JOB = 117.5e6
+# one ncu capture of the batch-4 launch ((146.8 MB read + 241.6 MB written) / 4); the jobs touch
+# disjoint arenas, so the launch's traffic scales with the batch
+FACTOR_DRAM_BYTES_PER_JOB = (146.834176e6 + 241.603328e6) / 4
 # DRAM bytes (read + write) per algorithmic byte of the mixed factor launch of the headline job,
-# from one ncu capture of the same launch at N = 16384 (28.2 GB read + 25.9 GB written against
-# 72.9 GB of algorithmic bytes); the full-size launch's traffic is estimated by this ratio
-C3_DRAM_PER_ALGORITHMIC_BYTE = (28.221709056e9 + 25.890199552e9) / 72.9413632e9
+# from one ncu capture of the same launch at N = 16384 (18.9 GB read + 15.8 GB written against
+# 46.8 GB of algorithmic bytes); the full-size launch's traffic is estimated by this ratio
+C3_DRAM_PER_ALGORITHMIC_BYTE = (18.939695872e9 + 15.805542144e9) / 46.785421312e9
 
 
 def load_pp():

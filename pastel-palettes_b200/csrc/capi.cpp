@@ -284,7 +284,9 @@ pp_status plan_to_device_multi(pp_context* ctx, const std::vector<pp_hmatrix*>& 
   // could do in that path's time.  Below that a task hardly ever waits for a CTA, and the one queue
   // hands it over sooner (one atomic instead of three).  On a B200, one queue against classes: factor of
   // a mixed-precision matrix with N = 32768 (0.7) 106 -> 95 ms, of 32 with 8192 unknowns (1.2) 10.8 -> 10.1
-  // ms, of 8192 unknowns in FP64 (0.5) 37.2 -> 36.1 ms, of 16 adaptive ones (0.4) 4.0 ms either way.
+  // ms, of 8192 unknowns in FP64 (0.5) 37.2 -> 36.1 ms, of 16 adaptive ones (0.4) 4.0 ms either way. All on
+  // the full grid: a launch limited to fewer CTAs (a served request, a batch's grid limit) queues up at a
+  // lower ratio and takes what its plan took for all of them.
   int64_t longest = 1;
   for (int64_t b : plan.prog.path_ns) longest = std::max(longest, b);
   plan.by_class = n < (1 << PP_VM_ID_BITS) && (double)plan.prog.work_ns >= 0.3 * (double)longest * ctx->sm_count;

@@ -1791,8 +1791,8 @@ __device__ __forceinline__ bool tri_step(int op, double* B, int ldb, const doubl
 // Measured on a B200, hop included (before: reductions with one k step of loads in flight, a
 // one-warp Cholesky, substitutions, a two-sided Jacobi on the Gram matrix):
 //   ACCUM 128 x 128, k 32, adaptive   430 -> 134 us      ACCUM 94 x 94, k 16   54 -> 24 us
-//   ORTH  512 x 32                    144 ->  78 us      LRTRUNC 512 x 512, k 32   420 -> 130 us
-// 17 us of the first are products at the FP64 tensor rate, 79 the chain of Jacobi steps.
+//   ORTH  512 x 32                    144 ->  78 us      LRTRUNC 512 x 512, k 32   420 -> 125 us
+// 17 us of the first are products at the FP64 tensor rate, about 80 the chain of Jacobi steps.
 template <int KB>
 struct LrSmem {  // doubles; KB: largest rank, 16 or 32
   static constexpr int LD = KB + 4;                       // row stride: 4 mod 16, no bank conflicts
